@@ -103,13 +103,20 @@ __host__ __device__ inline long long freq_index(int i, int n) {
     return (i < (n - 1) / 2 + 1) ? i : i - n;   // numpy fftfreq ordering
 }
 
+// (i, j, k) of a half-grid linear index.  A grid has fewer than 2^31 points, so
+// the divisions are 32-bit (the 64-bit ones are long subroutines).
+__host__ __device__ inline void half_index(const Geo& g, long long idx, int& i, int& j, int& k) {
+    const unsigned u = (unsigned)idx, t = u / (unsigned)g.n2h;
+    k = (int)(u - t * (unsigned)g.n2h);
+    i = (int)(t / (unsigned)g.n1);
+    j = (int)(t - (unsigned)i * (unsigned)g.n1);
+}
+
 // G vector and |G|^2 of half-grid linear index idx, evaluated with the same
 // operation order as the reference's einsum (no FMA contraction).
 __device__ inline void gvec(const Geo& g, long long idx, double& gx, double& gy, double& gz, double& gg) {
-    int k = (int)(idx % g.n2h);
-    long long t = idx / g.n2h;
-    int j = (int)(t % g.n1);
-    int i = (int)(t / g.n1);
+    int i, j, k;
+    half_index(g, idx, i, j, k);
     double f0 = __dmul_rn((double)freq_index(i, g.n0), g.fv[0]);
     double f1 = __dmul_rn((double)freq_index(j, g.n1), g.fv[1]);
     double f2 = __dmul_rn((double)k, g.fv[2]);
@@ -148,20 +155,16 @@ __device__ inline float gsq_f(const Geo& g, int i, int j, int k) {
 
 template <>
 __device__ inline float gsq_t<float>(const Geo& g, long long idx) {
-    int k = (int)(idx % g.n2h);
-    int t = (int)(idx / g.n2h);
-    int j = t % g.n1;
-    int i = t / g.n1;
+    int i, j, k;
+    half_index(g, idx, i, j, k);
     return gsq_f(g, i, j, k);
 }
 
 // Half-space mask that counts each +-G pair once (src/dftpy/grid.py:658-695,
 // serial case), as a predicate on the half-grid index.
 __device__ inline bool half_mask(const Geo& g, long long idx) {
-    int k = (int)(idx % g.n2h);
-    long long t = idx / g.n2h;
-    int j = (int)(t % g.n1);
-    int i = (int)(t / g.n1);
+    int i, j, k;
+    half_index(g, idx, i, j, k);
     int D0 = g.n0 / 2, D1 = g.n1 / 2, D2 = g.n2 / 2;
     int M0 = g.n0 % 2, M1 = g.n1 % 2, M2 = g.n2 % 2;
     if (k == 0) {
@@ -269,7 +272,8 @@ __device__ inline void block_reduce_store(double (&v)[NS], const int (&kind)[NS]
     }
 }
 
-// reduce nblk x ns partials into out[ns]; kinds: bit pattern 2 bits per slot
+// reduce nblk x ns partials into out[ns], one block per slot (launch ns blocks of
+// RED_THREADS); kinds: bit pattern 2 bits per slot
 __global__ void reduce_finalize(const double* partials, int nblk, int ns, unsigned long long kinds, double* out);
 
 // ------------------------------------------------------------------ scratch

@@ -322,7 +322,7 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
     OFDFT_REQUIRE(ablk <= g->red_blocks * 32, "Ewald: too many atoms for the reduction buffer");
     k_ewald_real<<<ablk, RED_THREADS, 0, st>>>(d_pos, d_q, nat, d_lat, cl, Rcut, eta, d_Fr, g->d_partials);
     OFDFT_LAUNCH_CHECK();
-    reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, ablk, 7, 0ull, g->d_results);
+    reduce_finalize<<<7, RED_THREADS, 0, st>>>(g->d_partials, ablk, 7, 0ull, g->d_results);
     OFDFT_LAUNCH_CHECK();
     OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 7 * sizeof(double), cudaMemcpyDeviceToHost, st));
     OFDFT_CK(cudaStreamSynchronize(st));
@@ -360,7 +360,7 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
             k_ewald_stress_rec<T><<<g->red_blocks, RED_THREADS, 0, st>>>(QG, nullptr, bre, bim, g->geo, eta,
                                                                          g->d_partials);
             OFDFT_LAUNCH_CHECK();
-            reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
+            reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
             OFDFT_LAUNCH_CHECK();
             OFDFT_CK(cudaMemcpyAsync(s_rec, g->d_results, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
             OFDFT_CK(cudaStreamSynchronize(st));
@@ -394,7 +394,7 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
             k_ewald_stress_rec<T><<<g->red_blocks, RED_THREADS, 0, st>>>(nullptr, S, nullptr, nullptr, g->geo, eta,
                                                                          g->d_partials);
             OFDFT_LAUNCH_CHECK();
-            reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
+            reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
             OFDFT_LAUNCH_CHECK();
             OFDFT_CK(cudaMemcpyAsync(s_rec, g->d_results, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
             OFDFT_CK(cudaStreamSynchronize(st));
@@ -405,7 +405,7 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
                 k_ewald_force_exact<<<g->red_blocks, RED_THREADS, 0, st>>>(d_pos, d_q, S, a0, na, g->geo, eta,
                                                                            g->d_partials);
                 OFDFT_LAUNCH_CHECK();
-                reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 3 * kChunk, 0ull,
+                reduce_finalize<<<3 * kChunk, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 3 * kChunk, 0ull,
                                                            g->d_results);
                 OFDFT_LAUNCH_CHECK();
                 OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 3 * kChunk * sizeof(double),

@@ -299,10 +299,8 @@ __global__ void k_grad_spectra(const typename Cplx<T>::type* __restrict__ rhoG, 
     const double s2 = sigma > 0.0 ? sigma * sigma / 2.0 : 0.0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < geo.Nc; idx += stride) {
-        const int k = (int)(idx % geo.n2h);
-        const long long t = idx / geo.n2h;
-        const int j = (int)(t % geo.n1);
-        const int i = (int)(t / geo.n1);
+        int i, j, k;
+        half_index(geo, idx, i, j, k);
         const bool edge = k == 0 || (geo.n2 % 2 == 0 && k == geo.n2 / 2);
         double f0 = (double)freq_index(i, geo.n0), f1 = (double)freq_index(j, geo.n1), f2 = (double)k;
         if (edge) {
@@ -341,10 +339,8 @@ __global__ void k_gga_div(const typename Cplx<T>::type* __restrict__ P, typename
     const double s2 = sigma > 0.0 ? sigma * sigma / 2.0 : 0.0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < geo.Nc; idx += stride) {
-        const int k = (int)(idx % geo.n2h);
-        const long long t = idx / geo.n2h;
-        const int j = (int)(t % geo.n1);
-        const int i = (int)(t / geo.n1);
+        int i, j, k;
+        half_index(geo, idx, i, j, k);
         const bool edge = k == 0 || (geo.n2 % 2 == 0 && k == geo.n2 / 2);
         double f0 = (double)freq_index(i, geo.n0), f1 = (double)freq_index(j, geo.n1), f2 = (double)k;
         if (edge) {
@@ -523,7 +519,7 @@ void gga_enqueue(ofdft_grid* g, Scratch& sc, const GgaSpec& sp, const T* rho, T*
     k_gga_point<T><<<g->red_blocks, RED_THREADS, 0, st>>>(rho, D, pot1, g->N, sp, V ? 1 : 0, want_stress ? 1 : 0,
                                                           g->d_partials);
     OFDFT_LAUNCH_CHECK();
-    reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 8, 0ull, out_dev);
+    reduce_finalize<<<8, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 8, 0ull, out_dev);
     OFDFT_LAUNCH_CHECK();
     if (!V) return;
     g->exec_r2c(D, X, np, st);

@@ -37,19 +37,20 @@ const char* cufft_str(cufftResult r) {
 
 __global__ void reduce_finalize(const double* partials, int nblk, int ns, unsigned long long kinds, double* out) {
     __shared__ double sh[RED_THREADS];
-    for (int s = 0; s < ns; ++s) {
-        int kind = (int)((kinds >> (2 * s)) & 3ull);
-        double id = kind == 0 ? 0.0 : (kind == 1 ? INFINITY : -INFINITY);
-        double x = id;
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x) x = red_op(x, partials[(long long)b * ns + s], kind);
-        sh[threadIdx.x] = x;
+    const int s = blockIdx.x;
+    const int kind = (int)((kinds >> (2 * s)) & 3ull);
+    double x = kind == 0 ? 0.0 : (kind == 1 ? INFINITY : -INFINITY);
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) x = red_op(x, partials[(long long)b * ns + s], kind);
+    sh[threadIdx.x] = x;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w >= 32; w >>= 1) {
+        if (threadIdx.x < w) sh[threadIdx.x] = x = red_op(x, sh[threadIdx.x + w], kind);
         __syncthreads();
-        for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) sh[threadIdx.x] = red_op(sh[threadIdx.x], sh[threadIdx.x + w], kind);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[s] = sh[0];
-        __syncthreads();
+    }
+    if (threadIdx.x < 32) {  // the same pairs as a tree in shared memory, without its barriers
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) x = red_op(x, __shfl_down_sync(0xffffffffu, x, w), kind);
+        if (threadIdx.x == 0) out[s] = x;
     }
 }
 

@@ -187,7 +187,7 @@ void gram_t(ofdft_grid* g, const void* const* fields, int nf, double* gram, cuda
         default: gram_launch<T, 9>(g, f, partials, st); break;
     }
     OFDFT_LAUNCH_CHECK();
-    reduce_finalize<<<1, RED_THREADS, 0, st>>>(partials, g->red_blocks, np, 0ull, res);
+    reduce_finalize<<<np, RED_THREADS, 0, st>>>(partials, g->red_blocks, np, 0ull, res);
     OFDFT_LAUNCH_CHECK();
     double tri[kMaxF * (kMaxF + 1) / 2];
     OFDFT_CK(cudaMemcpyAsync(tri, res, np * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -235,10 +235,8 @@ __global__ void k_pme_gather(const double* __restrict__ frac, const int* __restr
 // B(G) = bm0(i) bm1(j) bm2(k) from per-axis complex tables (ewald.py:44-55)
 __device__ inline void barray(const double* bre, const double* bim, const Geo& g, long long idx, double& br,
                               double& bi) {
-    int k = (int)(idx % g.n2h);
-    long long t = idx / g.n2h;
-    int j = (int)(t % g.n1);
-    int i = (int)(t / g.n1);
+    int i, j, k;
+    half_index(g, idx, i, j, k);
     // axis offsets in the packed tables: [0, n0), [n0, n0+n1), [n0+n1, ...)
     double ar = bre[i], ai = bim[i];
     double cr = bre[g.n0 + j], ci = bim[g.n0 + j];

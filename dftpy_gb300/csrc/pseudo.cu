@@ -173,7 +173,7 @@ __global__ void k_pp_grad_moments(const typename Cplx<T>::type* __restrict__ rho
         if (bre) barray(bre, bim, geo, i, br, bi);
         const double qr = (double)QG[i].x, qi = (double)QG[i].y;
         const double sr = qr * br - qi * bi, si = qr * bi + qi * br;
-        const int k2 = (int)(i % geo.n2h);
+        const int k2 = (int)((unsigned)i % (unsigned)geo.n2h);
         const double w = (k2 == 0 || (geo.n2 % 2 == 0 && k2 == geo.n2 / 2)) ? 1.0 : 2.0;
         const double h = scale * w * (sr * (double)rhoG[i].x + si * (double)rhoG[i].y);
         if (q < L.gp1) {
@@ -471,7 +471,7 @@ void forces_t(ofdft_pseudo* p, const T* rho, double* F, cudaStream_t st) {
             k_pp_force_exact<T><<<g->red_blocks, RED_THREADS, 0, st>>>(rhoG, p->lines(), p->d_pos, p->d_spec, a0, na,
                                                                        g->geo, rscale, g->d_partials);
             OFDFT_LAUNCH_CHECK();
-            reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 3 * kForceChunk, 0ull,
+            reduce_finalize<<<3 * kForceChunk, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 3 * kForceChunk, 0ull,
                                                        g->d_results);
             OFDFT_LAUNCH_CHECK();
             OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 3 * kForceChunk * sizeof(double),
@@ -501,7 +501,7 @@ void stress_t(ofdft_pseudo* p, const T* rho, double energy, double* S, cudaStrea
     g->exec_r2c(rho, rhoG, 1, st);
     double sum6[6] = {0, 0, 0, 0, 0, 0};
     auto fetch6 = [&] {
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
+        reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
         OFDFT_LAUNCH_CHECK();
         OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
         OFDFT_CK(cudaStreamSynchronize(st));

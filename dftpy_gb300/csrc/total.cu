@@ -1368,7 +1368,7 @@ void compute_t(ofdft_eval* e, const T* rho, T* V, unsigned calc, double* energie
     OFDFT_LAUNCH_CHECK();
     unsigned long long kinds = (1ull << (2 * 4)) | (2ull << (2 * 5)) | (2ull << (2 * 6));
     timed(e, P_REDUCE, (double)g->red_blocks * PRE_NS * 8, st, [&] {
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, PRE_NS, kinds, g->d_results);
+        reduce_finalize<<<PRE_NS, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, PRE_NS, kinds, g->d_results);
     });
     OFDFT_LAUNCH_CHECK();
     launches += 2;
@@ -1428,7 +1428,7 @@ void compute_t(ofdft_eval* e, const T* rho, T* V, unsigned calc, double* energie
         k_hc_point<T><<<g->red_blocks, RED_THREADS, 0, st>>>(rho, hcD, kfv, hc_c1, hc_c2, N, gga_spec(c),
                                                              g->d_partials);
         OFDFT_LAUNCH_CHECK();
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 2, (1ull << 0) | (2ull << 2),
+        reduce_finalize<<<2, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 2, (1ull << 0) | (2ull << 2),
                                                    g->d_results + 48);
         OFDFT_LAUNCH_CHECK();
         launches += 5;
@@ -1699,7 +1699,7 @@ void compute_t(ofdft_eval* e, const T* rho, T* V, unsigned calc, double* energie
     }
     OFDFT_LAUNCH_CHECK();
     timed(e, P_REDUCE, (double)g->red_blocks * POST_NS * 8, st, [&] {
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, POST_NS, 0ull, g->d_results + 16);
+        reduce_finalize<<<POST_NS, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, POST_NS, 0ull, g->d_results + 16);
     });
     OFDFT_LAUNCH_CHECK();
     launches += 2;
@@ -1931,7 +1931,7 @@ void stress_t(ofdft_eval* e, const T* rho, const double* energies, double* S, cu
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
     const int gblk = blocks_for(g->Nc, 256, g->sms * 16);
     auto fetch = [&](int nblk, int ns) {
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, nblk, ns, 0ull, g->d_results);
+        reduce_finalize<<<ns, RED_THREADS, 0, st>>>(g->d_partials, nblk, ns, 0ull, g->d_results);
         OFDFT_LAUNCH_CHECK();
         OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, ns * sizeof(double), cudaMemcpyDeviceToHost, st));
         OFDFT_CK(cudaStreamSynchronize(st));
