@@ -332,6 +332,7 @@ struct ofdft_grid {
     double* d_partials = nullptr;         // red_blocks * 32 doubles
     double* d_results = nullptr;          // 64 doubles
     double* h_results = nullptr;          // pinned mirror
+    void* fix = nullptr;                  // plans of the integer-pipe transforms (fix_eval.cu)
 
     cufftHandle plan(int dir, int batch);  // dir 0: R2C, 1: C2R
     void exec_r2c(const void* in, void* out, int batch, cudaStream_t s);

@@ -1,0 +1,468 @@
+// Float64 evaluation of TF, vW, LDA, Hartree, the local pseudopotential and the
+// Wang-Teter term with integer-pipe transforms (fix_fft.cuh, fix_3d.cuh).
+//
+// The same quantities as the evaluator's general path (total.cu), arranged for a GPU
+// whose float64 pipe is the bound of everything:
+//   k_pre       every power of rho from one pair of roots and a square root
+//   rows, cols  the forward transforms of rho, sqrt(rho), rho^beta (rho^alpha) in
+//               one launch per axis
+//   k_cols_mul  axis 0 forward, 4 pi/G^2 | G^2/2 | K(G), axis 0 inverse in one launch
+//   k_post      potential and energies, one reciprocal per point
+#include "fix_eval.h"
+
+#include "fix_3d.cuh"
+#include "pointwise.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+using namespace ofdft;
+using namespace ofdft::fix;
+
+namespace {
+
+// The range where float32 seeds hold (also: not zero, negative or NaN).
+__device__ __forceinline__ bool ordinary(double x) { return x > 1e-30 && x < 1e30; }
+
+// 1/x, 1e-30 < |x| < 1e30: a float32 seed y and one cubic Newton step
+// y (1 + e + e^2), e = 1 - x y.  Two conversions and three float64 operations, where
+// the division takes about ten.
+__device__ __forceinline__ double recip(double x) {
+    const double y = (double)__frcp_rn((float)x);
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// c = x^(1/3) and w = x^(-1/3): w from the float32 reciprocal cube root by one
+// Householder step (e = 1 - x w^3, w (1 + e/3 + 2 e^2/9)), c = x w^2 with one Newton
+// correction; 12 float64 operations for both, c within one unit in the last place.
+__device__ __forceinline__ void roots3(double x, double& c, double& w) {
+    if (ordinary(x)) {
+        const double w0 = (double)rcbrtf((float)x);
+        const double e = fma(-(x * w0), w0 * w0, 1.0);
+        w = fma(w0 * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), w0);
+        const double u = w * w, c0 = x * u;
+        c = fma(fma(-(c0 * c0), c0, x) * u, 1.0 / 3.0, c0);
+    } else {
+        c = cbrt(x);
+        w = 1.0 / c;
+    }
+}
+
+struct LdaRoots {
+    double rs, srs, ex, vx;  // cbrt(3/(4 pi)), its square root, exchange prefactors
+};
+
+// Slater exchange + PZ81 correlation (xc/semilocal_xc.py:283-319) from the roots of r:
+// cb = r^(1/3), w = r^(-1/3), sq = sqrt(r); sqrt(Rs) = sqrt(rs) r^(1/2) r^(-2/3)
+__device__ __forceinline__ void lda_roots(double r, double cb, double w, double sq, const LdaRoots& k, double& ex,
+                                          double& vx) {
+    const double tiny = 1e-30;
+    const double a = 0.0311, b = -0.048, c = 0.0020, d = -0.0116, g = -0.1423, b1 = 1.0529, b2 = 0.3334;
+    const double rc = cb < tiny ? tiny : cb;
+    const double Rs = cb < tiny ? k.rs / tiny : k.rs * w;
+    if (Rs < 1.0) {
+        const double lr = log(Rs);
+        ex = k.ex * rc + (a * lr + b + c * Rs * lr + d * Rs);
+        vx = k.vx * rc + (lr * (a + (2.0 / 3) * c * Rs) + b - (1.0 / 3) * a + (1.0 / 3) * (2 * d - c) * Rs);
+    } else {
+        const double sRs = ordinary(r) ? k.srs * (sq * (w * w)) : sqrt(Rs);
+        const double inv = recip(1.0 + b1 * sRs + b2 * Rs);
+        ex = k.ex * rc + g * inv;
+        vx = k.vx * rc + (g + (7.0 / 6.0 * g * b1) * sRs + (4.0 / 3.0 * g * b2) * Rs) * (inv * inv);
+    }
+}
+
+// NS block sums at partials[blockIdx.x * NS + s], a fixed tree per slot
+template <int NS>
+__device__ __forceinline__ void block_sums(double (&v)[NS], double* partials) {
+    block_sum_store<NS>(v, partials);
+}
+
+struct PreK {
+    const double* rho;
+    const double* vloc;
+    double* V;
+    double* sq;
+    double* rb;
+    double* ra;
+    long long N;
+    int tf, xc;
+    int b56, a53;  // beta = 5/6; alpha + beta = 5/3 to rounding
+    double tf_x, alpha, beta, cE, cV;
+    LdaRoots lda;
+};
+
+// Pointwise pre-pass: bound by the float64 pipe (about 70 operations per point with
+// TF, LDA, PP and vW).  rho^(5/6) = rho^(1/2) rho^(1/3) and, when the exponents add up
+// to 5/3, rho^alpha = rho^(5/3) / rho^beta need no pow().
+__global__ void __launch_bounds__(RED_THREADS) k_pre(PreK a, double* partials) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
+        const double r = a.rho[i];
+        double v = 0.0, cb, w;
+        s[3] += r;
+        roots3(r, cb, w);
+        const double c2 = cb * cb, sq = sqrt(r > 0.0 ? r : 1e-30);  // kedf/vw.py:34-44
+        if (a.tf) {
+            s[0] += r * c2 * a.cE;
+            v = a.cV * c2 * a.tf_x;
+        }
+        if (a.xc) {
+            double ex, vx;
+            lda_roots(r, cb, w, sq, a.lda, ex, vx);
+            s[1] += ex * r;
+            v += vx;
+        }
+        if (a.vloc) {
+            const double vl = a.vloc[i];
+            s[2] += vl * r;
+            v += vl;
+        }
+        if (a.sq) a.sq[i] = sq;
+        if (a.rb) {
+            const bool ord = ordinary(r);
+            const double rc = r < kZERO ? kZERO : r;  // wt.py:15-18
+            const double pb = a.b56 && ord ? sq * cb : pow(rc, a.beta);
+            a.rb[i] = pb;
+            if (a.ra) a.ra[i] = a.a53 && ord ? r * c2 / pb : pow(rc, a.alpha);
+        }
+        if (a.V) a.V[i] = v;
+    }
+    block_sums<4>(s, partials);
+}
+
+// Block sums of ns slots into out[0..ns), in a fixed order, and (plan != 0) the
+// Wang-Teter kernel state (wt.py:58-73: rebuilt when rho0 moves by more than 1e-6)
+__global__ void k_sums(const double* __restrict__ partials, int nblk, int ns, double* out, int plan, double* state,
+                       double rho0_fixed, double invN, double alpha, double beta, double cTF) {
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+    __shared__ double sh[4];
+    if (s < ns) {
+        double x = 0.0;
+#pragma unroll 4
+        for (int b = lane; b < nblk; b += 32) x += partials[(long long)b * ns + s];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) out[s] = sh[s] = x;
+    }
+    __syncthreads();
+    if (plan && threadIdx.x == 0) {
+        const double rho0 = rho0_fixed > 0.0 ? rho0_fixed : sh[3] * invN;
+        if (state[4] == 0.0 || fabs(state[0] - rho0) > 1e-6) {
+            state[0] = rho0;
+            state[1] = 1.0;
+            state[2] = 2.0 * pow(3.0 * rho0 * (M_PI * M_PI), 1.0 / 3.0);
+            state[3] = 5.0 / (9.0 * alpha * beta * pow(rho0, alpha + beta - 5.0 / 3.0)) * cTF;
+            state[4] = 1.0;
+        } else {
+            state[1] = 0.0;
+        }
+    }
+}
+
+enum { F_HARTREE = 0, F_VW = 1, F_WT = 2 };
+
+struct MulArgs {
+    ColArgs c;
+    int kind[kMaxFields];
+    Geo geo;
+    double* K;  // Wang-Teter kernel
+    const double* state;
+    double wt_x, invN;
+};
+
+__device__ __noinline__ double wt_build(const MulArgs& a, double gg) {
+    return lindhard_dev(sqrt(gg) / a.state[2], a.wt_x, 1.0) * a.state[3];
+}
+
+// Axis 0 forward, the field's factor, axis 0 inverse.  |G|^2 = A f0^2 + B f0 + C along a
+// line (f0 the axis-0 frequency), so a point pays two operations for it.
+__global__ void __launch_bounds__(kThreads, 3) k_cols_mul(MulArgs a) {
+    extern __shared__ __align__(16) unsigned char fix_smem[];
+    __shared__ LineSm sm;
+    const Plan& p = a.c.g.p0;
+    const int n = p.n, lb = a.c.lb, L = 1 << lb, LP = L + 1;
+    I2* b0 = reinterpret_cast<I2*>(fix_smem);
+    I2* b1 = b0 + n * LP;
+    double2* fq = reinterpret_cast<double2*>(b1 + n * LP);  // f0 and A f0^2
+    const int k1 = blockIdx.x / a.c.ktiles, k2 = (blockIdx.x % a.c.ktiles) * L;
+    const int nl = min(L, a.c.g.n2h - k2), l = threadIdx.x & (L - 1);
+    const long long stride = (long long)a.c.g.n1 * a.c.g.n2h;
+    const long long off = (long long)k1 * a.c.g.n2h + k2;
+    double2* base = a.c.sp[blockIdx.y] + off;
+    const int kind = a.kind[blockIdx.y];
+    const Geo& g = a.geo;
+    const double f1 = (double)freq_index(k1, g.n1) * g.fv[1], f2 = (double)(k2 + l) * g.fv[2];
+    const double ax = g.b[0] * g.fv[0], ay = g.b[1] * g.fv[0], az = g.b[2] * g.fv[0];
+    const double cx = f1 * g.b[3] + f2 * g.b[6], cy = f1 * g.b[4] + f2 * g.b[7], cz = f1 * g.b[5] + f2 * g.b[8];
+    const double A = ax * ax + ay * ay + az * az, B = 2.0 * (ax * cx + ay * cy + az * cz), C = cx * cx + cy * cy + cz * cz;
+    for (int i = threadIdx.x; i < n; i += kThreads) {
+        const double f = (double)freq_index(i, n);
+        fq[i] = make_double2(f, A * f * f);
+    }
+    const I2* z = tile_fft(b0, b1, p, lb, sm, [&](int i, int q) {
+        return q < nl ? base[i * stride + q] : make_double2(0.0, 0.0);
+    });
+    const Scale c = sm.c[l];
+    const int ds = sm.ds[l];
+    __syncthreads();  // every thread has its line's scale before the next transform resets them
+    const bool build = kind == F_WT && a.state[1] != 0.0;
+    const double hart = 4.0 * M_PI * a.invN, half = 0.5 * a.invN;
+    const I2* y = tile_fft(b0, b1, p, lb, sm, [&](int i, int q) {
+        if (q >= nl) return make_double2(0.0, 0.0);
+        double f;
+        if (kind == F_WT) {
+            const long long at = off + i * stride + q;
+            double K;
+            if (build) {
+                const double2 t = fq[i];
+                K = wt_build(a, fma(t.x, B, t.y) + C);
+                a.K[at] = K;
+            } else {
+                K = a.K[at];
+            }
+            f = K * a.invN;
+        } else {
+            const double2 t = fq[i];
+            const double gg = fma(t.x, B, t.y) + C;
+            if (kind == F_VW) f = gg * half;
+            else f = i == 0 && off + q == 0 ? 0.0 : (ordinary(gg) ? recip(gg) : 1.0 / gg) * hart;
+        }
+        const I2 v = z[i * LP + q];
+        return make_double2(to_dbl(v.y, c, ds) * f, to_dbl(v.x, c, ds) * f);
+    });
+    for (int e = threadIdx.x; e < n * L; e += kThreads) {
+        const int q = e & (L - 1), i = e >> lb;
+        if (q >= nl) continue;
+        const Scale d = sm.c[q];
+        const I2 v = y[i * LP + q];
+        base[i * stride + q] = make_double2(to_dbl(v.y, d, sm.ds[q]), to_dbl(v.x, d, sm.ds[q]));
+    }
+}
+
+struct PostK {
+    const double* rho;
+    double* V;
+    const double* sq;
+    const double* lap;
+    const double* vH;
+    const double* nl1;
+    const double* nl2;
+    const double* rb;
+    const double* ra;
+    long long N;
+    double vw_y, alpha, beta, half_alpha;  // 0.5 / alpha
+};
+
+// Pointwise post-pass: vW and Hartree potentials, the Wang-Teter potential
+// (wt.py:19-23, 44-56, 124-132) and their energies
+__global__ void __launch_bounds__(RED_THREADS) k_post(PostK a, double* partials) {
+    double s[3] = {0.0, 0.0, 0.0};
+    const double tiny = 1e-30;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
+        const double r = a.rho[i];
+        const bool ord = ordinary(r);
+        const double ri = ord ? recip(r) : 1.0 / (r < kZERO ? kZERO : r);
+        double v = a.V ? a.V[i] : 0.0;
+        if (a.lap) {
+            double q = a.sq[i];
+            if (fabs(q) < tiny) q = tiny;
+            const double pw = a.lap[i] * (ord ? q * ri : 1.0 / q);
+            if (r > 0.0) s[0] += r * pw;
+            v += pw * a.vw_y;
+        }
+        if (a.vH) {
+            const double vh = a.vH[i];
+            s[1] += vh * r;
+            v += vh;
+        }
+        if (a.nl1) {
+            const double pb = a.rb[i], c1 = a.nl1[i];
+            if (!a.ra) {
+                const double pot = 2.0 * a.alpha * (pb * ri) * c1;
+                if (a.V) s[2] += pot * r * a.half_alpha;
+                else s[2] += c1 * pb;
+                v += pot;
+            } else {
+                const double pa = a.ra[i];
+                s[2] += c1 * pa;
+                if (a.V) v += a.alpha * (pa * ri) * c1 + a.beta * (pb * ri) * a.nl2[i];
+            }
+        }
+        if (a.V) a.V[i] = v;
+    }
+    block_sums<3>(s, partials);
+}
+
+}  // namespace
+
+namespace ofdft {
+namespace fix {
+
+struct GridPlans {
+    Grid3 g;
+    I2* tw = nullptr;
+    bool ok = false;
+};
+
+const Grid3* grid_plans(ofdft_grid* g) {
+    if (g->prec != OFDFT_F64) return nullptr;
+    if (!g->fix) {
+        GridPlans* h = new GridPlans();
+        g->fix = h;
+        h->g.n0 = g->nr[0];
+        h->g.n1 = g->nr[1];
+        h->g.n2 = g->nr[2];
+        h->g.n2h = g->n2h;
+        Plan* p[3] = {&h->g.p0, &h->g.p1, &h->g.p2};
+        bool ok = true;
+        size_t total = 0;
+        for (int d = 0; d < 3; ++d) {
+            ok = ok && g->nr[d] <= kMaxAxis && plan_radices(g->nr[d], *p[d]);
+            total += (size_t)g->nr[d];
+        }
+        if (ok) {
+            // twiddles at scale 2^61 from long double trigonometry
+            std::vector<I2> tw(total);
+            size_t off = 0;
+            const long double pi = 3.14159265358979323846264338327950288L;
+            for (int d = 0; d < 3; ++d) {
+                const int n = g->nr[d];
+                for (int k = 0; k < n; ++k) {
+                    const long double t = -2.0L * pi * (long double)k / (long double)n;
+                    tw[off + k] = I2{(long long)std::llroundl(std::cos(t) * (long double)kOne),
+                                     (long long)std::llroundl(std::sin(t) * (long double)kOne)};
+                }
+                off += n;
+            }
+            OFDFT_CK(cudaMalloc(&h->tw, total * sizeof(I2)));
+            upload_now(h->tw, tw.data(), total * sizeof(I2));
+            off = 0;
+            for (int d = 0; d < 3; ++d) {
+                p[d]->tw = h->tw + off;
+                off += g->nr[d];
+            }
+            h->ok = true;
+        }
+    }
+    const GridPlans* h = static_cast<const GridPlans*>(g->fix);
+    return h->ok ? &h->g : nullptr;
+}
+
+void free_plans(ofdft_grid* g) {
+    GridPlans* h = static_cast<GridPlans*>(g->fix);
+    if (!h) return;
+    if (h->tw) cudaFree(h->tw);
+    delete h;
+    g->fix = nullptr;
+}
+
+void r2c(ofdft_grid* g, const double* const* in, double2* const* out, int nf, cudaStream_t st) {
+    const Grid3& p = *grid_plans(g);
+    rows_r2c(p, g->sms, in, out, nf, st);
+    cols<1>(p, g->sms, out, nf, false, st);
+    cols<0>(p, g->sms, out, nf, false, st);
+}
+
+void c2r(ofdft_grid* g, double2* const* in, double* const* out, int nf, cudaStream_t st) {
+    const Grid3& p = *grid_plans(g);
+    cols<0>(p, g->sms, in, nf, true, st);
+    cols<1>(p, g->sms, in, nf, true, st);
+    rows_c2r(p, g->sms, in, out, nf, st);
+}
+
+int local_enqueue(ofdft_grid* g, Scratch& sc, const LocalArgs& a, cudaStream_t st) {
+    const Grid3& p = *grid_plans(g);
+    const long long N = g->N;
+    const size_t rb = g->real_bytes(), cb = g->cplx_bytes();
+    const int sms = g->sms;
+    const bool same = std::fabs(a.wt_beta - a.wt_alpha) < 1e-9;
+    double* sq = a.vw ? (double*)sc.get("sq", rb) : nullptr;
+    double* rbp = a.wt ? (double*)sc.get("rb", rb) : nullptr;
+    double* rap = a.wt && !same ? (double*)sc.get("ra", rb) : nullptr;
+    const int blocks = (int)std::max(1LL, std::min((long long)sms * 8, (N + RED_THREADS - 1) / RED_THREADS));
+    double* part = (double*)sc.get("fix_part", (size_t)blocks * 4 * sizeof(double));
+    const Consts k = make_consts();
+
+    PreK pk{};
+    pk.rho = a.rho;
+    pk.vloc = a.vloc;
+    pk.V = a.V;
+    pk.sq = sq;
+    pk.rb = rbp;
+    pk.ra = rap;
+    pk.N = N;
+    pk.tf = a.tf;
+    pk.xc = a.xc;
+    pk.b56 = a.wt_beta == 5.0 / 6.0;
+    pk.a53 = std::fabs(a.wt_alpha + a.wt_beta - 5.0 / 3.0) < 4e-16;
+    pk.tf_x = a.tf_x;
+    pk.alpha = a.wt_alpha;
+    pk.beta = a.wt_beta;
+    pk.cE = k.cTF_E;
+    pk.cV = k.cTF_V;
+    pk.lda = LdaRoots{k.lda_rs, std::sqrt(k.lda_rs), k.lda_ex, k.lda_vx};
+    k_pre<<<blocks, RED_THREADS, 0, st>>>(pk, part);
+    OFDFT_LAUNCH_CHECK();
+    k_sums<<<1, 128, 0, st>>>(part, blocks, 4, g->d_results, a.wt, a.wtstate, a.wt_rho0, 1.0 / (double)N, a.wt_alpha,
+                              a.wt_beta, a.cTF_wt);
+    OFDFT_LAUNCH_CHECK();
+    int launches = 4;
+
+    // fields to transform, their factors and what they become
+    const double* in[4];
+    double2* sp[4];
+    double* out[4];
+    MulArgs m{};
+    int nf = 0;
+    auto field = [&](const double* src, const char* spec, const char* real, int kind) {
+        in[nf] = src;
+        sp[nf] = (double2*)sc.get(spec, cb);
+        out[nf] = (double*)sc.get(real, rb);
+        m.kind[nf] = kind;
+        return out[nf++];
+    };
+    PostK q{};
+    if (a.h) q.vH = field(a.rho, "rhoG", "vH", F_HARTREE);
+    if (a.vw) q.lap = field(sq, "sqG", "lap", F_VW);
+    if (a.wt) q.nl1 = field(rbp, "rbG", "nl1", F_WT);
+    if (rap) q.nl2 = field(rap, "raG", "nl2", F_WT);
+    if (nf > 0) {
+        rows_r2c(p, sms, in, sp, nf, st);
+        cols<1>(p, sms, sp, nf, false, st);
+        m.c = col_args(p, 0, sms);
+        for (int f = 0; f < nf; ++f) m.c.sp[f] = sp[f];
+        m.geo = g->geo;
+        m.K = a.wtK;
+        m.state = a.wtstate;
+        m.wt_x = a.wt_x;
+        m.invN = 1.0 / (double)N;
+        const size_t smem = tile_smem(p.p0, 1 << m.c.lb) + (size_t)p.n0 * sizeof(double2);
+        smem_optin(k_cols_mul, smem);
+        k_cols_mul<<<dim3(col_blocks(m.c, 0), nf), kThreads, smem, st>>>(m);
+        OFDFT_LAUNCH_CHECK();
+        cols<1>(p, sms, sp, nf, true, st);
+        rows_c2r(p, sms, sp, out, nf, st);
+        launches += 5;
+    }
+    q.rho = a.rho;
+    q.V = a.V;
+    q.sq = sq;
+    q.rb = rbp;
+    q.ra = rap;
+    q.N = N;
+    q.vw_y = a.vw_y;
+    q.alpha = a.wt_alpha;
+    q.beta = a.wt_beta;
+    q.half_alpha = 0.5 / a.wt_alpha;
+    k_post<<<blocks, RED_THREADS, 0, st>>>(q, part);
+    OFDFT_LAUNCH_CHECK();
+    k_sums<<<1, 128, 0, st>>>(part, blocks, 3, g->d_results + 16, 0, nullptr, 0.0, 0.0, 0.0, 0.0, 0.0);
+    OFDFT_LAUNCH_CHECK();
+    return launches;
+}
+
+}  // namespace fix
+}  // namespace ofdft

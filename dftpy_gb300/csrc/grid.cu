@@ -1,6 +1,7 @@
 // Grid handle, cuFFT plans, DirectField.fft / ReciprocalField.ifft and
 // float64 field reductions of the C ABI.
 #include "common.cuh"
+#include "fix_eval.h"
 
 #include <algorithm>
 
@@ -221,6 +222,7 @@ int ofdft_grid_create(const int nr[3], const double lattice[9], int precision, o
 void ofdft_grid_destroy(ofdft_grid* g) {
     if (!g) return;
     for (auto& kv : g->plans) cufftDestroy(kv.second);
+    fix::free_plans(g);
     g->scratch.release_all();
     if (g->d_partials) cudaFree(g->d_partials);
     if (g->d_results) cudaFree(g->d_results);

@@ -403,6 +403,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_dot2(long long n, const T* a, c
 
 // grid of an evaluator (the evaluator struct lives in total.cu)
 ofdft_grid* e_grid(ofdft_eval* e);
+// the general evaluation path (total.cu)
+void eval_general(ofdft_eval* e, const void* rho, void* v_out, unsigned calc, double* energies, cudaStream_t st);
 // an evaluation enqueued without waiting, and its energies after a synchronisation (total.cu)
 void eval_enqueue(ofdft_eval* e, const void* rho, void* v_out, unsigned calc, cudaStream_t st);
 void eval_collect(ofdft_eval* e, double* energies);
@@ -451,8 +453,7 @@ struct Opt {
     void copy(T* out, const T* in) { OFDFT_CK(cudaMemcpyAsync(out, in, g->real_bytes(), cudaMemcpyDeviceToDevice, st)); }
     double eval(const T* rho, T* V, unsigned calc) {
         double E[OFDFT_NE];
-        int rc = ofdft_eval_compute(e, rho, V, calc, E, st);
-        if (rc != OFDFT_OK) throw Error{rc};
+        eval_general(e, rho, V, calc, E, st);
         return E[OFDFT_E_TOTAL];
     }
     // OrthogonalNormalization (optimization.py:205-226): p -= (p.phi/Ne) phi; |p|^2 = Ne

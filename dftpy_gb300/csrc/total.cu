@@ -17,6 +17,7 @@
 #include "common.cuh"
 #include "pointwise.cuh"
 #include "gga.cuh"
+#include "fix_eval.h"
 #include "host_math.h"
 
 #include <algorithm>
@@ -835,6 +836,14 @@ void eval_enqueue(ofdft_eval* e, const void* rho, void* v_out, unsigned calc, cu
     else compute_t<float>(e, (const float*)rho, (float*)v_out, calc, nullptr, st);
 }
 void eval_collect(ofdft_eval* e, double* energies) { collect_energies(e, energies); }
+// For the optimiser: the general path whatever the configuration.  A trajectory
+// amplifies the rounding of its potentials (by about 1e7 over six L-BFGS iterations
+// from a smooth density: the preconditionerless steps grow the highest |G|), so the
+// optimisers keep one evaluation, the batched one included.
+void eval_general(ofdft_eval* e, const void* rho, void* v_out, unsigned calc, double* energies, cudaStream_t st) {
+    if (e->g->prec == OFDFT_F64) compute_t<double>(e, (const double*)rho, (double*)v_out, calc, energies, st);
+    else compute_t<float>(e, (const float*)rho, (float*)v_out, calc, energies, st);
+}
 // an evaluation that waits on the host mid-way (the k_F-node kernel reads its
 // k_F bounds back) cannot be captured into a CUDA graph
 bool eval_capturable(const ofdft_eval* e) { return !(e->cfg.kedf_terms & OFDFT_KE_LWT); }
@@ -1775,6 +1784,57 @@ void collect_energies(ofdft_eval* e, double* energies) {
     e->last_launches = p.launches;
 }
 
+// Whether ofdft_eval_compute takes the float64 evaluation on integer-pipe transforms
+// (fix_eval.cu): TF, vW, LDA, Hartree, PP and the Wang-Teter kernel without smoothing
+// or corrections, on axes the plans cover.  It is 2 to 8 times faster than the general
+// path, whose float64 transforms and powers saturate the slow float64 pipe.
+bool fix_applies(ofdft_eval* e) {
+    const ofdft_config& c = e->cfg;
+    const int known = OFDFT_KE_TF | OFDFT_KE_VW | OFDFT_KE_WT;
+    return e->g->prec == OFDFT_F64 && !(c.kedf_terms & ~known) && !(c.vw_sigma > 0.0) && !c.wte && !c.external &&
+           !((c.kedf_terms & OFDFT_KE_WT) && c.wt_kernel != OFDFT_LWT_KERNEL_WT) && !e->prof &&
+           fix::grid_plans(e->g) != nullptr;
+}
+
+void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, double* energies, cudaStream_t st) {
+    ofdft_grid* g = e->g;
+    const ofdft_config& c = e->cfg;
+    const bool wantV = (calc & OFDFT_CALC_V) != 0;
+    OFDFT_REQUIRE(!(c.pseudo && !e->have_vloc), "ofdft_eval_compute: pseudo enabled but no v_loc set");
+    OFDFT_REQUIRE(!(wantV && !V), "ofdft_eval_compute: V requested but v_out is NULL");
+    const bool wt = c.kedf_terms & OFDFT_KE_WT;
+    fix::LocalArgs a{};
+    a.rho = rho;
+    a.vloc = c.pseudo ? (const double*)e->vloc : nullptr;
+    a.V = wantV ? V : nullptr;
+    a.tf = (c.kedf_terms & OFDFT_KE_TF) != 0;
+    a.vw = (c.kedf_terms & OFDFT_KE_VW) != 0;
+    a.wt = wt;
+    a.xc = c.xc_lda != 0;
+    a.h = c.hartree != 0;
+    a.tf_x = c.tf_x;
+    a.vw_y = c.vw_y;
+    a.wt_alpha = c.wt_alpha;
+    a.wt_beta = c.wt_beta;
+    a.wt_x = c.wt_x;
+    a.wt_rho0 = c.wt_rho0;
+    a.wtstate = e->wtstate;
+    a.wtK = wt ? (double*)e->sc.get("wtK", (size_t)g->Nc * sizeof(double)) : nullptr;
+    a.cTF_wt = e->k.cTF_wt;
+    const int launches = fix::local_enqueue(g, e->sc, a, st);
+    OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 24 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    e->pend = {};
+    e->pend.tf = a.tf;
+    e->pend.vw = a.vw;
+    e->pend.wt = wt;
+    e->pend.xc = a.xc;
+    e->pend.h = a.h;
+    e->pend.pp = a.vloc != nullptr;
+    e->pend.launches = launches;
+    OFDFT_CK(cudaStreamSynchronize(st));
+    collect_energies(e, energies);
+}
+
 // ------------------------------------------------------------------ stress
 // Stress tensors of the evaluator's terms (TotalFunctional.get_stress,
 // total_functional.py:176-208): TF (kedf/tf.py:52-63), vW (kedf/vw.py:97-111),
@@ -2224,7 +2284,9 @@ int ofdft_eval_compute(ofdft_eval* e, const void* rho, void* v_out, unsigned cal
     return guard([&] {
         OFDFT_REQUIRE(e && rho && energies, "ofdft_eval_compute: null argument");
         OFDFT_REQUIRE(calc & (OFDFT_CALC_E | OFDFT_CALC_V), "ofdft_eval_compute: calc must include E or V");
-        if (e->g->prec == OFDFT_F64)
+        if (fix_applies(e))
+            fix_compute(e, (const double*)rho, (double*)v_out, calc, energies, (cudaStream_t)s);
+        else if (e->g->prec == OFDFT_F64)
             compute_t<double>(e, (const double*)rho, (double*)v_out, calc, energies, (cudaStream_t)s);
         else
             compute_t<float>(e, (const float*)rho, (float*)v_out, calc, energies, (cudaStream_t)s);
