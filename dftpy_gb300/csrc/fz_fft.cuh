@@ -190,6 +190,15 @@ __device__ __forceinline__ void line_fft(float2 (&v)[E], float2* sm, Idx ix, int
     Stockham<N, E, S, 1, Idx>::run(v, sm, ix, t, tw);
 }
 
+// Who exchanges through a row's buffers: the block, or (rows that lie within a warp) the
+// warp, whose barrier costs a few cycles and couples nothing else.
+struct BlockSync {
+    __device__ __forceinline__ static void run() { __syncthreads(); }
+};
+struct WarpSync {
+    __device__ __forceinline__ static void run() { __syncwarp(); }
+};
+
 // Row placement: one pad slot per 16 elements.  With 8 points per thread the
 // loads of every pass (16 consecutive elements per half-warp) and the stores
 // of the first radix-8 pass fall in distinct banks; the second radix-8 pass of
@@ -219,7 +228,7 @@ struct RowLayout {
 // one barrier instead of two.  Entry: buffer 0 is free.  Exit: both buffers are
 // free for the next transform (a trailing barrier is added when the number of
 // exchanges is odd, because the last reads then come from buffer 0).
-template <int N, int E, int S, int NS, int PASS, class Idx>
+template <int N, int E, int S, int NS, int PASS, class Idx, class Sync>
 struct StockhamPP {
     static constexpr int T = N / E;
     static constexpr int R = PassRadix<N, E, NS>::R;
@@ -232,7 +241,7 @@ struct StockhamPP {
         __builtin_assume(t >= 0 && t < T);
         if constexpr (NS > 1) {
             const float2* src = ((PASS - 1) & 1) ? b1 : b0;
-            __syncthreads();  // the previous pass's outputs are in src
+            Sync::run();  // the previous pass's outputs are in src
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = src[ix(t + T * e)];
         }
@@ -262,9 +271,9 @@ struct StockhamPP {
             }
         }
         if constexpr (!LAST) {
-            StockhamPP<N, E, S, NS * R, PASS + 1, Idx>::run(v, b0, b1, ix, t, tw);
+            StockhamPP<N, E, S, NS * R, PASS + 1, Idx, Sync>::run(v, b0, b1, ix, t, tw);
         } else if constexpr ((PASS & 1) == 1) {
-            __syncthreads();  // odd number of exchanges: the last reads were from buffer 0
+            Sync::run();  // odd number of exchanges: the last reads were from buffer 0
         }
     }
 };
@@ -314,7 +323,7 @@ __device__ __forceinline__ void tw_load(float2 (&w)[tw_count<N, E>()], int t, co
 // The Stockham passes with register twiddles (OFF: this pass's first twiddle)
 // and one exchange buffer (PP false: two barriers per exchange) or two used in
 // turn (PP true: one barrier per exchange, as StockhamPP).
-template <int N, int E, int S, int NS, int PASS, int OFF, bool PP, class Idx, class Idx1 = Idx>
+template <int N, int E, int S, int NS, int PASS, int OFF, bool PP, class Sync, class Idx, class Idx1 = Idx>
 struct StockhamR {
     static constexpr int T = N / E;
     static constexpr int R = PassRadix<N, E, NS>::R;
@@ -338,10 +347,10 @@ struct StockhamR {
         const float2* src = SB ? b1 : b0;
         float2* dst = DB ? b1 : b0;
         if constexpr (NS > 1) {
-            __syncthreads();  // the previous pass's outputs are in src
+            Sync::run();  // the previous pass's outputs are in src
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = src[at<SB>(ix, ix1, t + T * e)];
-            if constexpr (!PP && !LAST) __syncthreads();  // every input read before the buffer is overwritten
+            if constexpr (!PP && !LAST) Sync::run();  // every input read before the buffer is overwritten
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
@@ -368,9 +377,9 @@ struct StockhamR {
             }
         }
         if constexpr (!LAST) {
-            StockhamR<N, E, S, NS * R, PASS + 1, OFF + HERE, PP, Idx, Idx1>::run(v, b0, b1, ix, t, w, ix1);
+            StockhamR<N, E, S, NS * R, PASS + 1, OFF + HERE, PP, Sync, Idx, Idx1>::run(v, b0, b1, ix, t, w, ix1);
         } else if constexpr (PP && (PASS & 1) == 1) {
-            __syncthreads();  // odd number of exchanges: the last reads were from buffer 0
+            Sync::run();  // odd number of exchanges: the last reads were from buffer 0
         }
     }
 };
@@ -378,14 +387,14 @@ struct StockhamR {
 // single exchange buffer `sm`, free on entry; the last pass has read it on return
 template <int N, int E, int S, class Idx>
 __device__ __forceinline__ void line_fft_r(float2 (&v)[E], float2* sm, Idx ix, int t, const float2* w) {
-    StockhamR<N, E, S, 1, 0, 0, false, Idx>::run(v, sm, sm, ix, t, w);
+    StockhamR<N, E, S, 1, 0, 0, false, BlockSync, Idx>::run(v, sm, sm, ix, t, w);
 }
 // two exchange buffers used in turn (entry: b0 free; exit: both free), laid out
 // by ix and ix1
-template <int N, int E, int S, class Idx, class Idx1>
+template <int N, int E, int S, class Sync = BlockSync, class Idx, class Idx1>
 __device__ __forceinline__ void line_fft_ppr(float2 (&v)[E], float2* b0, float2* b1, Idx ix, Idx1 ix1, int t,
                                              const float2* w) {
-    StockhamR<N, E, S, 1, 0, 0, true, Idx, Idx1>::run(v, b0, b1, ix, t, w, ix1);
+    StockhamR<N, E, S, 1, 0, 0, true, Sync, Idx, Idx1>::run(v, b0, b1, ix, t, w, ix1);
 }
 
 // ---- 1-D bulk asynchronous copies (TMA) into shared memory, completed on an
@@ -442,10 +451,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     }
 }
 
-template <int N, int E, int S, class Idx>
+template <int N, int E, int S, class Sync = BlockSync, class Idx>
 __device__ __forceinline__ void line_fft_pp(float2 (&v)[E], float2* b0, float2* b1, Idx ix, int t,
                                             const float2* __restrict__ tw) {
-    StockhamPP<N, E, S, 1, 0, Idx>::run(v, b0, b1, ix, t, tw);
+    StockhamPP<N, E, S, 1, 0, Idx, Sync>::run(v, b0, b1, ix, t, tw);
 }
 
 }  // namespace fz

@@ -11,7 +11,8 @@
 // with the Hermite basis weights W_j, WD_j (fz_hermite_w)
 // with the node kernel, the interpolation and the hat weights folded into
 // hand-written tile FFTs, so the node planes cross HBM three times each
-// instead of five and no real-space plane is stored:
+// instead of five and no real-space plane is stored.  Rows that no point ties to a
+// node are left out of that node's planes after axis 1 (FzNeed):
 //   C2R: k_fz_nodes    axis 0 inverse, K_j and K'_j applied on load
 //        k_fz_axis1    axis 1 inverse
 //        k_fz_c2r_rows axis 2 C2R, interpolated into pot1/pot3 per point
@@ -50,6 +51,7 @@ constexpr int kFzLines = 16;  // lines per column tile
 constexpr int kFzColE = 16;   // points per thread along a column
 constexpr int kFzRowE = 8;    // complex points per thread along a row
 constexpr int kFzRowThreads = 256;
+constexpr int kFzMaxBatch = 256;  // nodes per batch (their reciprocals, and lists of them, sit in shared memory)
 
 // float32 copy of the kernel-table parameters
 struct FzTab {
@@ -240,38 +242,73 @@ __global__ void __launch_bounds__(kFzLines * (N0 / kFzColE), 2)
     }
 }
 
-// Axis-1 transform of every plane, in place.  Main tiles: (i0, 16 consecutive
-// k2) with lines across threads; Nyquist tiles: 16 consecutive i0, whose lines
-// are contiguous, with the points of a line across threads.
+// Which rows need which nodes.  A point takes part in the two nodes of its k_F interval
+// only, and along one row (i0, i1) a density crosses about half of the nodes: the C2R
+// chain computes, stores and reads the other rows of a node's plane for nothing, and the
+// R2C chain's are zero.  need[(i0 m + j) n1/32 + w] holds a bit per i1 of node j's plane:
+// 256^3 with 64 nodes: 0.41 to 0.50 of the rows for densities spread over the node range.
+struct FzNeed {
+    const unsigned* bits;
+    int m, words;  // nodes, n1 / 32
+    __device__ __forceinline__ const unsigned* of(int i0, int j) const {
+        return bits + ((long long)i0 * m + j) * words;
+    }
+};
+
+// Axis-1 transform of every plane, in place; plane p belongs to node j0 + p % nb.  The
+// inverse stores, and the forward transform reads, only the rows that their node needs
+// (the others count as zero).  Main tiles: (i0, 16 consecutive k2) with lines across
+// threads; Nyquist tiles: 16 consecutive i0, whose lines are contiguous, with the points
+// of a line across threads.
 template <int N1, int S>
 __global__ void __launch_bounds__(kFzLines * (N1 / kFzColE))
-    k_fz_axis1(float2* __restrict__ XY, FzDims d, const float2* __restrict__ tw) {
+    k_fz_axis1(float2* __restrict__ XY, FzDims d, const float2* __restrict__ tw, FzNeed need, int j0, int nb) {
     constexpr int E = kFzColE, T = N1 / E;
     extern __shared__ float2 fz_sm[];
     const int per_row = d.H / kFzLines;
     const int tiles_main = d.n0 * per_row;
     const int tiles = tiles_main + d.n0 / kFzLines;
     const int p = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+    const int j = j0 + p % nb;
     float2* base = XY + (long long)p * d.plane;
     float2 v[E];
+    // bit t + T e of the line's node, for the thread's elements e
+    auto mine = [&](int i0, int t) {
+        const unsigned* w = need.of(i0, j);
+        unsigned b = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int i1 = t + T * e;
+            b |= ((__ldg(w + (i1 >> 5)) >> (i1 & 31)) & 1u) << e;
+        }
+        return b;
+    };
     if (tile < tiles_main) {
         const int l = threadIdx.x % kFzLines, t = threadIdx.x / kFzLines;
         const int i0 = tile / per_row, k2 = (tile % per_row) * kFzLines + l;
         float2* line = base + (long long)i0 * N1 * d.H + k2;
+        unsigned on = S < 0 ? mine(i0, t) : 0u;
 #pragma unroll
-        for (int e = 0; e < E; ++e) v[e] = __ldcs(line + (long long)(t + T * e) * d.H);
+        for (int e = 0; e < E; ++e)
+            v[e] = S > 0 || (on >> e & 1u) ? __ldcs(line + (long long)(t + T * e) * d.H) : make_float2(0.0f, 0.0f);
         fz::line_fft<N1, E, S>(v, fz_sm + l, fz::ColIdx(), t, tw);
+        if (S > 0) on = mine(i0, t);
 #pragma unroll
-        for (int e = 0; e < E; ++e) __stcs(line + (long long)(t + T * e) * d.H, v[e]);
+        for (int e = 0; e < E; ++e)
+            if (S < 0 || (on >> e & 1u)) __stcs(line + (long long)(t + T * e) * d.H, v[e]);
     } else {
         const int t = threadIdx.x % T, l = threadIdx.x / T;
         const int i0 = (tile - tiles_main) * kFzLines + l;
         float2* line = base + d.nyq + (long long)i0 * N1;
+        unsigned on = S < 0 ? mine(i0, t) : 0u;
 #pragma unroll
-        for (int e = 0; e < E; ++e) v[e] = __ldcs(line + t + T * e);
+        for (int e = 0; e < E; ++e)
+            v[e] = S > 0 || (on >> e & 1u) ? __ldcs(line + t + T * e) : make_float2(0.0f, 0.0f);
         fz::line_fft<N1, E, S>(v, fz_sm + l * fz::row_slots(N1), fz::RowIdx(), t, tw);
+        if (S > 0) on = mine(i0, t);
 #pragma unroll
-        for (int e = 0; e < E; ++e) __stcs(line + t + T * e, v[e]);
+        for (int e = 0; e < E; ++e)
+            if (S < 0 || (on >> e & 1u)) __stcs(line + t + T * e, v[e]);
     }
 }
 
@@ -288,6 +325,7 @@ struct FzRowArgs {
     FzDims d;
     FzTw tw;
     unsigned* err;  // set to 1 when a copy into shared memory did not complete in time
+    FzNeed need;    // rows of each node
 };
 
 // Node bounds of the interval search in float32, staged per block (6 m floats):
@@ -406,12 +444,73 @@ __device__ __forceinline__ float fz_hat(float jf, float fi, float tr) {
     return fmaxf(0.0f, 1.0f - fabsf((jf - fi) - tr));
 }
 
-// Row l of a staged block (ROWS rows of H complex, then their ROWS Nyquist
-// values) pre-processed for the half-length complex C2R:
+// The need bits of 32 rows (one i0, one word of i1): a warp walks its rows, every lane
+// collects the nodes of its points, and lane q enters bit i1 for nodes q and q + 32 (nodes
+// from 64 on are entered point by point).  m <= kFzMaxNodes.
+__global__ void __launch_bounds__(kFzRowThreads) k_fz_need(FzRowArgs a, unsigned* __restrict__ out) {
+    extern __shared__ float fz_need_sm[];
+    const FzNodeSm nodes = fz_stage_nodes(a, fz_need_sm);
+    unsigned* bits = reinterpret_cast<unsigned*>(fz_need_sm + 6 * a.m);
+    const int words = a.need.words, i0 = blockIdx.x / words, word = blockIdx.x % words;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int q = threadIdx.x; q < a.m; q += blockDim.x) bits[q] = 0;
+    __syncthreads();
+    const float clipdn = __double2float_rd(a.kfclip);
+    const int n1 = a.d.n1, n2 = a.d.n2;
+    for (int r = warp; r < 32; r += kFzRowThreads / 32) {
+        const float* row = a.kf + ((long long)i0 * n1 + word * 32 + r) * n2;
+        const unsigned bit = 1u << r;
+        unsigned lo = 0, hi = 0;  // nodes below 64
+        for (int i = lane; i < n2; i += 32) {
+            const float kf = __ldg(row + i);
+            float fi, tr;
+            fz_interval_state(kf, a, nodes, clipdn, fi, tr);
+            const int il = (int)fi;
+            if (il >= 0) {
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int j = il + s;
+                    if (j < 32) lo |= 1u << j;
+                    else if (j < 64) hi |= 1u << (j - 32);
+                    else if (j < a.m) atomicOr(bits + j, bit);
+                }
+            }
+            if (kf < nodes.kupu[0]) lo |= 1u;  // the small-k_F branch of node 0
+        }
+        lo = __reduce_or_sync(0xffffffffu, lo);
+        hi = __reduce_or_sync(0xffffffffu, hi);
+        if ((lo >> lane & 1u) && lane < a.m) atomicOr(bits + lane, bit);
+        if ((hi >> lane & 1u) && lane + 32 < a.m) atomicOr(bits + lane + 32, bit);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < a.m; q += blockDim.x) out[((long long)i0 * a.m + q) * words + word] = bits[q];
+}
+inline size_t fz_need_smem(int m) { return (size_t)m * (6 * sizeof(float) + sizeof(unsigned)); }
+
+// The nodes of the batch that the warp's rows [row0, row0 + rows) need, in order, as a list
+// in shared memory; returns their number.  All lanes of the warp call it.
+__device__ __forceinline__ int fz_need_list(const FzRowArgs& a, long long row0, int rows, unsigned char* list) {
+    const int lane = threadIdx.x & 31;
+    const int i0 = (int)(row0 / a.d.n1), i1 = (int)(row0 % a.d.n1);  // rows divides n1
+    const unsigned mask = (rows < 32 ? (1u << rows) - 1u : 0xffffffffu) << (i1 & 31);
+    int n = 0;
+    for (int q0 = 0; q0 < a.nb; q0 += 32) {
+        const int q = q0 + lane;
+        const bool on = q < a.nb && (__ldg(a.need.of(i0, a.j0 + q) + (i1 >> 5)) & mask);
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        if (on) list[n + __popc(b & ((1u << lane) - 1u))] = (unsigned char)q;
+        n += __popc(b);
+    }
+    __syncwarp();
+    return n;
+}
+
+// Row l of a warp's stage (ROWS rows of H complex, then their Nyquist values from
+// slot nyq on) pre-processed for the half-length complex C2R:
 // Z[k] = (X[k] + conj X[H-k]) + i w^k (X[k] - conj X[H-k]), w = exp(+2 pi i/n2),
 // the imaginary parts of X[0] and X[H] dropped.
-template <int H, int ROWS = kFzRowThreads / (H / kFzRowE)>
-__device__ __forceinline__ void fz_c2r_pre(const float2* st, int l, int t, const float2* __restrict__ twr,
+template <int H>
+__device__ __forceinline__ void fz_c2r_pre(const float2* st, int l, int nyq, int t, const float2* __restrict__ twr,
                                            float2 (&v)[kFzRowE]) {
     constexpr int E = kFzRowE, T = H / E;
     const float2* r = st + l * H;
@@ -421,7 +520,7 @@ __device__ __forceinline__ void fz_c2r_pre(const float2* st, int l, int t, const
         float2 X = r[k];
         float2 Y = r[(H - k) & (H - 1)];
         if (e == 0 && k == 0) {
-            Y = st[ROWS * H + l];
+            Y = st[nyq + l];
             X.y = 0.0f;
             Y.y = 0.0f;
         }
@@ -432,64 +531,77 @@ __device__ __forceinline__ void fz_c2r_pre(const float2* st, int l, int t, const
     }
 }
 
+// A warp's share of the row passes: rows per warp, its stage of one plane (256 complex
+// values, then the Nyquist values of its rows, at least two for the 16-byte copies), and
+// its list of needed nodes.
+template <int H>
+struct FzWarpRows {
+    static constexpr int T = H / kFzRowE, ROWS = 32 / T, NYQ = ROWS * H, STAGE = NYQ + (ROWS < 2 ? 2 : ROWS);
+    using Lay = fz::RowLayout<H>;
+    static constexpr int EXCH = ROWS * (Lay::slots + Lay::slots1);
+};
+
 // shared memory of k_fz_c2r_rows (with_stages) and k_fz_r2c_rows
 inline size_t fz_row_smem(int H, int m, bool with_stages) {
-    const int T = H / kFzRowE, ROWS = kFzRowThreads / T;
+    const int rows = 32 / (H / kFzRowE), warps = kFzRowThreads / 32;
     const size_t slots = (H + (H >> 4) + 1) + (H + 8 * (H >> 6) + 1);
-    size_t b = 16 + (size_t)ROWS * slots * sizeof(float2) + (size_t)6 * m * sizeof(float);
-    if (with_stages) b += 2 * (size_t)(ROWS * H + ROWS) * sizeof(float2);
+    const size_t stage = (size_t)rows * H + (rows < 2 ? 2 : rows);
+    size_t b = 16 * warps + kFzMaxBatch * (size_t)warps + warps * rows * slots * sizeof(float2) + 8 +
+               (size_t)6 * m * sizeof(float);
+    if (with_stages) b += 2 * warps * stage * sizeof(float2);
     return b;
 }
 
 // Axis-2 C2R of the batch's planes plane0 .. plane0 + nb - 1 (node j0 + jj),
 // row by row, interpolated into `pot` at every point of the row: pot1 from the
 // P planes, pot3 from the M planes (SMALL: the small-k_F branch of node 0
-// counts, which it does for pot1 only).  The block's rows of each plane (16 KB
-// at n2 = 256) arrive by bulk copy two planes ahead of their use.
+// counts, which it does for pot1 only).  Every warp works alone: on its own rows, over
+// the planes of the nodes that they need, each 2 KB stage arriving by bulk copy two
+// planes ahead of its use, with warp barriers in the exchanges.  256^3, 64 nodes, P and M:
+// 2.65 ms with block-wide rows over every plane.
 // HERM = 1 (P planes) or 2 (M planes): the cubic Hermite interpolation, whose
 // P and M planes both feed pot1 and (kdd = 3) pot3 (fz_hermite_w); `pot` is
 // then unused, and the M pass adds to what the P pass of the batch wrote.
 template <int H, bool SMALL, int HERM = 0>
 __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_c2r_rows(FzRowArgs a, int plane0, float* __restrict__ pot) {
-    constexpr int E = kFzRowE, T = H / E, ROWS = kFzRowThreads / T, P = 2 * E;
-    constexpr int STAGE = ROWS * H + ROWS;  // float2: the block's rows, then their Nyquist values
-    using Lay = fz::RowLayout<H>;
+    using W = FzWarpRows<H>;
+    constexpr int E = kFzRowE, T = W::T, P = 2 * E, WARPS = kFzRowThreads / 32;
+    using Lay = typename W::Lay;
     extern __shared__ float4 fz_rsm4[];
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(fz_rsm4);
-    float2* stage = reinterpret_cast<float2*>(fz_rsm4 + 1);
-    float2* buf0 = stage + 2 * STAGE;
-    float2* buf1 = buf0 + ROWS * Lay::slots;
-    float* fs = reinterpret_cast<float*>(buf1 + ROWS * Lay::slots1);
-    const long long row0 = (long long)blockIdx.x * ROWS;
-    auto issue = [&](int jj) {  // one thread: plane jj into stage jj & 1
-        const int s = jj & 1;
-        const float2* src = a.XY + (long long)(plane0 + jj) * a.d.plane;
-        fz::mbar_expect_tx(&bar[s], STAGE * (unsigned)sizeof(float2));
-        fz::bulk_load(stage + s * STAGE, src + row0 * H, ROWS * H * (unsigned)sizeof(float2), &bar[s]);
-        fz::bulk_load(stage + s * STAGE + ROWS * H, src + a.d.nyq + row0, ROWS * (unsigned)sizeof(float2), &bar[s]);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(fz_rsm4) + 2 * warp;
+    float2* stages = reinterpret_cast<float2*>(fz_rsm4 + WARPS);
+    float2* stage = stages + 2 * W::STAGE * warp;
+    float2* exch = stages + 2 * W::STAGE * WARPS + W::EXCH * warp;
+    unsigned char* lists = reinterpret_cast<unsigned char*>(stages + (2 * W::STAGE + W::EXCH) * WARPS);
+    unsigned char* list = lists + kFzMaxBatch * warp;
+    float* fs = reinterpret_cast<float*>(lists + kFzMaxBatch * WARPS);
+    const long long row0 = ((long long)blockIdx.x * WARPS + warp) * W::ROWS;
+    const int need = fz_need_list(a, row0, W::ROWS, list);
+    // one lane: the rows of the q-th needed plane into stage q & 1
+    auto issue = [&](int q) {
+        const int s = q & 1;
+        const float2* src = a.XY + (long long)(plane0 + list[q]) * a.d.plane;
+        fz::mbar_expect_tx(&bar[s], W::STAGE * (unsigned)sizeof(float2));
+        fz::bulk_load(stage + s * W::STAGE, src + row0 * H, W::NYQ * (unsigned)sizeof(float2), &bar[s]);
+        fz::bulk_load(stage + s * W::STAGE + W::NYQ, src + a.d.nyq + (row0 & ~1LL),
+                      (W::STAGE - W::NYQ) * (unsigned)sizeof(float2), &bar[s]);
     };
-    __shared__ volatile int fail_flag;
-    volatile int* fail = &fail_flag;
-    int last_issued = -1;  // thread 0: the last plane whose copy it issued
-    if (threadIdx.x == 0) {
-        fail_flag = 0;
+    if (lane == 0) {
         fz::mbar_init(&bar[0], 1);
         fz::mbar_init(&bar[1], 1);
         fz::mbar_fence_init();
-        issue(0);
-        last_issued = 0;
-        if (a.nb > 1) {
-            issue(1);
-            last_issued = 1;
-        }
+        if (need > 0) issue(0);
+        if (need > 1) issue(1);
     }
     const FzNodeSm nodes = fz_stage_nodes(a, fs);
     __syncthreads();
-    const int t = threadIdx.x % T, l = threadIdx.x / T;
+    const int t = lane % T, l = lane / T;
+    const int nyq = W::NYQ + (W::ROWS < 2 ? (int)(row0 & 1) : 0);
     const long long row = row0 + l;
     const int n2 = 2 * H;
-    float2* b0 = buf0 + l * Lay::slots;
-    float2* b1 = buf1 + l * Lay::slots1;
+    float2* b0 = exch + l * Lay::slots;
+    float2* b1 = exch + W::ROWS * Lay::slots + l * Lay::slots1;
     const typename Lay::Idx ix;
     const typename Lay::Idx1 ix1;
     const float clipdn = __double2float_rd(a.kfclip);
@@ -508,45 +620,46 @@ __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_c2r_rows(FzRowArgs a, i
     // register twiddles, except for the Hermite passes (their second accumulator takes the registers)
     float2 twr[HERM ? 1 : fz::tw_count<H, E>()];
     if constexpr (HERM == 0) fz::tw_load<H, E>(twr, t, a.tw.th);
-    for (int jj = 0; jj < a.nb; ++jj) {
-        const int j = a.j0 + jj;
-        const int s = jj & 1;
-        // a copy that did not complete in time sets the error word and the block's
-        // flag; later waits are skipped, no more copies are issued, and the copies
-        // in flight are drained after the loop (the results are then garbage and
-        // the host raises the error).  Every thread runs the same barriers either way.
-        if (!*fail && !fz::mbar_wait(&bar[s], (jj >> 1) & 1)) {
-            *fail = 1;
-            atomicOr(a.err, 1u);
+    for (int q = 0; q < need; ++q) {
+        const int j = a.j0 + list[q];
+        const int s = q & 1;
+        // a copy that did not complete in time sets the error word, and the warp gives up
+        // (the results are then garbage and the host raises the error): it lets the copy
+        // still in flight land, with the same limit, and returns
+        if (__any_sync(0xffffffffu, !fz::mbar_wait(&bar[s], (q >> 1) & 1))) {
+            if (lane == 0) {
+                atomicOr(a.err, 1u);
+                if (q + 1 < need) fz::mbar_wait(&bar[s ^ 1], ((q + 1) >> 1) & 1);
+            }
+            return;
         }
         float2 v[E];
-        fz_c2r_pre<H>(stage + s * STAGE, l, t, a.tw.tr, v);
-        if constexpr (HERM == 0) fz::line_fft_ppr<H, E, +1>(v, b0, b1, ix, ix1, t, twr);
-        else fz::line_fft_pp<H, E, +1>(v, b0, b1, ix, t, a.tw.th);
-        // every thread has passed the transform's first barrier, so stage s is read
-        if (threadIdx.x == 0 && jj + 2 < a.nb && !*fail) {
+        fz_c2r_pre<H>(stage + s * W::STAGE, l, nyq, t, a.tw.tr, v);
+        __syncwarp();  // stage s is read
+        if (lane == 0 && q + 2 < need) {
             fz::fence_proxy_async();
-            issue(jj + 2);
-            last_issued = jj + 2;
+            issue(q + 2);
         }
+        if constexpr (HERM == 0) fz::line_fft_ppr<H, E, +1, fz::WarpSync>(v, b0, b1, ix, ix1, t, twr);
+        else fz::line_fft_pp<H, E, +1, fz::WarpSync>(v, b0, b1, ix, t, a.tw.th);
         const float jf = (float)j;
         if constexpr (HERM == 0) {
 #pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const float pv = (q & 1) ? v[q >> 1].y : v[q >> 1].x;
-                acc[q] = fmaf(fz_hat(jf, fi[q], tr[q]), pv, acc[q]);
+            for (int p = 0; p < P; ++p) {
+                const float pv = (p & 1) ? v[p >> 1].y : v[p >> 1].x;
+                acc[p] = fmaf(fz_hat(jf, fi[p], tr[p]), pv, acc[p]);
             }
         } else {
             const float D0 = nodes.dk[j], D1 = j > 0 ? nodes.dk[j - 1] : 0.0f;
             const float iD0 = D0 > 0.0f ? 1.0f / D0 : 0.0f, iD1 = D1 > 0.0f ? 1.0f / D1 : 0.0f;
 #pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const float pv = (q & 1) ? v[q >> 1].y : v[q >> 1].x;
-                const float dd = jf - fi[q];
+            for (int p = 0; p < P; ++p) {
+                const float pv = (p & 1) ? v[p >> 1].y : v[p >> 1].x;
+                const float dd = jf - fi[p];
                 float w1, w3;
-                fz_hermite_w<HERM == 2>(tr[q], dd == 0.0f, dd == 1.0f, D0, D1, iD0, iD1, w1, w3);
-                acc[q] = fmaf(w1, pv, acc[q]);
-                if (has3) acc3[q] = fmaf(w3, pv, acc3[q]);
+                fz_hermite_w<HERM == 2>(tr[p], dd == 0.0f, dd == 1.0f, D0, D1, iD0, iD1, w1, w3);
+                acc[p] = fmaf(w1, pv, acc[p]);
+                if (has3) acc3[p] = fmaf(w3, pv, acc3[p]);
             }
         }
         if (SMALL && j == 0) {
@@ -557,11 +670,6 @@ __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_c2r_rows(FzRowArgs a, i
                 acc[2 * e + 1] = fmaf(fz_small_weight(kk.y, a, nodes, clipdn, true), v[e].y, acc[2 * e + 1]);
             }
         }
-    }
-    if (threadIdx.x == 0 && *fail) {
-        // let the copies still in flight land before the block exits (bounded)
-        for (int q = (last_issued > 0 ? last_issued - 1 : 0); q <= last_issued; ++q)
-            fz::mbar_wait(&bar[q & 1], (q >> 1) & 1);
     }
     // the P pass of a first batch writes; every other pass adds
     const bool add = !a.first || HERM == 2;
@@ -596,22 +704,30 @@ __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_c2r_rows(FzRowArgs a, i
 // HERM: the cubic Hermite interpolation's two hat planes per node, rho^alpha
 // times h00 | h01 into plane jj and rho^alpha times D0 h10 | D1 h11 into plane
 // nb + jj (lwt.py:285-296; fz_hermite_w's w1 of the P and M planes).
+// Every warp works alone, over the nodes that its rows need (the planes' other rows are
+// zero: the axis-1 pass does not read them).
 template <int H, bool HERM = false>
 __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_r2c_rows(FzRowArgs a) {
-    constexpr int E = kFzRowE, T = H / E, ROWS = kFzRowThreads / T, P = 2 * E;
+    using W = FzWarpRows<H>;
+    constexpr int E = kFzRowE, T = W::T, P = 2 * E, WARPS = kFzRowThreads / 32;
     static_assert(T <= 32, "a row must fit in one warp");
-    using Lay = fz::RowLayout<H>;
+    using Lay = typename W::Lay;
     extern __shared__ float4 fz_rsm4[];
-    float2* buf0 = reinterpret_cast<float2*>(fz_rsm4 + 1);
-    float2* buf1 = buf0 + ROWS * Lay::slots;
-    float* fs = reinterpret_cast<float*>(buf1 + ROWS * Lay::slots1);
+    const int warp = threadIdx.x >> 5;
+    float2* exchs = reinterpret_cast<float2*>(fz_rsm4);
+    float2* exch = exchs + W::EXCH * warp;
+    unsigned char* lists = reinterpret_cast<unsigned char*>(exchs + W::EXCH * WARPS);
+    unsigned char* list = lists + kFzMaxBatch * warp;
+    float* fs = reinterpret_cast<float*>(lists + kFzMaxBatch * WARPS);
+    const long long row0 = ((long long)blockIdx.x * WARPS + warp) * W::ROWS;
+    const int need = fz_need_list(a, row0, W::ROWS, list);
     const FzNodeSm nodes = fz_stage_nodes(a, fs);
     __syncthreads();
-    const int t = threadIdx.x % T, l = threadIdx.x / T;
-    const long long row = (long long)blockIdx.x * ROWS + l;
+    const int t = (threadIdx.x & 31) % T, l = (threadIdx.x & 31) / T;
+    const long long row = row0 + l;
     const int n2 = 2 * H;
-    float2* b0 = buf0 + l * Lay::slots;
-    float2* b1 = buf1 + l * Lay::slots1;
+    float2* b0 = exch + l * Lay::slots;
+    float2* b1 = exch + W::ROWS * Lay::slots + l * Lay::slots1;
     const typename Lay::Idx ix;
     const typename Lay::Idx1 ix1;
     const float clipdn = __double2float_rd(a.kfclip);
@@ -645,8 +761,8 @@ __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_r2c_rows(FzRowArgs a) {
     if constexpr (!HERM) fz::tw_load<H, E>(twr, t, a.tw.th);
     // the row transform of v, post-processed and stored into plane pl
     auto emit = [&](float2 (&v)[E], int pl) {
-        if constexpr (!HERM) fz::line_fft_ppr<H, E, -1>(v, b0, b1, ix, ix1, t, twr);
-        else fz::line_fft_pp<H, E, -1>(v, b0, b1, ix, t, a.tw.th);
+        if constexpr (!HERM) fz::line_fft_ppr<H, E, -1, fz::WarpSync>(v, b0, b1, ix, ix1, t, twr);
+        else fz::line_fft_pp<H, E, -1, fz::WarpSync>(v, b0, b1, ix, t, a.tw.th);
         float2* dst = a.XY + (long long)pl * a.d.plane;
 #pragma unroll
         for (int e = 0; e < E; ++e) {
@@ -664,7 +780,8 @@ __global__ void __launch_bounds__(kFzRowThreads, 2) k_fz_r2c_rows(FzRowArgs a) {
         }
         if (t == 0) __stcs(dst + a.d.nyq + row, make_float2(v[0].x - v[0].y, 0.0f));
     };
-    for (int jj = 0; jj < a.nb; ++jj) {
+    for (int qn = 0; qn < need; ++qn) {
+        const int jj = list[qn];
         const int j = a.j0 + jj;
         const float jf = (float)j;
         float2 v[E];

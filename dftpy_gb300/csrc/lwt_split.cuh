@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kS8RowThreads, 1) k_fz_c2r_s8(FzRowArgs a, int
         }
         __syncthreads();  // rows r1 = d + 8 c are in st; every thread is done with buf0
         float2 v[E];
-        fz_c2r_pre<H, ROWS>(st, l, t, a.tw.tr, v);
+        fz_c2r_pre<H>(st, l, ROWS * H, t, a.tw.tr, v);
         fz::fence_proxy_async();  // this thread's accesses to st come before the next copy into it
         fz::line_fft_ppr<H, E, +1>(v, b0, b1, ix, ix1, t, twr);
         // every thread has passed the transform's first barrier, so stage s is read

@@ -999,7 +999,6 @@ struct LwtPlan {
 
 // ------------------------------------------------ fused k_F-node pipeline (host)
 constexpr int kFzMaxNodes = 1024;  // node bounds (6 floats each) staged in shared memory
-constexpr int kFzMaxBatch = 256;   // node reciprocals staged in shared memory
 
 bool fz_applies(const ofdft_grid* g, int m) {
     auto p2 = [](int n, int lo, int hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; };
@@ -1127,10 +1126,6 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
     // kernel's events time that kernel alone.
     const bool two = r.kdd > 1 && !e->prof;
     cudaStream_t st2 = two ? e->fz_st2 : st;
-    if (two) {
-        OFDFT_CK(cudaEventRecord(e->fz_fork, st));
-        OFDFT_CK(cudaStreamWaitEvent(st2, e->fz_fork, 0));
-    }
     const double Ncd = (double)g->Nc, Nd = (double)g->N;
     const float invN = (float)(1.0 / Nd);
     const int tiles0 = n1 * (H / kFzLines) + n1 / kFzLines;
@@ -1138,6 +1133,31 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
     const double* knode = r.nd.k;
     const double* invk = r.nd.invk;
     int launches = 0;
+    // the rows that each node needs
+    FzNeed need{};
+    if (!split) {
+        const int words = n1 / 32;
+        unsigned* bits = (unsigned*)e->sc.get("fz_need", (size_t)n0 * r.m * words * sizeof(unsigned));
+        need.bits = bits;
+        need.m = r.m;
+        need.words = words;
+        FzRowArgs na{};
+        na.kf = r.kf;
+        na.kn = e->d_nodes;
+        na.kup = e->d_nodes + 2 * kMaxNodes;
+        na.m = r.m;
+        na.kfclip = r.kfclip;
+        na.d = d;
+        na.need = need;
+        const size_t smem = fz_need_smem(r.m);
+        timed(e, P_LWT_INTERP, Nd * 4.0, st, [&] { k_fz_need<<<n0 * words, kFzRowThreads, smem, st>>>(na, bits); });
+        OFDFT_LAUNCH_CHECK();
+        ++launches;
+    }
+    if (two) {
+        OFDFT_CK(cudaEventRecord(e->fz_fork, st));
+        OFDFT_CK(cudaStreamWaitEvent(st2, e->fz_fork, 0));
+    }
     for (int j0 = 0; j0 < r.m; j0 += B) {
         const int nb = std::min(B, r.m - j0);
         const int nplanes = mc ? 2 * nb : nb;
@@ -1162,6 +1182,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
         ra.d = d;
         ra.tw = tw;
         ra.err = e->d_fz_err;
+        ra.need = need;
         if (split) {
             // axis 0 + the radix-8 stage of axis 1, then the 32-point stage with the rows
             with_col(n0, [&](auto c0) {
@@ -1209,7 +1230,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
             constexpr int N1 = decltype(c1)::value;
             const size_t smem = std::max(fz::col_slots(N1), kFzLines * fz::row_slots(N1)) * sizeof(float2);
             timed(e, P_FZ_AXIS1, Ncd * 16.0 * nplanes, st,
-                  [&] { k_fz_axis1<N1, +1><<<tiles1 * nplanes, N1, smem, st>>>(XY, d, tw.t1); });
+                  [&] { k_fz_axis1<N1, +1><<<tiles1 * nplanes, N1, smem, st>>>(XY, d, tw.t1, need, j0, nb); });
         });
         OFDFT_LAUNCH_CHECK();
         // ---- axis 2 C2R with the interpolation into pot1 (pot3)
@@ -1277,7 +1298,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
                 constexpr int N1 = decltype(c1)::value;
                 const size_t smem = std::max(fz::col_slots(N1), kFzLines * fz::row_slots(N1)) * sizeof(float2);
                 timed(e, P_FZ_AXIS1, Ncd * 16.0 * hp * nb, st2,
-                      [&] { k_fz_axis1<N1, -1><<<tiles1 * hp * nb, N1, smem, st2>>>(XY2, d, tw.t1); });
+                      [&] { k_fz_axis1<N1, -1><<<tiles1 * hp * nb, N1, smem, st2>>>(XY2, d, tw.t1, need, j0, nb); });
             });
             OFDFT_LAUNCH_CHECK();
             if (!split) with_col(n0, [&](auto c0) {
