@@ -8,6 +8,7 @@
 //   stress     Stress_real (:609-662) with the real-space sum; Stress_rec_PME
 //              (:915-968) or Stress_rec (:719-763) over the mask, G = 0 term
 #include "common.cuh"
+#include "fix_eval.h"
 #include "host_math.h"
 #include "pme.cuh"
 
@@ -19,7 +20,7 @@ using namespace ofdft;
 namespace ofdft {
 void frac_coords(const double* lattice, int nat, const double* pos, std::vector<double>& frac);
 void lattice_inverse(const double* a, double* inv);
-void bspline_tables(const ofdft_grid* g, int order, double** d_re, double** d_im);
+void bspline_tables(const ofdft_grid* g, int order, std::vector<double>& re, std::vector<double>& im);
 }  // namespace ofdft
 
 namespace {
@@ -32,94 +33,158 @@ struct CellList {
     const int* cellof;  // cell of each atom
 };
 
-// one thread per atom: sum over the (2K+1)^3 neighbour cells (unwrapped, so
-// each periodic image of each atom is visited exactly once).  Partials: the
-// energy sum, then the six sums of Stress_real (:645-654),
-// q_i q_j (2 sqrt(eta/pi) exp(-eta d^2) + erfc(sqrt(eta) d)/d) R_a R_b / d^2.
-__global__ void __launch_bounds__(RED_THREADS) k_ewald_real(const double* __restrict__ pos,
-                                                            const double* __restrict__ q, int nat,
-                                                            const double* __restrict__ lat, CellList cl, double Rcut,
-                                                            double eta, double* F, double* partials) {
+// One warp per atom over the atoms of the (2K+1)^3 neighbour cells (unwrapped, so each
+// periodic image of each atom is visited exactly once), 32 candidates at a time: every lane
+// computes one candidate's terms, then ten lanes add one component each, in the order of
+// the candidates, so the sums are those of a serial loop (the optimisers' line searches
+// see the energy's last bits).  One thread per atom took 143 us, a serial chain of float64
+// functions.  Per atom: the energy sum, then the six sums of Stress_real (:645-654),
+// q_i q_j (2 sqrt(eta/pi) exp(-eta d^2) + erfc(sqrt(eta) d)/d) R_a R_b / d^2, to sums[7 i].
+constexpr int kRealWarps = 4;
+__global__ void __launch_bounds__(32 * kRealWarps)
+    k_ewald_real(const double* __restrict__ pos, const double* __restrict__ q, int nat, const double* __restrict__ lat,
+                 CellList cl, double Rcut, double eta, double* F, double* __restrict__ sums) {
+    __shared__ double term[kRealWarps][32][10];
+    __shared__ int first[kRealWarps][32];  // candidates before each cell of the batch
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * kRealWarps + warp;
+    if (i >= nat) return;
+    const double es = sqrt(eta);
+    const double rtol = 0.001;
+    const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
+    const int c = cl.cellof[i];
+    const int c0 = c / (cl.nc[1] * cl.nc[2]), c1 = (c / cl.nc[2]) % cl.nc[1], c2 = c % cl.nc[2];
+    const double sp2 = 2.0 * es / sqrt(M_PI);
+    const int m1 = 2 * cl.K[1] + 1, m2 = 2 * cl.K[2] + 1, cells = (2 * cl.K[0] + 1) * m1 * m2;
+    double s = 0.0;  // component `lane` < 10: energy, force, stress
+    auto unwrapped = [&](int t, int (&u)[3]) {
+        u[0] = c0 + t / (m1 * m2) - cl.K[0];
+        u[1] = c1 + (t / m2) % m1 - cl.K[1];
+        u[2] = c2 + t % m2 - cl.K[2];
+    };
+    auto cell_of = [&](const int (&u)[3]) {
+        return (pmod(u[0], cl.nc[0]) * cl.nc[1] + pmod(u[1], cl.nc[1])) * cl.nc[2] + pmod(u[2], cl.nc[2]);
+    };
+    for (int t0 = 0; t0 < cells; t0 += 32) {
+        // the batch's cells, one per lane, and where their atoms start in its candidates
+        int u[3], count = 0;
+        if (t0 + lane < cells) {
+            unwrapped(t0 + lane, u);
+            const int cell = cell_of(u);
+            count = cl.start[cell + 1] - cl.start[cell];
+        }
+        int upto = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+        }
+        __syncwarp();
+        first[warp][lane] = upto - count;
+        __syncwarp();
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+        for (int h0 = 0; h0 < total; h0 += 32) {
+            const int h = h0 + lane;
+            bool in = false;
+            if (h < total) {
+                int lo = 0, hi = 32;  // the last cell that starts at or before h (empty ones share its start)
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (first[warp][mid] <= h) lo = mid;
+                    else hi = mid;
+                }
+                unwrapped(t0 + lo, u);
+                const int cell = cell_of(u);
+                const int j = cl.atoms[cl.start[cell] + h - first[warp][lo]];
+                const double n0 = floor((double)u[0] / cl.nc[0]), n1 = floor((double)u[1] / cl.nc[1]),
+                             n2 = floor((double)u[2] / cl.nc[2]);
+                const double tx = n0 * lat[0] + n1 * lat[3] + n2 * lat[6];
+                const double ty = n0 * lat[1] + n1 * lat[4] + n2 * lat[7];
+                const double tz = n0 * lat[2] + n1 * lat[5] + n2 * lat[8];
+                const double dx = xi - (pos[3 * j] + tx), dy = yi - (pos[3 * j + 1] + ty),
+                             dz = zi - (pos[3 * j + 2] + tz);
+                const double d = sqrt(dx * dx + dy * dy + dz * dz);
+                in = d < Rcut && d > rtol;
+                if (in) {
+                    const double x = es * d;
+                    const double ec = erfc(x);
+                    double* o = term[warp][lane];
+                    o[0] = q[j] * ec / d;
+                    const double w = q[j] * (ec / (x * x * x) + 2.0 / sqrt(M_PI) * exp(-x * x) / (x * x));
+                    o[1] = dx * w;
+                    o[2] = dy * w;
+                    o[3] = dz * w;
+                    const double ws = q[j] * (sp2 * exp(-eta * d * d) + ec / d) / (d * d);
+                    o[4] = ws * dx * dx;
+                    o[5] = ws * dx * dy;
+                    o[6] = ws * dx * dz;
+                    o[7] = ws * dy * dy;
+                    o[8] = ws * dy * dz;
+                    o[9] = ws * dz * dz;
+                }
+            }
+            unsigned hits = __ballot_sync(0xffffffffu, in);
+            __syncwarp();
+            if (lane < 10)
+                for (; hits; hits &= hits - 1) s += term[warp][__ffs(hits) - 1][lane];
+            __syncwarp();
+        }
+    }
+    if (lane == 0) sums[7 * i] = q[i] * s;
+    else if (lane < 4) F[3 * i + lane - 1] = q[i] * s * (es * es * es);
+    else if (lane < 10) sums[7 * i + lane - 3] = q[i] * s;
+}
+
+// block sums of the atoms' seven values, one thread per atom
+__global__ void __launch_bounds__(RED_THREADS) k_ewald_real_sum(const double* __restrict__ sums, int nat,
+                                                                double* partials) {
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nat) {
-        const double es = sqrt(eta);
-        const double rtol = 0.001;
-        const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-        const int c = cl.cellof[i];
-        const int c0 = c / (cl.nc[1] * cl.nc[2]), c1 = (c / cl.nc[2]) % cl.nc[1], c2 = c % cl.nc[2];
-        double e = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
-        double s6[6] = {0, 0, 0, 0, 0, 0};
-        const double sp2 = 2.0 * es / sqrt(M_PI);
-        for (int d0 = -cl.K[0]; d0 <= cl.K[0]; ++d0)
-            for (int d1 = -cl.K[1]; d1 <= cl.K[1]; ++d1)
-                for (int d2 = -cl.K[2]; d2 <= cl.K[2]; ++d2) {
-                    const int u0 = c0 + d0, u1 = c1 + d1, u2 = c2 + d2;
-                    const int w0 = pmod(u0, cl.nc[0]), w1 = pmod(u1, cl.nc[1]), w2 = pmod(u2, cl.nc[2]);
-                    const double n0 = floor((double)u0 / cl.nc[0]), n1 = floor((double)u1 / cl.nc[1]),
-                                 n2 = floor((double)u2 / cl.nc[2]);
-                    const double tx = n0 * lat[0] + n1 * lat[3] + n2 * lat[6];
-                    const double ty = n0 * lat[1] + n1 * lat[4] + n2 * lat[7];
-                    const double tz = n0 * lat[2] + n1 * lat[5] + n2 * lat[8];
-                    const int cell = (w0 * cl.nc[1] + w1) * cl.nc[2] + w2;
-                    for (int p = cl.start[cell]; p < cl.start[cell + 1]; ++p) {
-                        const int j = cl.atoms[p];
-                        const double dx = xi - (pos[3 * j] + tx), dy = yi - (pos[3 * j + 1] + ty),
-                                     dz = zi - (pos[3 * j + 2] + tz);
-                        const double d = sqrt(dx * dx + dy * dy + dz * dz);
-                        if (d < Rcut && d > rtol) {
-                            const double x = es * d;
-                            const double ec = erfc(x);
-                            e += q[j] * ec / d;
-                            const double w = q[j] * (ec / (x * x * x) + 2.0 / sqrt(M_PI) * exp(-x * x) / (x * x));
-                            fx += dx * w;
-                            fy += dy * w;
-                            fz += dz * w;
-                            const double ws = q[j] * (sp2 * exp(-eta * d * d) + ec / d) / (d * d);
-                            s6[0] += ws * dx * dx;
-                            s6[1] += ws * dx * dy;
-                            s6[2] += ws * dx * dz;
-                            s6[3] += ws * dy * dy;
-                            s6[4] += ws * dy * dz;
-                            s6[5] += ws * dz * dz;
-                        }
-                    }
-                }
-        acc[0] = q[i] * e;
-        for (int k = 0; k < 6; ++k) acc[1 + k] = q[i] * s6[k];
-        const double e3 = es * es * es;
-        F[3 * i] = q[i] * fx * e3;
-        F[3 * i + 1] = q[i] * fy * e3;
-        F[3 * i + 2] = q[i] * fz * e3;
-    }
+    if (i < nat)
+        for (int k = 0; k < 7; ++k) acc[k] = sums[7 * i + k];
     block_sum_store<7>(acc, partials);
 }
 
-// PME reciprocal energy partials and the force convolution input:
+// PME reciprocal energy and the force convolution input:
 // E = 4 pi/V sum_mask |Q(G) B(G)|^2 exp(-G^2/4 eta)/G^2 (raw FFT, dV factors cancel);
-// X = Q(G) |B(G)|^2 exp(-G^2/4 eta)/G^2 / N
+// X = Q(G) |B(G)|^2 exp(-G^2/4 eta)/G^2 / N.  The factors of the energy's terms go to
+// terms (zero outside the mask) and are summed by k_ewald_rec_sum, whose order of the
+// points does not depend on how this pass walks the rows.
 template <typename T>
-__global__ void __launch_bounds__(RED_THREADS) k_ewald_rec_pme(const typename Cplx<T>::type* __restrict__ QG,
-                                                               typename Cplx<T>::type* X, const double* bre,
-                                                               const double* bim, Geo geo, double eta,
+__global__ void __launch_bounds__(32 * kRowWarps)
+    k_ewald_rec_pme(const typename Cplx<T>::type* __restrict__ QG, typename Cplx<T>::type* X, const double* bre,
+                    const double* bim, Geo geo, double eta, double2* __restrict__ terms) {
+    const int rows = geo.n0 * geo.n1;
+    const double invN = 1.0 / (double)geo.N;
+    for (int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kRowWarps) {
+        const HalfRow r = half_row(geo, row, bre, bim);
+        for (int k = threadIdx.x & 31; k < geo.n2h; k += 32) {
+            const long long i = (long long)row * geo.n2h + k;
+            const double gg = row_gsq(geo, r, k);
+            double br, bi;
+            row_barray(geo, r, bre, bim, k, br, bi);
+            const double qr = (double)QG[i].x, qi = (double)QG[i].y;
+            const double sr = qr * br - qi * bi, si = qr * bi + qi * br;
+            const double inv = (i == 0) ? 0.0 : 1.0 / gg;
+            const double w = exp(-gg / (4.0 * eta)) * inv;
+            terms[i] = half_mask(geo, i) ? make_double2(sr * sr + si * si, w) : make_double2(0.0, 0.0);
+            if (X) {
+                const double f = (br * br + bi * bi) * w * invN;
+                X[i].x = (T)(qr * f);
+                X[i].y = (T)(qi * f);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(RED_THREADS) k_ewald_rec_sum(const double2* __restrict__ terms, long long n,
                                                                double* partials) {
     double acc[1] = {0.0};
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < geo.Nc; i += stride) {
-        double gg = gsq(geo, i);
-        double br, bi;
-        barray(bre, bim, geo, i, br, bi);
-        double qr = (double)QG[i].x, qi = (double)QG[i].y;
-        double sr = qr * br - qi * bi, si = qr * bi + qi * br;
-        double inv = (i == 0) ? 0.0 : 1.0 / gg;
-        double w = exp(-gg / (4.0 * eta)) * inv;
-        if (half_mask(geo, i)) acc[0] += (sr * sr + si * si) * w;
-        if (X) {
-            double b2 = br * br + bi * bi;
-            double f = b2 * w / (double)geo.N;
-            X[i].x = (T)(qr * f);
-            X[i].y = (T)(qi * f);
-        }
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+        const double2 t = terms[i];
+        acc[0] = fma(t.x, t.y, acc[0]);
     }
     block_sum_store<1>(acc, partials);
 }
@@ -296,107 +361,115 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
         std::vector<int> fill(start.begin(), start.end() - 1);
         for (int a = 0; a < nat; ++a) order_atoms[fill[cellof[a]]++] = a;
     }
-    Scratch sc;
-    double* d_pos = (double*)sc.get("pos", 3 * (size_t)nat * sizeof(double));
-    double* d_q = (double*)sc.get("q", (size_t)nat * sizeof(double));
-    double* d_lat = (double*)sc.get("lat", 9 * sizeof(double));
-    int* d_start = (int*)sc.get("start", (ncell + 1) * sizeof(int));
-    int* d_atoms = (int*)sc.get("atoms", (size_t)nat * sizeof(int));
-    int* d_cellof = (int*)sc.get("cellof", (size_t)nat * sizeof(int));
-    double* d_F = (double*)sc.get("F", 3 * (size_t)nat * sizeof(double));
-    double* d_Fr = (double*)sc.get("Fr", 3 * (size_t)nat * sizeof(double));
-    double* d_frac = (double*)sc.get("frac", 3 * (size_t)nat * sizeof(double));
-    double* d_scale = (double*)sc.get("scale", (size_t)nat * sizeof(double));
-    double* d_cinv = (double*)sc.get("cinv", 9 * sizeof(double));
-    OFDFT_CK(cudaMemcpyAsync(d_pos, wpos.data(), 3 * (size_t)nat * sizeof(double), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(d_q, q.data(), (size_t)nat * sizeof(double), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(d_lat, g->lattice, 9 * sizeof(double), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(d_start, start.data(), (ncell + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(d_atoms, order_atoms.data(), (size_t)nat * sizeof(int), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(d_cellof, cellof.data(), (size_t)nat * sizeof(int), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(d_frac, frac.data(), 3 * (size_t)nat * sizeof(double), cudaMemcpyHostToDevice, st));
-    cl.start = d_start;
-    cl.atoms = d_atoms;
-    cl.cellof = d_cellof;
+    // Device buffers live in the grid's scratch; what the host prepares goes up in one copy
+    Scratch& sc = g->scratch;
+    const size_t n = (size_t)nat;
+    double cinv[9];
+    lattice_inverse(g->lattice, cinv);
+    std::vector<double> up(8 * n + 18);
+    double *u_pos = up.data(), *u_q = u_pos + 3 * n, *u_frac = u_q + n, *u_scale = u_frac + 3 * n, *u_lat = u_scale + n,
+           *u_cinv = u_lat + 9;
+    std::copy(wpos.begin(), wpos.end(), u_pos);
+    std::copy(q.begin(), q.end(), u_q);
+    std::copy(frac.begin(), frac.end(), u_frac);
+    for (int a = 0; a < nat; ++a) u_scale[a] = -q[a] * 4.0 * M_PI / g->dV;
+    std::copy(g->lattice, g->lattice + 9, u_lat);
+    std::copy(cinv, cinv + 9, u_cinv);
+    std::vector<int> ui(start);
+    ui.insert(ui.end(), order_atoms.begin(), order_atoms.end());
+    ui.insert(ui.end(), cellof.begin(), cellof.end());
+    double* d_up = (double*)sc.get("ew_up", up.size() * sizeof(double));
+    int* d_ui = (int*)sc.get("ew_ui", ui.size() * sizeof(int));
+    OFDFT_CK(cudaMemcpyAsync(d_up, up.data(), up.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    OFDFT_CK(cudaMemcpyAsync(d_ui, ui.data(), ui.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    double *d_pos = d_up, *d_q = d_pos + 3 * n, *d_frac = d_q + n, *d_scale = d_frac + 3 * n, *d_lat = d_scale + n,
+           *d_cinv = d_lat + 9;
+    double* d_F = (double*)sc.get("ew_F", 6 * n * sizeof(double));  // real-space, then reciprocal forces
+    cl.start = d_ui;
+    cl.atoms = d_ui + ncell + 1;
+    cl.cellof = cl.atoms + nat;
     const int ablk = (nat + RED_THREADS - 1) / RED_THREADS;
-    OFDFT_REQUIRE(ablk <= g->red_blocks * 32, "Ewald: too many atoms for the reduction buffer");
-    k_ewald_real<<<ablk, RED_THREADS, 0, st>>>(d_pos, d_q, nat, d_lat, cl, Rcut, eta, d_Fr, g->d_partials);
+    double* d_part = (double*)sc.get("ew_part", (size_t)std::max(ablk * 7, g->red_blocks) * sizeof(double));
+    double* d_sums = (double*)sc.get("ew_sums", 7 * n * sizeof(double));
+    k_ewald_real<<<(nat + kRealWarps - 1) / kRealWarps, 32 * kRealWarps, 0, st>>>(d_pos, d_q, nat, d_lat, cl, Rcut, eta,
+                                                                                 d_F, d_sums);
     OFDFT_LAUNCH_CHECK();
-    reduce_finalize<<<7, RED_THREADS, 0, st>>>(g->d_partials, ablk, 7, 0ull, g->d_results);
+    k_ewald_real_sum<<<ablk, RED_THREADS, 0, st>>>(d_sums, nat, d_part);
     OFDFT_LAUNCH_CHECK();
-    OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 7 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    OFDFT_CK(cudaStreamSynchronize(st));
-    const double e_real = g->h_results[0] / 2.0;
-    double s_real[6];
-    for (int k = 0; k < 6; ++k) s_real[k] = g->h_results[1 + k] * (-0.5 / g->volume);
-    std::vector<double> Freal(3 * (size_t)nat);
-    OFDFT_CK(cudaMemcpyAsync(Freal.data(), d_Fr, 3 * (size_t)nat * sizeof(double), cudaMemcpyDeviceToHost, st));
-    OFDFT_CK(cudaStreamSynchronize(st));
+    reduce_finalize<<<7, RED_THREADS, 0, st>>>(d_part, ablk, 7, 0ull, g->d_results);
+    OFDFT_LAUNCH_CHECK();
 
     // ---- reciprocal space
+    // results: [0, 7) real-space sums, 7 the reciprocal energy, [8, 14) the reciprocal stress
     double e_rec = 0.0;
     double s_rec[6] = {0, 0, 0, 0, 0, 0};
-    std::vector<double> Frec(3 * (size_t)nat, 0.0);
+    std::vector<double> Fall(6 * n, 0.0);
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
     if (pme) {
         OFDFT_REQUIRE(g->nr[0] >= order && g->nr[1] >= order && g->nr[2] >= order,
                       "PME needs at least %d grid points per axis", order);
-        double *bre = nullptr, *bim = nullptr;
-        bspline_tables(g, order, &bre, &bim);
-        T* Q = (T*)sc.get("Q", rb);
-        C* QG = (C*)sc.get("QG", cb);
-        C* X = forces ? (C*)sc.get("X", cb) : nullptr;
-        const PmeTiles tiles = pme_tiles_build(sc, "pme_", frac.data(), nullptr, nat, order, g->nr, st);
-        pme_spread<T>(tiles, d_frac, nullptr, d_q, g->geo, Q, rb, st);
+        std::vector<double> bm, bi;
+        bspline_tables(g, order, bm, bi);
+        const size_t nb = bm.size();
+        bm.insert(bm.end(), bi.begin(), bi.end());
+        double* bre = (double*)sc.get("ew_b", bm.size() * sizeof(double));
+        double* bim = bre + nb;
+        OFDFT_CK(cudaMemcpyAsync(bre, bm.data(), bm.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        T* Q = (T*)sc.get("ew_Q", rb);
+        C* QG = (C*)sc.get("ew_QG", cb);
+        C* X = forces ? (C*)sc.get("ew_X", cb) : nullptr;
+        pme_spread<T>(sc, "ew_", nat, order, d_frac, nullptr, d_q, g->geo, Q, st);
         g->exec_r2c(Q, QG, 1, st);
-        k_ewald_rec_pme<T><<<g->red_blocks, RED_THREADS, 0, st>>>(QG, X, bre, bim, g->geo, eta, g->d_partials);
+        double2* terms = (double2*)sc.get("ew_terms", (size_t)g->Nc * sizeof(double2));
+        k_ewald_rec_pme<T><<<row_grid(g->geo, g->sms), 32 * kRowWarps, 0, st>>>(QG, X, bre, bim, g->geo, eta, terms);
         OFDFT_LAUNCH_CHECK();
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 1, 0ull, g->d_results);
+        k_ewald_rec_sum<<<g->red_blocks, RED_THREADS, 0, st>>>(terms, g->Nc, d_part);
         OFDFT_LAUNCH_CHECK();
-        OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, sizeof(double), cudaMemcpyDeviceToHost, st));
-        OFDFT_CK(cudaStreamSynchronize(st));
-        e_rec = 4.0 * M_PI * g->h_results[0] / g->volume;
+        reduce_finalize<<<1, RED_THREADS, 0, st>>>(d_part, g->red_blocks, 1, 0ull, g->d_results + 7);
+        OFDFT_LAUNCH_CHECK();
         if (stress) {
             k_ewald_stress_rec<T><<<g->red_blocks, RED_THREADS, 0, st>>>(QG, nullptr, bre, bim, g->geo, eta,
                                                                          g->d_partials);
             OFDFT_LAUNCH_CHECK();
-            reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
+            reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results + 8);
             OFDFT_LAUNCH_CHECK();
-            OFDFT_CK(cudaMemcpyAsync(s_rec, g->d_results, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
-            OFDFT_CK(cudaStreamSynchronize(st));
         }
         if (forces) {
-            T* conv = (T*)sc.get("conv", rb);
-            g->exec_c2r(X, conv, 1, st);
-            double cinv[9];
-            lattice_inverse(g->lattice, cinv);
-            std::vector<double> scale(nat);
-            for (int a = 0; a < nat; ++a) scale[a] = -q[a] * 4.0 * M_PI / g->dV;
-            OFDFT_CK(cudaMemcpyAsync(d_cinv, cinv, 9 * sizeof(double), cudaMemcpyHostToDevice, st));
-            OFDFT_CK(cudaMemcpyAsync(d_scale, scale.data(), (size_t)nat * sizeof(double), cudaMemcpyHostToDevice, st));
-            k_pme_gather<T><<<nat, 256, 0, st>>>(d_frac, nullptr, order, g->geo, conv, d_cinv, d_scale, d_F);
+            T* conv = Q;  // the mesh charges are done with
+            if (sizeof(T) == 8 && fix::grid_plans(g)) {
+                double2* in = (double2*)X;
+                double* out = (double*)conv;
+                fix::c2r(g, &in, &out, 1, st);
+            } else {
+                g->exec_c2r(X, conv, 1, st);
+            }
+            k_pme_gather<T><<<nat, kGatherThreads, 0, st>>>(d_frac, nullptr, order, g->geo, conv, d_cinv, d_scale,
+                                                            d_F + 3 * n);
             OFDFT_LAUNCH_CHECK();
-            OFDFT_CK(cudaMemcpyAsync(Frec.data(), d_F, 3 * (size_t)nat * sizeof(double), cudaMemcpyDeviceToHost, st));
-            OFDFT_CK(cudaStreamSynchronize(st));
         }
-        cudaFree(bre);
-        cudaFree(bim);
+        OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 14 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (forces)
+            OFDFT_CK(cudaMemcpyAsync(Fall.data(), d_F, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, st));
+        OFDFT_CK(cudaStreamSynchronize(st));
+        e_rec = 4.0 * M_PI * g->h_results[7] / g->volume;
+        for (int k = 0; k < 6; ++k) s_rec[k] = stress ? g->h_results[8 + k] : 0.0;
     } else {
-        double* S = (double*)sc.get("S", (size_t)g->Nc * 2 * sizeof(double));
+        OFDFT_CK(cudaMemcpyAsync(Fall.data(), d_F, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, st));
+        double* S = (double*)sc.get("ew_S", (size_t)g->Nc * 2 * sizeof(double));
         k_ewald_rec_exact<T><<<g->red_blocks, RED_THREADS, 0, st>>>(d_pos, d_q, nat, g->geo, eta, S, g->d_partials);
         OFDFT_LAUNCH_CHECK();
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 1, 0ull, g->d_results);
+        reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 1, 0ull, g->d_results + 7);
         OFDFT_LAUNCH_CHECK();
-        OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, sizeof(double), cudaMemcpyDeviceToHost, st));
+        OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
         OFDFT_CK(cudaStreamSynchronize(st));
-        e_rec = 4.0 * M_PI * g->h_results[0] / g->volume;
+        e_rec = 4.0 * M_PI * g->h_results[7] / g->volume;
         if (stress) {
             k_ewald_stress_rec<T><<<g->red_blocks, RED_THREADS, 0, st>>>(nullptr, S, nullptr, nullptr, g->geo, eta,
                                                                          g->d_partials);
             OFDFT_LAUNCH_CHECK();
-            reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results);
+            reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results + 8);
             OFDFT_LAUNCH_CHECK();
-            OFDFT_CK(cudaMemcpyAsync(s_rec, g->d_results, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
+            OFDFT_CK(cudaMemcpyAsync(s_rec, g->d_results + 8, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
             OFDFT_CK(cudaStreamSynchronize(st));
         }
         if (forces) {
@@ -406,22 +479,26 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
                                                                            g->d_partials);
                 OFDFT_LAUNCH_CHECK();
                 reduce_finalize<<<3 * kChunk, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 3 * kChunk, 0ull,
-                                                           g->d_results);
+                                                           g->d_results + 16);
                 OFDFT_LAUNCH_CHECK();
-                OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 3 * kChunk * sizeof(double),
+                OFDFT_CK(cudaMemcpyAsync(g->h_results + 16, g->d_results + 16, 3 * kChunk * sizeof(double),
                                          cudaMemcpyDeviceToHost, st));
                 OFDFT_CK(cudaStreamSynchronize(st));
                 for (int t = 0; t < na; ++t)
-                    for (int c = 0; c < 3; ++c) Frec[3 * (a0 + t) + c] = g->h_results[3 * t + c] * 8.0 * M_PI / g->volume;
+                    for (int c = 0; c < 3; ++c)
+                        Fall[3 * (n + a0 + t) + c] = g->h_results[16 + 3 * t + c] * 8.0 * M_PI / g->volume;
             }
         }
     }
+    const double e_real = g->h_results[0] / 2.0;
+    double s_real[6];
+    for (int k = 0; k < 6; ++k) s_real[k] = g->h_results[1 + k] * (-0.5 / g->volume);
     out_energy[0] = e_corr + e_real + e_rec;
     out_energy[1] = e_real;
     out_energy[2] = e_rec;
     out_energy[3] = e_corr;
     if (forces)
-        for (size_t k = 0; k < 3 * (size_t)nat; ++k) forces[k] = Freal[k] + Frec[k];
+        for (size_t k = 0; k < 3 * n; ++k) forces[k] = Fall[k] + Fall[3 * n + k];
     if (stress) {
         // both reciprocal forms reduce to 4 pi / V^2 times the mask sums (the PME
         // form's 2 x 2 pi / V^2 / dV^2 with the dV^2 of its transforms); the G = 0

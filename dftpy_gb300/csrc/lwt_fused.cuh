@@ -277,10 +277,8 @@ __global__ void __launch_bounds__(kFzLines * (N1 / kFzColE))
         const unsigned* w = need.of(i0, j);
         unsigned b = 0;
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int i1 = t + T * e;
-            b |= ((__ldg(w + (i1 >> 5)) >> (i1 & 31)) & 1u) << e;
-        }
+        for (int e = 0; e < E; ++e)  // t < T, and T divides 32
+            b |= ((__ldg(w + (T * e >> 5)) >> ((T * e & 31) + t)) & 1u) << e;
         return b;
     };
     if (tile < tiles_main) {

@@ -6,10 +6,7 @@
 #pragma once
 #include "common.cuh"
 
-#include <algorithm>
-#include <cmath>
 #include <string>
-#include <vector>
 
 namespace ofdft {
 
@@ -34,179 +31,195 @@ __device__ inline int pmod(long long a, int n) {
     return (int)(r < 0 ? r + n : r);
 }
 
-// ---------------------------------------------------------------------------
-// Deterministic spreading.  The grid is cut into 8^3 tiles; the host lists, for
-// every tile that some atom's order^3 stencil touches, the atoms (positions in
-// the spread list) that touch it, in list order.  One block per touched tile,
-// one thread per grid point: the thread sums the contributions of its tile's
-// atoms in that order in float64 and stores the point once.  The sum at every
-// point therefore has a fixed order and Q is the same bits on every run (a
-// per-atom scatter with global atomics sums in arrival order).
-constexpr int kPmeTile = 8;
-
-struct PmeTiles {
-    int ntiles = 0, nlist = 0, order = 0;
-    int* tile = nullptr;   // tile ids (t0 T1 + t1) T2 + t2
-    int* start = nullptr;  // ntiles + 1 offsets into atom
-    int* atom = nullptr;   // list positions
-    int* base = nullptr;   // 3 per list position: floor(u_d)
-    double* M = nullptr;   // 3 (order + 1) per list position: M_order(x + n - 1), n = 0..order
-};
-
-// Builds the tile lists on the host and uploads them into buffers of sc named
-// prefix + "...".  frac: 3 per atom of the whole set (host); list: the atoms to
-// spread (host, nullptr = 0..nlist-1).  The stencil base floor(frac n) is the
-// same IEEE product and floor the device computes.
-inline PmeTiles pme_tiles_build(Scratch& sc, const std::string& prefix, const double* frac, const int* list,
-                                int nlist, int order, const int nr[3], cudaStream_t st) {
-    PmeTiles t;
-    t.nlist = nlist;
-    t.order = order;
-    if (nlist <= 0) return t;
-    int nt[3];
-    for (int d = 0; d < 3; ++d) nt[d] = (nr[d] + kPmeTile - 1) / kPmeTile;
-    std::vector<long long> key;
-    key.reserve((size_t)nlist * 27);
-    for (int q = 0; q < nlist; ++q) {
-        const int a = list ? list[q] : q;
-        std::vector<int> tl[3];
-        for (int d = 0; d < 3; ++d) {
-            const long long b = (long long)std::floor(frac[3 * (size_t)a + d] * (double)nr[d]);
-            for (int i = 0; i < order; ++i) {
-                long long l = (1 + b - i) % nr[d];
-                if (l < 0) l += nr[d];
-                const int tt = (int)(l / kPmeTile);
-                if (std::find(tl[d].begin(), tl[d].end(), tt) == tl[d].end()) tl[d].push_back(tt);
-            }
-        }
-        for (int x : tl[0])
-            for (int y : tl[1])
-                for (int z : tl[2]) key.push_back((((long long)x * nt[1] + y) * nt[2] + z) * nlist + q);
+// B-spline values with one lane per n: lane n - 1 of a group of 16 holds M_i(x + n - 1)
+// after step i, the same recursion step by step (and the same roundings).  before: the
+// values of order - 1 (what the derivatives need).
+__device__ __forceinline__ double bspline_mn_lane(double x, int order, int n, double& before) {
+    double v = n == 1 ? x : (n == 2 ? 1.0 - x : 0.0);
+    before = v;
+    for (int i = 3; i <= order; ++i) {
+        before = v;
+        double below = __shfl_up_sync(0xffffffffu, v, 1, 16);
+        if (n == 1) below = 0.0;
+        const int j = i - n;
+        double w = (x + n - 1) * v + (j + 1 - x) * below;
+        w /= (double)(i - 1);
+        v = n <= i ? w : 0.0;
     }
-    std::sort(key.begin(), key.end());
-    std::vector<int> tile, start, atom(key.size());
-    for (size_t p = 0; p < key.size(); ++p) {
-        const int tid = (int)(key[p] / nlist);
-        atom[p] = (int)(key[p] % nlist);
-        if (tile.empty() || tile.back() != tid) {
-            tile.push_back(tid);
-            start.push_back((int)p);
-        }
-    }
-    start.push_back((int)key.size());
-    t.ntiles = (int)tile.size();
-    t.tile = (int*)sc.get(prefix + "tile", tile.size() * sizeof(int));
-    t.start = (int*)sc.get(prefix + "start", start.size() * sizeof(int));
-    t.atom = (int*)sc.get(prefix + "atom", atom.size() * sizeof(int));
-    t.base = (int*)sc.get(prefix + "base", 3 * (size_t)nlist * sizeof(int));
-    t.M = (double*)sc.get(prefix + "M", 3 * (size_t)(order + 1) * nlist * sizeof(double));
-    OFDFT_CK(cudaMemcpyAsync(t.tile, tile.data(), tile.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(t.start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    OFDFT_CK(cudaMemcpyAsync(t.atom, atom.data(), atom.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    // the host vectors die with this call: let the copies finish first
-    OFDFT_CK(cudaStreamSynchronize(st));
-    return t;
+    return v;
 }
 
-// stencil base and B-spline weights of every list position (one thread each)
+// ---------------------------------------------------------------------------
+// Deterministic spreading.  The grid is cut into 8^3 tiles, one block each, one thread per
+// grid point.  The block goes through the atoms in list order, 512 at a time: every thread
+// tests one atom's order^3 stencil against the tile, the hits are compacted in order into
+// shared memory, and every thread sums their contributions in that order in float64 and
+// stores its point once.  The sum at every point has a fixed order, so Q is the same bits on
+// every run (a per-atom scatter with global atomics sums in arrival order).  The test costs
+// tiles x atoms comparisons, 67 million for 2048 atoms on 256^3 (about 30 us); lists built
+// and sorted on the host took 2.5 ms there.
+constexpr int kPmeTile = 8;
+constexpr int kPmeThreads = kPmeTile * kPmeTile * kPmeTile;
+
+// Stencil base and B-spline weights of every list position: 16 lanes per atom and axis
 static __global__ void k_pme_prep(const double* __restrict__ frac, const int* __restrict__ list, int nlist, int order,
                                   Geo geo, int* base, double* M) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nlist) return;
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, n = (threadIdx.x & 15) + 1;
+    const bool on = g < 3 * nlist;
+    const int q = on ? g / 3 : 0, d = on ? g - 3 * q : 0;
     const int a = list ? list[q] : q;
-    for (int d = 0; d < 3; ++d) {
-        const int n = d == 0 ? geo.n0 : (d == 1 ? geo.n1 : geo.n2);
-        const double up = frac[3 * a + d] * (double)n;
-        const double fl = floor(up);
-        bspline_mn_dev(up - fl, order, M + (3 * (size_t)q + d) * (order + 1));
-        base[3 * q + d] = (int)fl;
+    const int nr = d == 0 ? geo.n0 : (d == 1 ? geo.n1 : geo.n2);
+    const double up = frac[3 * a + d] * (double)nr;
+    const double fl = floor(up);
+    double before;
+    const double v = bspline_mn_lane(up - fl, order, n, before);
+    if (!on) return;
+    double* out = M + (size_t)g * (order + 1);
+    if (n <= order) out[n] = v;
+    if (n == 1) {
+        out[0] = 0.0;
+        base[g] = (int)fl;
     }
 }
 
-// Q at every point of a touched tile: sum over the tile's atoms, in list order,
-// of w_a M0(i) M1(j) M2(k) with i = (1 + base_0 - l0) mod n0 (< order), etc.
+// Q at every point of a tile: sum over the atoms that touch it, in list order, of
+// w_a M0(i) M1(j) M2(k) with i = (1 + base_0 - l0) mod n0 (< order), etc.
 template <typename T>
-__global__ void __launch_bounds__(kPmeTile* kPmeTile* kPmeTile)
-    k_pme_tiles(PmeTiles t, const double* __restrict__ w, const int* __restrict__ list, Geo geo, T* Q) {
-    const int tid = t.tile[blockIdx.x];
+__global__ void __launch_bounds__(kPmeThreads)
+    k_pme_tiles(int nlist, int order, const int* __restrict__ base, const double* __restrict__ M,
+                const double* __restrict__ w, const int* __restrict__ list, Geo geo, T* Q) {
+    __shared__ int hit[kPmeThreads];
+    __shared__ int off[kPmeThreads][3];  // (1 + base - first point of the tile) mod n per axis
+    __shared__ int count[kPmeThreads / 32];
     const int T1 = (geo.n1 + kPmeTile - 1) / kPmeTile, T2 = (geo.n2 + kPmeTile - 1) / kPmeTile;
-    const int l0 = (tid / (T1 * T2)) * kPmeTile + (threadIdx.x >> 6);
-    const int l1 = ((tid / T2) % T1) * kPmeTile + ((threadIdx.x >> 3) & 7);
-    const int l2 = (tid % T2) * kPmeTile + (threadIdx.x & 7);
-    if (l0 >= geo.n0 || l1 >= geo.n1 || l2 >= geo.n2) return;
-    const int order = t.order, o1 = order + 1;
+    const int tid = blockIdx.x, nr[3] = {geo.n0, geo.n1, geo.n2};
+    const int lo[3] = {(tid / (T1 * T2)) * kPmeTile, ((tid / T2) % T1) * kPmeTile, (tid % T2) * kPmeTile};
+    const int p[3] = {(int)(threadIdx.x >> 6), (int)((threadIdx.x >> 3) & 7), (int)(threadIdx.x & 7)};
+    const bool in = lo[0] + p[0] < nr[0] && lo[1] + p[1] < nr[1] && lo[2] + p[2] < nr[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o1 = order + 1;
     double v = 0.0;
-    for (int p = t.start[blockIdx.x]; p < t.start[blockIdx.x + 1]; ++p) {
-        const int q = t.atom[p];
-        const int* b = t.base + 3 * q;
-        const double* M0 = t.M + (3 * (size_t)q) * o1;
-        const double* M1 = M0 + o1;
-        const double* M2 = M1 + o1;
-        const double wa = w ? w[list ? list[q] : q] : 1.0;
-        // n >= order in practice; the loops also cover a stencil that wraps onto itself
-        for (int i = pmod(1LL + b[0] - l0, geo.n0); i < order; i += geo.n0)
-            for (int j = pmod(1LL + b[1] - l1, geo.n1); j < order; j += geo.n1)
-                for (int k = pmod(1LL + b[2] - l2, geo.n2); k < order; k += geo.n2)
-                    v += wa * M0[i + 1] * M1[j + 1] * M2[k + 1];
+    for (int q0 = 0; q0 < nlist; q0 += kPmeThreads) {
+        const int q = q0 + threadIdx.x;
+        int o[3] = {0, 0, 0};
+        bool on = q < nlist;
+        if (on) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                int t = 1 + base[3 * q + d] - lo[d];  // base in [0, n): t in (-n, n]
+                t = t < 0 ? t + nr[d] : (t >= nr[d] ? t - nr[d] : t);
+                o[d] = t;
+                on = on && t <= order + min(kPmeTile, nr[d] - lo[d]) - 2;
+            }
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        __syncthreads();  // the previous chunk's list is done with
+        if (lane == 0) count[warp] = __popc(b);
+        __syncthreads();
+        int at = 0, total = 0;
+#pragma unroll
+        for (int k = 0; k < kPmeThreads / 32; ++k) {
+            const int c = count[k];
+            at += k < warp ? c : 0;
+            total += c;
+        }
+        if (on) {
+            at += __popc(b & ((1u << lane) - 1u));
+            hit[at] = q;
+            off[at][0] = o[0];
+            off[at][1] = o[1];
+            off[at][2] = o[2];
+        }
+        __syncthreads();
+        if (!in) continue;
+        for (int h = 0; h < total; ++h) {
+            int i0 = off[h][0] - p[0], j0 = off[h][1] - p[1], k0 = off[h][2] - p[2];
+            i0 += i0 < 0 ? nr[0] : 0;
+            j0 += j0 < 0 ? nr[1] : 0;
+            k0 += k0 < 0 ? nr[2] : 0;
+            if (i0 >= order || j0 >= order || k0 >= order) continue;
+            const int a = hit[h];
+            const double* M0 = M + (3 * (size_t)a) * o1;
+            const double* M1 = M0 + o1;
+            const double* M2 = M1 + o1;
+            const double wa = w ? w[list ? list[a] : a] : 1.0;
+            // n >= order in practice; the loops also cover a stencil that wraps onto itself
+            for (int i = i0; i < order; i += nr[0])
+                for (int j = j0; j < order; j += nr[1])
+                    for (int k = k0; k < order; k += nr[2]) v += wa * M0[i + 1] * M1[j + 1] * M2[k + 1];
+        }
     }
-    Q[((long long)l0 * geo.n1 + l1) * geo.n2 + l2] = (T)v;
+    if (in) Q[((long long)(lo[0] + p[0]) * geo.n1 + lo[1] + p[1]) * geo.n2 + lo[2] + p[2]] = (T)v;
 }
 
-// Q = the spread of the list (Q zeroed here); t from pme_tiles_build with the
-// same list and order.  d_frac, d_list, d_w on the device (d_list, d_w may be null).
+// Q = the spread of the list's atoms with weights w (null: 1).  d_frac, d_list and d_w on
+// the device (d_list and d_w may be null); work buffers of sc named prefix + "...".
 template <typename T>
-void pme_spread(const PmeTiles& t, const double* d_frac, const int* d_list, const double* d_w, const Geo& geo, T* Q,
-                size_t qbytes, cudaStream_t st) {
-    OFDFT_CK(cudaMemsetAsync(Q, 0, qbytes, st));
-    if (t.nlist <= 0 || t.ntiles <= 0) return;
-    k_pme_prep<<<(t.nlist + 127) / 128, 128, 0, st>>>(d_frac, d_list, t.nlist, t.order, geo, t.base, t.M);
+void pme_spread(Scratch& sc, const std::string& prefix, int nlist, int order, const double* d_frac, const int* d_list,
+                const double* d_w, const Geo& geo, T* Q, cudaStream_t st) {
+    const size_t qbytes = (size_t)geo.N * sizeof(T);
+    if (nlist <= 0) {
+        OFDFT_CK(cudaMemsetAsync(Q, 0, qbytes, st));
+        return;
+    }
+    int* base = (int*)sc.get(prefix + "base", 3 * (size_t)nlist * sizeof(int));
+    double* M = (double*)sc.get(prefix + "M", 3 * (size_t)(order + 1) * nlist * sizeof(double));
+    const int groups = 3 * nlist;
+    k_pme_prep<<<(groups + 7) / 8, 128, 0, st>>>(d_frac, d_list, nlist, order, geo, base, M);
     OFDFT_LAUNCH_CHECK();
-    k_pme_tiles<T><<<t.ntiles, kPmeTile * kPmeTile * kPmeTile, 0, st>>>(t, d_w, d_list, geo, Q);
+    auto tiles = [](int n) { return (n + kPmeTile - 1) / kPmeTile; };
+    const unsigned nt = (unsigned)tiles(geo.n0) * tiles(geo.n1) * tiles(geo.n2);
+    k_pme_tiles<T><<<nt, kPmeThreads, 0, st>>>(nlist, order, base, M, d_w, d_list, geo, Q);
     OFDFT_LAUNCH_CHECK();
 }
 
 // One block per atom: g_a = sum_{ijk} (dQ/du . cinv) * field[l(ijk)], the PME
 // gradient of _ForcePME / Forces_rec_PME with dQ_d = n_d dM_d (M_{order-1}
 // differences) times the other two M_order factors.  out[3a+c] = scale_a * g_c.
+// A thread takes the k2 row of one (i, j): sums of the row with M2 and with dM2 (two
+// operations per point), then its three products.
+constexpr int kGatherThreads = 128;
 template <typename T>
-__global__ void k_pme_gather(const double* __restrict__ frac, const int* __restrict__ sel, int order, Geo geo,
-                             const T* __restrict__ field, const double* __restrict__ cinv,
-                             const double* __restrict__ scale, double* out) {
-    __shared__ double M[3][kMaxOrder + 1];
-    __shared__ double dM[3][kMaxOrder + 1];
-    __shared__ int base[3];
-    __shared__ double red[3][RED_THREADS / 32];
+__global__ void __launch_bounds__(kGatherThreads)
+    k_pme_gather(const double* __restrict__ frac, const int* __restrict__ sel, int order, Geo geo,
+                 const T* __restrict__ field, const double* __restrict__ cinv, const double* __restrict__ scale,
+                 double* out) {
+    __shared__ double M[3][kMaxOrder];
+    __shared__ double dM[3][kMaxOrder];
+    __shared__ int at[3][kMaxOrder];
+    __shared__ double red[3][kGatherThreads / 32];
     const int a = sel ? sel[blockIdx.x] : blockIdx.x;
-    if (threadIdx.x < 3) {
-        const int d = threadIdx.x;
-        const int n = d == 0 ? geo.n0 : (d == 1 ? geo.n1 : geo.n2);
-        double up = frac[3 * a + d] * (double)n;
-        double fl = floor(up);
-        double M2[kMaxOrder + 1];
-        bspline_mn_dev(up - fl, order, M[d]);
-        bspline_mn_dev(up - fl, order - 1, M2);
-        M2[order] = 0.0;
-        for (int i = 0; i < order; ++i) dM[d][i] = (double)n * (M2[i + 1] - M2[i]);
-        base[d] = (int)fl;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x < 64) {  // two whole warps: the fourth group of 16 repeats an axis
+        const int d = (int)(threadIdx.x >> 4) % 3, n = (threadIdx.x & 15) + 1;
+        const int nr = d == 0 ? geo.n0 : (d == 1 ? geo.n1 : geo.n2);
+        const double up = frac[3 * a + d] * (double)nr, fl = floor(up);
+        double before;
+        const double v = bspline_mn_lane(up - fl, order, n, before);
+        // dM[i] = n_d (M_{order-1}(i+1) - M_{order-1}(i)), M_{order-1}(0) = M_{order-1}(order) = 0
+        const double mine = n < order ? before : 0.0;
+        double below = __shfl_up_sync(0xffffffffu, mine, 1, 16);
+        if (n == 1) below = 0.0;
+        if (n <= order && threadIdx.x < 48) {
+            M[d][n - 1] = v;
+            dM[d][n - 1] = (double)nr * (mine - below);
+            at[d][n - 1] = pmod(1LL + (long long)fl - (n - 1), nr);
+        }
     }
     __syncthreads();
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    const int o3 = order * order * order;
-    for (int t = threadIdx.x; t < o3; t += blockDim.x) {
-        int i = t / (order * order), j = (t / order) % order, k = t % order;
-        int l0 = pmod(1LL + base[0] - i, geo.n0);
-        int l1 = pmod(1LL + base[1] - j, geo.n1);
-        int l2 = pmod(1LL + base[2] - k, geo.n2);
-        double f = (double)field[((long long)l0 * geo.n1 + l1) * geo.n2 + l2];
-        double q0 = dM[0][i] * M[1][j + 1] * M[2][k + 1];
-        double q1 = M[0][i + 1] * dM[1][j] * M[2][k + 1];
-        double q2 = M[0][i + 1] * M[1][j + 1] * dM[2][k];
-        // (dQ . cinv)_c = sum_d dQ_d cinv[d][c]
-        g0 += (q0 * cinv[0] + q1 * cinv[3] + q2 * cinv[6]) * f;
-        g1 += (q0 * cinv[1] + q1 * cinv[4] + q2 * cinv[7]) * f;
-        g2 += (q0 * cinv[2] + q1 * cinv[5] + q2 * cinv[8]) * f;
+    for (int t = threadIdx.x; t < order * order; t += kGatherThreads) {
+        const int i = t / order, j = t - i * order;
+        const T* row = field + ((long long)at[0][i] * geo.n1 + at[1][j]) * geo.n2;
+        double s = 0.0, e = 0.0;
+        for (int k = 0; k < order; ++k) {
+            const double f = (double)row[at[2][k]];
+            s += M[2][k] * f;
+            e += dM[2][k] * f;
+        }
+        g0 += dM[0][i] * M[1][j] * s;
+        g1 += M[0][i] * dM[1][j] * s;
+        g2 += M[0][i] * M[1][j] * e;
     }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) {
         g0 += __shfl_down_sync(0xffffffffu, g0, o);
         g1 += __shfl_down_sync(0xffffffffu, g1, o);
@@ -218,18 +231,60 @@ __global__ void k_pme_gather(const double* __restrict__ frac, const int* __restr
         red[2][wid] = g2;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 3) {
         double s0 = 0, s1 = 0, s2 = 0;
-        for (int w = 0; w < (int)(blockDim.x / 32); ++w) {
+        for (int w = 0; w < kGatherThreads / 32; ++w) {
             s0 += red[0][w];
             s1 += red[1][w];
             s2 += red[2][w];
         }
-        const double sc = scale ? scale[a] : 1.0;
-        out[3 * a + 0] = sc * s0;
-        out[3 * a + 1] = sc * s1;
-        out[3 * a + 2] = sc * s2;
+        // (dQ . cinv)_c = sum_d dQ_d cinv[d][c]
+        const int c = threadIdx.x;
+        out[3 * a + c] = (scale ? scale[a] : 1.0) * (s0 * cinv[c] + s1 * cinv[3 + c] + s2 * cinv[6 + c]);
     }
+}
+
+// One warp per row (i, j) of the half grid, lanes along k: what a row shares is computed
+// once per row instead of once per point.
+struct HalfRow {
+    int i, j;
+    double px, py, pz;  // f0 b0 + f1 b1, rounded as gvec rounds it
+    double xr, xi;      // bm0(i) bm1(j)
+};
+__device__ __forceinline__ HalfRow half_row(const Geo& g, int row, const double* bre, const double* bim) {
+    HalfRow r;
+    r.i = row / g.n1;
+    r.j = row - r.i * g.n1;
+    const double f0 = __dmul_rn((double)freq_index(r.i, g.n0), g.fv[0]);
+    const double f1 = __dmul_rn((double)freq_index(r.j, g.n1), g.fv[1]);
+    r.px = __dadd_rn(__dmul_rn(f0, g.b[0]), __dmul_rn(f1, g.b[3]));
+    r.py = __dadd_rn(__dmul_rn(f0, g.b[1]), __dmul_rn(f1, g.b[4]));
+    r.pz = __dadd_rn(__dmul_rn(f0, g.b[2]), __dmul_rn(f1, g.b[5]));
+    r.xr = r.xi = 0.0;
+    if (bre) {
+        const double ar = bre[r.i], ai = bim[r.i], cr = bre[g.n0 + r.j], ci = bim[g.n0 + r.j];
+        r.xr = ar * cr - ai * ci;
+        r.xi = ar * ci + ai * cr;
+    }
+    return r;
+}
+// |G|^2 of element k of the row, the bits of gsq()
+__device__ __forceinline__ double row_gsq(const Geo& g, const HalfRow& r, int k) {
+    const double f2 = __dmul_rn((double)k, g.fv[2]);
+    const double gx = __dadd_rn(r.px, __dmul_rn(f2, g.b[6]));
+    const double gy = __dadd_rn(r.py, __dmul_rn(f2, g.b[7]));
+    const double gz = __dadd_rn(r.pz, __dmul_rn(f2, g.b[8]));
+    return __dadd_rn(__dadd_rn(__dmul_rn(gx, gx), __dmul_rn(gy, gy)), __dmul_rn(gz, gz));
+}
+__device__ __forceinline__ void row_barray(const Geo& g, const HalfRow& r, const double* bre, const double* bim, int k,
+                                           double& br, double& bi) {
+    const double er = bre[g.n0 + g.n1 + k], ei = bim[g.n0 + g.n1 + k];
+    br = r.xr * er - r.xi * ei;
+    bi = r.xr * ei + r.xi * er;
+}
+constexpr int kRowWarps = 8;  // warps (rows) per block of the row kernels
+inline int row_grid(const Geo& g, int sms) {
+    return blocks_for((long long)g.n0 * g.n1, kRowWarps, sms * 16);
 }
 
 // B(G) = bm0(i) bm1(j) bm2(k) from per-axis complex tables (ewald.py:44-55)

@@ -3,6 +3,7 @@
 // splines of the tabulated potential, the structure factor by smooth PME
 // (B-spline spreading + R2C) or exactly, and the forces of both paths.
 #include "common.cuh"
+#include "fix_eval.h"
 #include "host_math.h"
 #include "pme.cuh"
 
@@ -22,12 +23,36 @@ struct Line {
     int n;             // number of knots
     double gp1, gplast, dp;
     double v0, v1, v2;  // vp[0..2] for the quartic near q = 0
+    float x0, inv;      // first knot and intervals per unit length of a uniform table
 };
 
 struct Lines {
     Line s[kMaxSpecies];
     int ns;
 };
+
+// The largest i with x[i] <= q, clamped to [0, n-2].  Tables are uniform: a float32 guess is
+// the interval or its neighbour; a binary search (a dozen float64 comparisons on the slow
+// pipe) serves any other table.
+__device__ __forceinline__ int knot_of(const Line& L, double q) {
+    int lo = min(max((int)(((float)q - L.x0) * L.inv), 0), L.n - 2);
+    if (L.x[lo] > q) {
+        if (lo > 0) --lo;
+    } else if (lo < L.n - 2 && L.x[lo + 1] <= q) {
+        ++lo;
+    }
+    const bool fits = (lo == 0 || L.x[lo] <= q) && (lo == L.n - 2 || q < L.x[lo + 1]);
+    if (!fits) {
+        lo = 0;
+        int hi = L.n - 1;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (L.x[mid] <= q) lo = mid;
+            else hi = mid;
+        }
+    }
+    return lo;
+}
 
 // LocalPseudo.calc_vlines (pseudo/__init__.py:398-423)
 __device__ inline double vline_eval(const Line& L, double q) {
@@ -43,12 +68,7 @@ __device__ inline double vline_eval(const Line& L, double q) {
         return t0 + dx * (t1 + dx * (t2 + dx * (t3 + dx * t4))) / 24.0;
     }
     if (q < L.gplast) {
-        int lo = 0, hi = L.n - 1;  // largest i with x[i] <= q, clamped to [0, n-2]
-        while (hi - lo > 1) {
-            int mid = (lo + hi) >> 1;
-            if (L.x[mid] <= q) lo = mid;
-            else hi = mid;
-        }
+        const int lo = knot_of(L, q);
         double u = q - L.x[lo];
         const double* c = L.c + 4 * (long long)lo;
         return c[0] + u * (c[1] + u * (c[2] + u * c[3]));
@@ -56,25 +76,32 @@ __device__ inline double vline_eval(const Line& L, double q) {
     return 0.0;
 }
 
-// v(G) (+)= vline_s(|G|) * F(G) * B(G) * scale   (PME, _PP_Reciprocal_PME :437-452)
+// v(G) (+)= vline_s(|G|) * F(G) * B(G) * scale   (PME, _PP_Reciprocal_PME :437-452); the
+// radial values go to vl, for the forces at the same geometry
 template <typename T>
-__global__ void k_pp_accum_pme(const typename Cplx<T>::type* __restrict__ QG, typename Cplx<T>::type* vG, Line L,
-                               const double* bre, const double* bim, int first, Geo geo, double scale) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < geo.Nc; i += stride) {
-        double q = sqrt(gsq(geo, i));
-        double vl = vline_eval(L, q);
-        double br, bi;
-        barray(bre, bim, geo, i, br, bi);
-        double qr = (double)QG[i].x, qi = (double)QG[i].y;
-        double xr = vl * (qr * br - qi * bi) * scale;
-        double xi = vl * (qr * bi + qi * br) * scale;
-        if (!first) {
-            xr += (double)vG[i].x;
-            xi += (double)vG[i].y;
+__global__ void __launch_bounds__(32 * kRowWarps)
+    k_pp_accum_pme(const typename Cplx<T>::type* __restrict__ QG, typename Cplx<T>::type* vG, Line L, const double* bre,
+                   const double* bim, int first, Geo geo, double scale, double* __restrict__ vlg) {
+    const int rows = geo.n0 * geo.n1;
+    for (int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kRowWarps) {
+        const HalfRow r = half_row(geo, row, bre, bim);
+        for (int k = threadIdx.x & 31; k < geo.n2h; k += 32) {
+            const long long i = (long long)row * geo.n2h + k;
+            double q = sqrt(row_gsq(geo, r, k));
+            double vl = vline_eval(L, q);
+            vlg[i] = vl;
+            double br, bi;
+            row_barray(geo, r, bre, bim, k, br, bi);
+            double qr = (double)QG[i].x, qi = (double)QG[i].y;
+            double xr = vl * (qr * br - qi * bi) * scale;
+            double xi = vl * (qr * bi + qi * br) * scale;
+            if (!first) {
+                xr += (double)vG[i].x;
+                xi += (double)vG[i].y;
+            }
+            vG[i].x = (T)xr;
+            vG[i].y = (T)xi;
         }
-        vG[i].x = (T)xr;
-        vG[i].y = (T)xi;
     }
 }
 
@@ -102,22 +129,27 @@ __global__ void k_pp_exact(typename Cplx<T>::type* vG, Lines LS, const double* _
     }
 }
 
-// rho(G) conj(B(G)) vline_s(|G|) / N with G = 0 removed (_ForcePME :527-536)
+// rho(G) conj(B(G)) vline_s(|G|) / N with G = 0 removed (_ForcePME :527-536); vlg: the
+// radial values that k_pp_accum_pme left, or null
 template <typename T>
-__global__ void k_pp_force_pme(const typename Cplx<T>::type* __restrict__ rhoG, typename Cplx<T>::type* out, Line L,
-                               const double* bre, const double* bim, Geo geo, double scale) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < geo.Nc; i += stride) {
-        double q = sqrt(gsq(geo, i));
-        double vl = vline_eval(L, q);
-        double br, bi;
-        barray(bre, bim, geo, i, br, bi);
-        double qr = (double)rhoG[i].x, qi = (double)rhoG[i].y;
-        double xr = vl * (qr * br + qi * bi) * scale;   // rho * conj(B)
-        double xi = vl * (qi * br - qr * bi) * scale;
-        if (i == 0) xr = xi = 0.0;
-        out[i].x = (T)xr;
-        out[i].y = (T)xi;
+__global__ void __launch_bounds__(32 * kRowWarps)
+    k_pp_force_pme(const typename Cplx<T>::type* __restrict__ rhoG, typename Cplx<T>::type* out, Line L,
+                   const double* bre, const double* bim, Geo geo, double scale, const double* __restrict__ vlg) {
+    const int rows = geo.n0 * geo.n1;
+    for (int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kRowWarps) {
+        const HalfRow r = half_row(geo, row, bre, bim);
+        for (int k = threadIdx.x & 31; k < geo.n2h; k += 32) {
+            const long long i = (long long)row * geo.n2h + k;
+            const double vl = vlg ? vlg[i] : vline_eval(L, sqrt(row_gsq(geo, r, k)));
+            double br, bi;
+            row_barray(geo, r, bre, bim, k, br, bi);
+            double qr = (double)rhoG[i].x, qi = (double)rhoG[i].y;
+            double xr = vl * (qr * br + qi * bi) * scale;   // rho * conj(B)
+            double xi = vl * (qi * br - qr * bi) * scale;
+            if (i == 0) xr = xi = 0.0;
+            out[i].x = (T)xr;
+            out[i].y = (T)xi;
+        }
     }
 }
 
@@ -160,41 +192,58 @@ __global__ void __launch_bounds__(RED_THREADS) k_pp_force_exact(const typename C
 // Per G this kernel adds h = (dV/V) w_G Re(S conj rho) times the derivative of
 // vline with respect to the quartic's three values, or times u^p (p = 0..3) to
 // the spline interval holding |G|; the host applies the spline adjoint.
+// The moments of the intervals are summed in shared memory, `copies` of them so that the
+// lanes of a warp rarely meet in one (range intervals can hold a |G|), and added to the
+// result once per block; range = 0: straight into the result, for tables too fine to fit.
+// 160^3 with 256 table points: 1.48 ms per species with every point's atomics in global memory.
 template <typename T>
-__global__ void k_pp_grad_moments(const typename Cplx<T>::type* __restrict__ rhoG,
-                                  const typename Cplx<T>::type* __restrict__ QG, const double* bre,
-                                  const double* bim, Line L, Geo geo, double scale, double* moments,
-                                  double* quart) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < geo.Nc; i += stride) {
-        double q = sqrt(gsq(geo, i));
-        if (q >= L.gplast) continue;
-        double br = 1.0, bi = 0.0;  // no B-spline factor for exact structure factors
-        if (bre) barray(bre, bim, geo, i, br, bi);
-        const double qr = (double)QG[i].x, qi = (double)QG[i].y;
-        const double sr = qr * br - qi * bi, si = qr * bi + qi * br;
-        const int k2 = (int)((unsigned)i % (unsigned)geo.n2h);
-        const double w = (k2 == 0 || (geo.n2 % 2 == 0 && k2 == geo.n2 / 2)) ? 1.0 : 2.0;
-        const double h = scale * w * (sr * (double)rhoG[i].x + si * (double)rhoG[i].y);
-        if (q < L.gp1) {
-            const double dx = q / L.dp, x2 = dx * dx, x4 = x2 * x2;
-            atomicAdd(&quart[0], (1.0 + (-30.0 * x2 + 6.0 * x4) / 24.0) * h);
-            atomicAdd(&quart[1], ((32.0 * x2 - 8.0 * x4) / 24.0) * h);
-            atomicAdd(&quart[2], ((-2.0 * x2 + 2.0 * x4) / 24.0) * h);
-            continue;
+__global__ void __launch_bounds__(32 * kRowWarps)
+    k_pp_grad_moments(const typename Cplx<T>::type* __restrict__ rhoG, const typename Cplx<T>::type* __restrict__ QG,
+                      const double* bre, const double* bim, Line L, Geo geo, double scale, int range, int copies,
+                      double* moments, double* quart) {
+    extern __shared__ double hist[];
+    const int hs = 4 * range + 3;  // one copy: four moments per interval, then the quartic's three
+    for (int t = threadIdx.x; t < copies * hs; t += blockDim.x) hist[t] = 0.0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    double* mo = range ? hist + (lane % copies) * hs : moments;
+    double* qu = range ? mo + 4 * range : quart;
+    const int rows = geo.n0 * geo.n1;
+    for (int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kRowWarps) {
+        const HalfRow r = half_row(geo, row, bre, bim);
+        for (int k = lane; k < geo.n2h; k += 32) {
+            const long long i = (long long)row * geo.n2h + k;
+            const double q = sqrt(row_gsq(geo, r, k));
+            if (q >= L.gplast) continue;
+            double br = 1.0, bi = 0.0;  // no B-spline factor for exact structure factors
+            if (bre) row_barray(geo, r, bre, bim, k, br, bi);
+            const double qr = (double)QG[i].x, qi = (double)QG[i].y;
+            const double sr = qr * br - qi * bi, si = qr * bi + qi * br;
+            const double w = (k == 0 || (geo.n2 % 2 == 0 && k == geo.n2 / 2)) ? 1.0 : 2.0;
+            const double h = scale * w * (sr * (double)rhoG[i].x + si * (double)rhoG[i].y);
+            if (q < L.gp1) {
+                const double dx = q / L.dp, x2 = dx * dx, x4 = x2 * x2;
+                atomicAdd(&qu[0], (1.0 + (-30.0 * x2 + 6.0 * x4) / 24.0) * h);
+                atomicAdd(&qu[1], ((32.0 * x2 - 8.0 * x4) / 24.0) * h);
+                atomicAdd(&qu[2], ((-2.0 * x2 + 2.0 * x4) / 24.0) * h);
+                continue;
+            }
+            const int lo = knot_of(L, q);
+            const double u = q - L.x[lo];
+            double* mp = mo + 4 * (long long)lo;
+            const double hu = h * u, huu = hu * u;
+            atomicAdd(&mp[0], h);
+            atomicAdd(&mp[1], hu);
+            atomicAdd(&mp[2], huu);
+            atomicAdd(&mp[3], huu * u);
         }
-        int lo = 0, hi = L.n - 1;
-        while (hi - lo > 1) {
-            int mid = (lo + hi) >> 1;
-            if (L.x[mid] <= q) lo = mid;
-            else hi = mid;
-        }
-        const double u = q - L.x[lo];
-        double* mp = moments + 4 * (long long)lo;
-        atomicAdd(&mp[0], h);
-        atomicAdd(&mp[1], h * u);
-        atomicAdd(&mp[2], h * u * u);
-        atomicAdd(&mp[3], h * u * u * u);
+    }
+    if (!range) return;
+    __syncthreads();
+    for (int t = threadIdx.x; t < hs; t += blockDim.x) {
+        double s = 0.0;
+        for (int c = 0; c < copies; ++c) s += hist[c * hs + t];
+        if (s != 0.0) atomicAdd(t < 4 * range ? &moments[t] : &quart[t - 4 * range], s);
     }
 }
 
@@ -204,12 +253,7 @@ __global__ void k_pp_grad_moments(const typename Cplx<T>::type* __restrict__ rho
 // below gp[1]); the quartic near q = 0 is not differentiated.
 __device__ inline double vline_deriv(const Line& L, double q) {
     if (!(q < L.gplast)) return 0.0;
-    int lo = 0, hi = L.n - 1;  // largest i with x[i] <= q, clamped to [0, n-2]
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (L.x[mid] <= q) lo = mid;
-        else hi = mid;
-    }
+    const int lo = knot_of(L, q);
     const double u = q - L.x[lo];
     const double* c = L.c + 4 * (long long)lo;
     return c[1] + u * (2.0 * c[2] + u * 3.0 * c[3]);
@@ -328,7 +372,7 @@ struct ofdft_pseudo {
     double* d_bim = nullptr;
     double* d_cinv = nullptr;     // inv(lattice), row-major
     double* d_scale = nullptr;    // per-atom gather scale
-    std::vector<ofdft::PmeTiles> tiles;  // deterministic spreading work list per species (PME)
+    bool have_vl = false;         // sc "vl<s>" holds the radial values on the half grid
     Scratch sc;
 
     Line line(int s) const {
@@ -342,6 +386,8 @@ struct ofdft_pseudo {
         L.v0 = v0[s];
         L.v1 = v1[s];
         L.v2 = v2[s];
+        L.x0 = (float)spl[s].x.front();
+        L.inv = (float)((double)(L.n - 1) / (spl[s].x.back() - spl[s].x.front()));
         return L;
     }
     Lines lines() const {
@@ -393,22 +439,46 @@ void lattice_inverse(const double* a, double* inv) {
 }
 
 // per-axis B-spline Euler factor tables packed [axis0 | axis1 | axis2(half)]
-void bspline_tables(const ofdft_grid* g, int order, double** d_re, double** d_im) {
-    std::vector<double> re, im, r, i;
+void bspline_tables(const ofdft_grid* g, int order, std::vector<double>& re, std::vector<double>& im) {
+    std::vector<double> r, i;
+    re.clear();
+    im.clear();
     for (int d = 0; d < 3; ++d) {
         int nG = d == 2 ? g->n2h : g->nr[d];
         bspline_bm(g->nr[d], nG, order, r, i);
         re.insert(re.end(), r.begin(), r.end());
         im.insert(im.end(), i.begin(), i.end());
     }
-    OFDFT_CK(cudaMalloc(d_re, re.size() * sizeof(double)));
-    OFDFT_CK(cudaMalloc(d_im, im.size() * sizeof(double)));
-    upload_now(*d_re, re.data(), re.size() * sizeof(double));
-    upload_now(*d_im, im.data(), im.size() * sizeof(double));
 }
 }  // namespace ofdft
 
 namespace {
+
+// Transforms whose result does not enter a potential: on the integer pipe in float64
+template <typename T>
+void real_to_half(ofdft_grid* g, const T* in, typename Cplx<T>::type* out, cudaStream_t st) {
+    if constexpr (sizeof(T) == 8) {
+        if (fix::grid_plans(g)) {
+            const double* i = in;
+            double2* o = out;
+            fix::r2c(g, &i, &o, 1, st);
+            return;
+        }
+    }
+    g->exec_r2c(in, out, 1, st);
+}
+template <typename T>
+void half_to_real(ofdft_grid* g, typename Cplx<T>::type* in, T* out, cudaStream_t st) {
+    if constexpr (sizeof(T) == 8) {
+        if (fix::grid_plans(g)) {
+            double2* i = in;
+            double* o = out;
+            fix::c2r(g, &i, &o, 1, st);
+            return;
+        }
+    }
+    g->exec_c2r(in, out, 1, st);
+}
 
 template <typename T>
 void vloc_t(ofdft_pseudo* p, T* out, cudaStream_t st) {
@@ -424,13 +494,15 @@ void vloc_t(ofdft_pseudo* p, T* out, cudaStream_t st) {
         bool first = true;
         for (int s = 0; s < p->ns; ++s) {
             const int n_s = p->sel_off[s + 1] - p->sel_off[s];
-            if (n_s > 0) pme_spread<T>(p->tiles[s], p->d_frac, p->d_sel + p->sel_off[s], nullptr, g->geo, Q, rb, st);
-            else OFDFT_CK(cudaMemsetAsync(Q, 0, rb, st));
+            pme_spread<T>(p->sc, "pme", n_s, p->order, p->d_frac, p->d_sel + p->sel_off[s], nullptr, g->geo, Q, st);
             g->exec_r2c(Q, QG, 1, st);
-            k_pp_accum_pme<T><<<gblk, 256, 0, st>>>(QG, vG, p->line(s), p->d_bre, p->d_bim, first, g->geo, scale);
+            double* vl = (double*)p->sc.get("vl" + std::to_string(s), (size_t)g->Nc * sizeof(double));
+            k_pp_accum_pme<T><<<row_grid(g->geo, g->sms), 32 * kRowWarps, 0, st>>>(
+                QG, vG, p->line(s), p->d_bre, p->d_bim, first, g->geo, scale, vl);
             OFDFT_LAUNCH_CHECK();
             first = false;
         }
+        p->have_vl = true;
     } else {
         k_pp_exact<T><<<gblk, 256, 0, st>>>(vG, p->lines(), p->d_pos, p->d_spec, p->nat, g->geo, scale);
         OFDFT_LAUNCH_CHECK();
@@ -444,8 +516,7 @@ void forces_t(ofdft_pseudo* p, const T* rho, double* F, cudaStream_t st) {
     using C = typename Cplx<T>::type;
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
     C* rhoG = (C*)p->sc.get("rhoG", cb);
-    g->exec_r2c(rho, rhoG, 1, st);
-    const int gblk = blocks_for(g->Nc, 256, g->sms * 16);
+    real_to_half(g, rho, rhoG, st);
     double* dF = (double*)p->sc.get("F", 3 * (size_t)std::max(1, p->nat) * sizeof(double));
     if (p->pme) {
         C* X = (C*)p->sc.get("X", cb);
@@ -453,11 +524,13 @@ void forces_t(ofdft_pseudo* p, const T* rho, double* F, cudaStream_t st) {
         for (int s = 0; s < p->ns; ++s) {
             const int n_s = p->sel_off[s + 1] - p->sel_off[s];
             if (n_s == 0) continue;
-            k_pp_force_pme<T><<<gblk, 256, 0, st>>>(rhoG, X, p->line(s), p->d_bre, p->d_bim, g->geo,
-                                                    1.0 / (double)g->N);
+            const double* vl =
+                p->have_vl ? (double*)p->sc.get("vl" + std::to_string(s), (size_t)g->Nc * sizeof(double)) : nullptr;
+            k_pp_force_pme<T><<<row_grid(g->geo, g->sms), 32 * kRowWarps, 0, st>>>(
+                rhoG, X, p->line(s), p->d_bre, p->d_bim, g->geo, 1.0 / (double)g->N, vl);
             OFDFT_LAUNCH_CHECK();
-            g->exec_c2r(X, rhoPB, 1, st);
-            k_pme_gather<T><<<n_s, 256, 0, st>>>(p->d_frac, p->d_sel + p->sel_off[s], p->order, g->geo, rhoPB,
+            half_to_real(g, X, rhoPB, st);
+            k_pme_gather<T><<<n_s, kGatherThreads, 0, st>>>(p->d_frac, p->d_sel + p->sel_off[s], p->order, g->geo, rhoPB,
                                                  p->d_cinv, p->d_scale, dF);
             OFDFT_LAUNCH_CHECK();
         }
@@ -514,7 +587,7 @@ void stress_t(ofdft_pseudo* p, const T* rho, double energy, double* S, cudaStrea
         for (int s = 0; s < p->ns; ++s) {
             const int n_s = p->sel_off[s + 1] - p->sel_off[s];
             if (n_s == 0) continue;
-            pme_spread<T>(p->tiles[s], p->d_frac, p->d_sel + p->sel_off[s], nullptr, g->geo, Q, rb, st);
+            pme_spread<T>(p->sc, "pme", n_s, p->order, p->d_frac, p->d_sel + p->sel_off[s], nullptr, g->geo, Q, st);
             g->exec_r2c(Q, QG, 1, st);
             k_pp_stress_pme<T><<<g->red_blocks, RED_THREADS, 0, st>>>(rhoG, QG, p->line(s), p->d_bre, p->d_bim,
                                                                       g->geo, g->d_partials);
@@ -543,9 +616,15 @@ void vloc_grad_t(ofdft_pseudo* p, const T* rho, double* grad, cudaStream_t st) {
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
     C* rhoG = (C*)p->sc.get("rhoG", cb);
     C* SG = (C*)p->sc.get("QG", cb);
-    g->exec_r2c(rho, rhoG, 1, st);
+    real_to_half(g, rho, rhoG, st);
     const int gblk = blocks_for(g->Nc, 256, g->sms * 16);
     const double scale = g->dV / g->volume;
+    // no |G| is longer than the sum of the half-axis lengths
+    double gmax = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        const double* b = g->rlattice + 3 * d;
+        gmax += (g->nr[d] / 2) * std::sqrt(b[0] * b[0] + b[1] * b[1] + b[2] * b[2]);
+    }
     size_t off = 0;
     for (int s = 0; s < p->ns; ++s) {
         const int n_s = p->sel_off[s + 1] - p->sel_off[s];
@@ -555,16 +634,27 @@ void vloc_grad_t(ofdft_pseudo* p, const T* rho, double* grad, cudaStream_t st) {
         if (n_s > 0) {
             if (p->pme) {
                 T* Q = (T*)p->sc.get("Q", rb);
-                pme_spread<T>(p->tiles[s], p->d_frac, p->d_sel + p->sel_off[s], nullptr, g->geo, Q, rb, st);
-                g->exec_r2c(Q, SG, 1, st);
-                k_pp_grad_moments<T><<<gblk, 256, 0, st>>>(rhoG, SG, p->d_bre, p->d_bim, p->line(s), g->geo, scale,
-                                                           mom, mom + 4 * (size_t)nint);
+                pme_spread<T>(p->sc, "pme", n_s, p->order, p->d_frac, p->d_sel + p->sel_off[s], nullptr, g->geo, Q, st);
+                real_to_half(g, Q, SG, st);
             } else {
                 k_strf_species<T><<<gblk, 256, 0, st>>>(SG, p->d_pos, p->d_sel + p->sel_off[s], n_s, g->geo);
                 OFDFT_LAUNCH_CHECK();
-                k_pp_grad_moments<T><<<gblk, 256, 0, st>>>(rhoG, SG, nullptr, nullptr, p->line(s), g->geo, scale, mom,
-                                                           mom + 4 * (size_t)nint);
             }
+            // intervals a |G| can fall in; up to 16 copies of their moments in 160 KB
+            const std::vector<double>& x = p->spl[s].x;
+            int range = (int)(std::upper_bound(x.begin(), x.end(), 1.000001 * gmax) - x.begin());
+            range = std::min(nint, std::max(1, range));
+            const size_t one = (4 * (size_t)range + 3) * sizeof(double), most = 160 * 1024;
+            const int copies = (int)std::min<size_t>(16, most / one);
+            if (copies == 0) range = 0;
+            const size_t smem = copies * one;
+            if (smem > 40 * 1024)
+                OFDFT_CK(cudaFuncSetAttribute(k_pp_grad_moments<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)most));
+            const int grid = std::min(row_grid(g->geo, g->sms), 2 * g->sms);
+            k_pp_grad_moments<T><<<grid, 32 * kRowWarps, smem, st>>>(rhoG, SG, p->pme ? p->d_bre : nullptr,
+                                                                     p->pme ? p->d_bim : nullptr, p->line(s), g->geo,
+                                                                     scale, range, copies, mom, mom + 4 * (size_t)nint);
             OFDFT_LAUNCH_CHECK();
         }
         std::vector<double> h(4 * (size_t)nint + 3);
@@ -636,7 +726,12 @@ int ofdft_pseudo_create(ofdft_grid* g, int nspecies, const int* npts, const doub
                 upload_now(dx, S.x.data(), S.x.size() * sizeof(double));
                 upload_now(dc, S.c.data(), S.c.size() * sizeof(double));
             }
-            bspline_tables(g, bspline_order, &p->d_bre, &p->d_bim);
+            std::vector<double> re, im;
+            bspline_tables(g, bspline_order, re, im);
+            OFDFT_CK(cudaMalloc(&p->d_bre, re.size() * sizeof(double)));
+            OFDFT_CK(cudaMalloc(&p->d_bim, im.size() * sizeof(double)));
+            upload_now(p->d_bre, re.data(), re.size() * sizeof(double));
+            upload_now(p->d_bim, im.data(), im.size() * sizeof(double));
             double inv[9];
             lattice_inverse(g->lattice, inv);
             OFDFT_CK(cudaMalloc(&p->d_cinv, 9 * sizeof(double)));
@@ -701,14 +796,6 @@ int ofdft_pseudo_set_ions(ofdft_pseudo* p, int nat, const double* pos, const int
         upload_now(p->d_spec, species, (size_t)nat * sizeof(int));
         upload_now(p->d_sel, sel.data(), (size_t)nat * sizeof(int));
         upload_now(p->d_scale, scale.data(), (size_t)nat * sizeof(double));
-        p->tiles.assign(p->ns, ofdft::PmeTiles());
-        if (p->pme) {
-            const int nr[3] = {p->g->nr[0], p->g->nr[1], p->g->nr[2]};
-            for (int s = 0; s < p->ns; ++s)
-                p->tiles[s] = ofdft::pme_tiles_build(p->sc, "pme" + std::to_string(s) + "_", p->frac.data(),
-                                                     sel.data() + p->sel_off[s], p->sel_off[s + 1] - p->sel_off[s],
-                                                     p->order, nr, cudaStreamPerThread);
-        }
     });
 }
 
