@@ -77,19 +77,24 @@ __device__ inline double vline_eval(const Line& L, double q) {
 }
 
 // v(G) (+)= vline_s(|G|) * F(G) * B(G) * scale   (PME, _PP_Reciprocal_PME :437-452); the
-// radial values go to vl, for the forces at the same geometry
+// radial values on the grid are formed once per handle (have = 0) and kept in vlg, as the
+// reference keeps its vlines
 template <typename T>
 __global__ void __launch_bounds__(32 * kRowWarps)
     k_pp_accum_pme(const typename Cplx<T>::type* __restrict__ QG, typename Cplx<T>::type* vG, Line L, const double* bre,
-                   const double* bim, int first, Geo geo, double scale, double* __restrict__ vlg) {
+                   const double* bim, int first, Geo geo, double scale, double* __restrict__ vlg, int have) {
     const int rows = geo.n0 * geo.n1;
     for (int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kRowWarps) {
         const HalfRow r = half_row(geo, row, bre, bim);
         for (int k = threadIdx.x & 31; k < geo.n2h; k += 32) {
             const long long i = (long long)row * geo.n2h + k;
-            double q = sqrt(row_gsq(geo, r, k));
-            double vl = vline_eval(L, q);
-            vlg[i] = vl;
+            double vl;
+            if (have) {
+                vl = vlg[i];
+            } else {
+                vl = vline_eval(L, sqrt(row_gsq(geo, r, k)));
+                vlg[i] = vl;
+            }
             double br, bi;
             row_barray(geo, r, bre, bim, k, br, bi);
             double qr = (double)QG[i].x, qi = (double)QG[i].y;
@@ -373,6 +378,18 @@ struct ofdft_pseudo {
     double* d_cinv = nullptr;     // inv(lattice), row-major
     double* d_scale = nullptr;    // per-atom gather scale
     bool have_vl = false;         // sc "vl<s>" holds the radial values on the half grid
+    // recorded after the kernels that a call leaves running: moved ions wait for them on the
+    // host, other streams on the device
+    cudaEvent_t busy = nullptr;
+    bool running = false;
+    void follow(cudaStream_t st) {
+        if (running) OFDFT_CK(cudaStreamWaitEvent(st, busy, 0));
+    }
+    void mark(cudaStream_t st) {
+        if (!busy) OFDFT_CK(cudaEventCreateWithFlags(&busy, cudaEventDisableTiming));
+        OFDFT_CK(cudaEventRecord(busy, st));
+        running = true;
+    }
     Scratch sc;
 
     Line line(int s) const {
@@ -485,6 +502,7 @@ void vloc_t(ofdft_pseudo* p, T* out, cudaStream_t st) {
     ofdft_grid* g = p->g;
     using C = typename Cplx<T>::type;
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
+    p->follow(st);
     C* vG = (C*)p->sc.get("vG", cb);
     const int gblk = blocks_for(g->Nc, 256, g->sms * 16);
     const double scale = 1.0 / g->volume;  // irfftn(v)/dV = raw/(N dV)
@@ -498,7 +516,7 @@ void vloc_t(ofdft_pseudo* p, T* out, cudaStream_t st) {
             g->exec_r2c(Q, QG, 1, st);
             double* vl = (double*)p->sc.get("vl" + std::to_string(s), (size_t)g->Nc * sizeof(double));
             k_pp_accum_pme<T><<<row_grid(g->geo, g->sms), 32 * kRowWarps, 0, st>>>(
-                QG, vG, p->line(s), p->d_bre, p->d_bim, first, g->geo, scale, vl);
+                QG, vG, p->line(s), p->d_bre, p->d_bim, first, g->geo, scale, vl, p->have_vl);
             OFDFT_LAUNCH_CHECK();
             first = false;
         }
@@ -508,6 +526,7 @@ void vloc_t(ofdft_pseudo* p, T* out, cudaStream_t st) {
         OFDFT_LAUNCH_CHECK();
     }
     g->exec_c2r(vG, out, 1, st);
+    p->mark(st);
 }
 
 template <typename T>
@@ -515,6 +534,7 @@ void forces_t(ofdft_pseudo* p, const T* rho, double* F, cudaStream_t st) {
     ofdft_grid* g = p->g;
     using C = typename Cplx<T>::type;
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
+    p->follow(st);
     C* rhoG = (C*)p->sc.get("rhoG", cb);
     real_to_half(g, rho, rhoG, st);
     double* dF = (double*)p->sc.get("F", 3 * (size_t)std::max(1, p->nat) * sizeof(double));
@@ -561,6 +581,7 @@ void stress_t(ofdft_pseudo* p, const T* rho, double energy, double* S, cudaStrea
     ofdft_grid* g = p->g;
     using C = typename Cplx<T>::type;
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
+    p->follow(st);
     const double V = g->volume, dV = g->dV;
     if (std::isnan(energy)) {  // E_PP = int v_loc rho dV (LocalPseudo.__call__)
         T* v = (T*)p->sc.get("st_v", rb);
@@ -614,6 +635,7 @@ void vloc_grad_t(ofdft_pseudo* p, const T* rho, double* grad, cudaStream_t st) {
     ofdft_grid* g = p->g;
     using C = typename Cplx<T>::type;
     const size_t cb = g->cplx_bytes(), rb = g->real_bytes();
+    p->follow(st);
     C* rhoG = (C*)p->sc.get("rhoG", cb);
     C* SG = (C*)p->sc.get("QG", cb);
     real_to_half(g, rho, rhoG, st);
@@ -747,16 +769,12 @@ int ofdft_pseudo_create(ofdft_grid* g, int nspecies, const int* npts, const doub
 void ofdft_pseudo_destroy(ofdft_pseudo* p) {
     if (!p) return;
     p->sc.release_all();
+    if (p->busy) cudaEventDestroy(p->busy);
     for (auto x : p->d_x) cudaFree(x);
     for (auto x : p->d_c) cudaFree(x);
-    cudaFree(p->d_pos);
-    cudaFree(p->d_frac);
-    cudaFree(p->d_spec);
-    cudaFree(p->d_sel);
     cudaFree(p->d_bre);
     cudaFree(p->d_bim);
     cudaFree(p->d_cinv);
-    cudaFree(p->d_scale);
     delete p;
 }
 
@@ -766,6 +784,8 @@ int ofdft_pseudo_set_ions(ofdft_pseudo* p, int nat, const double* pos, const int
         for (int a = 0; a < nat; ++a)
             OFDFT_REQUIRE(species[a] >= 0 && species[a] < p->ns, "atom %d has species %d outside 0..%d", a,
                           species[a], p->ns - 1);
+        if (p->running) OFDFT_CK(cudaEventSynchronize(p->busy));  // they read the ions that move
+        p->running = false;
         p->nat = nat;
         p->pos.assign(pos, pos + 3 * (size_t)nat);
         p->spec.assign(species, species + nat);
@@ -778,24 +798,22 @@ int ofdft_pseudo_set_ions(ofdft_pseudo* p, int nat, const double* pos, const int
                 if (species[a] == s) sel.push_back(a);
         }
         p->sel_off[p->ns] = (int)sel.size();
-        std::vector<double> scale(nat, -1.0);
-        cudaFree(p->d_pos);
-        cudaFree(p->d_frac);
-        cudaFree(p->d_spec);
-        cudaFree(p->d_sel);
-        cudaFree(p->d_scale);
-        p->d_pos = p->d_frac = p->d_scale = nullptr;
-        p->d_spec = p->d_sel = nullptr;
-        OFDFT_CK(cudaMalloc(&p->d_pos, 3 * (size_t)nat * sizeof(double)));
-        OFDFT_CK(cudaMalloc(&p->d_frac, 3 * (size_t)nat * sizeof(double)));
-        OFDFT_CK(cudaMalloc(&p->d_spec, (size_t)nat * sizeof(int)));
-        OFDFT_CK(cudaMalloc(&p->d_sel, (size_t)nat * sizeof(int)));
-        OFDFT_CK(cudaMalloc(&p->d_scale, (size_t)nat * sizeof(double)));
-        upload_now(p->d_pos, pos, 3 * (size_t)nat * sizeof(double));
-        upload_now(p->d_frac, p->frac.data(), 3 * (size_t)nat * sizeof(double));
-        upload_now(p->d_spec, species, (size_t)nat * sizeof(int));
-        upload_now(p->d_sel, sel.data(), (size_t)nat * sizeof(int));
-        upload_now(p->d_scale, scale.data(), (size_t)nat * sizeof(double));
+        // positions, fractional coordinates, gather scale, species, atoms by species: one buffer,
+        // one upload, allocated again only for more atoms
+        const size_t n = (size_t)nat, bytes = 7 * n * sizeof(double) + 2 * n * sizeof(int);
+        std::vector<double> up((bytes + sizeof(double) - 1) / sizeof(double));
+        std::copy(pos, pos + 3 * n, up.begin());
+        std::copy(p->frac.begin(), p->frac.end(), up.begin() + 3 * n);
+        std::fill(up.begin() + 6 * n, up.begin() + 7 * n, -1.0);
+        int* ints = reinterpret_cast<int*>(up.data() + 7 * n);
+        std::copy(species, species + n, ints);
+        std::copy(sel.begin(), sel.end(), ints + n);
+        p->d_pos = (double*)p->sc.get("ions", bytes);
+        p->d_frac = p->d_pos + 3 * n;
+        p->d_scale = p->d_pos + 6 * n;
+        p->d_spec = reinterpret_cast<int*>(p->d_pos + 7 * n);
+        p->d_sel = p->d_spec + n;
+        upload_now(p->d_pos, up.data(), bytes);
     });
 }
 

@@ -48,8 +48,10 @@ class ewald:
 
     @property
     def energy(self):
+        # with the forces: they share the mesh, its transform and the pair sum with the
+        # energy, and cost one inverse transform more
         if self._parts is None:
-            self._run(False)
+            self._run(True)
         return float(self._parts[0])
 
     def Energy_real(self):

@@ -6,6 +6,7 @@ binds any per-grid data the native evaluator needs (``prepare``).  Calling a
 functional alone runs an evaluator configured with that functional only;
 ``TotalFunctional`` fuses all of its functionals into one evaluator.
 """
+import copy
 from abc import ABC, abstractmethod
 
 import numpy as np
@@ -56,7 +57,9 @@ class NativeEval:
             pass
 
     def set_vloc(self, vloc, token):
-        if self.vloc_token is token:
+        """Copy a local potential in, unless the evaluator holds it already: ``token``
+        names its geometry, precision and in-place version (None: always copied)."""
+        if token is not None and self.vloc_token == token:
             return
         t = vloc.as_subclass(torch.Tensor).contiguous()
         _lib.check(self.lib.ofdft_eval_set_vloc(self.h, _lib.C.c_void_p(t.data_ptr()), stream_ptr()))
@@ -174,6 +177,37 @@ def config_key(cfg):
     return tuple(key(getattr(cfg, f)) for f, _ in cfg._fields_)
 
 
+class ConfigCache:
+    """The native configuration of a set of functionals, filled again only when a
+    functional's ``config_state`` differs from the one it was filled from (building the
+    ctypes structure and its key takes about 40 us)."""
+
+    def __init__(self):
+        self._states = None
+        self.cfg = self.key = None
+        self.fusable = False
+
+    def update(self, functionals):
+        states = [(f, f.config_state()) for f in functionals]
+        try:
+            same = self._states is not None and len(states) == len(self._states) and all(
+                f is g and a is not None and bool(a == b) for (f, a), (g, b) in zip(states, self._states))
+        except (ValueError, TypeError, RuntimeError):  # option values that do not compare to a truth value
+            same = False
+        if not same:
+            cfg, seen, fusable = empty_config(), 0, True
+            for f in functionals:
+                one = empty_config()
+                f.configure(one)
+                bits = one.kedf_terms | (one.xc_lda << 8) | (one.hartree << 9) | (one.pseudo << 10) | (one.external << 11)
+                fusable = fusable and not bits & seen  # a term configured twice: evaluate separately and sum
+                seen |= bits
+                f.configure(cfg)
+            self.cfg, self.key, self.fusable = cfg, config_key(cfg), fusable
+            self._states = [(f, copy.deepcopy(a)) for f, a in states]
+        return self
+
+
 class NativeFunctional(AbstractFunctional):
     """A functional evaluated by the native library."""
 
@@ -182,6 +216,9 @@ class NativeFunctional(AbstractFunctional):
 
     def configure(self, cfg):  # fill this functional's part of the evaluator config
         raise NotImplementedError
+
+    def config_state(self):  # what configure() depends on, comparable with ==; None: not known
+        return None
 
     def prepare(self, ev, grid, dtype):  # bind per-grid data (v_loc, k_F state) before a compute
         pass
@@ -194,12 +231,11 @@ class NativeFunctional(AbstractFunctional):
 
     def _evaluator(self, grid, dtype):
         cache = self.__dict__.setdefault("_evals", {})
-        cfg = empty_config()
-        self.configure(cfg)
-        key = (id(grid), dtype, config_key(cfg))
+        c = self.__dict__.setdefault("_config_cache", ConfigCache()).update([self])
+        key = (id(grid), dtype, c.key)
         ev = cache.get(key)
         if ev is None:
-            ev = NativeEval(grid, dtype, cfg)
+            ev = NativeEval(grid, dtype, c.cfg)
             cache[key] = ev
         return ev
 

@@ -225,6 +225,9 @@ class KEDF(NativeFunctional):
     def engines(self, name=None):
         return KEDFEngines[(name or self.name).upper()]
 
+    def config_state(self):
+        return self.name, self.options
+
     def configure(self, cfg, engines=None):
         o = self.options
         for e in (engines if engines is not None else self.engines()):

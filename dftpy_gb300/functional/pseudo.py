@@ -208,16 +208,17 @@ class LocalPseudo(NativeFunctional):
             ptr = _lib.C.c_void_p()
             _lib.check(lib.ofdft_pseudo_create(self.grid.native_for(dtype), len(keys), npts, gpp, vpp,
                                                1 if self.PME else 0, int(self.BsplineOrder), _lib.C.byref(ptr)))
-            ions = self.ions
-            pos = np.ascontiguousarray(ions.positions, dtype=np.float64)
-            spec = np.ascontiguousarray([keys.index(s) for s in ions.symbols], dtype=np.int32)
-            rc = lib.ofdft_pseudo_set_ions(ptr, ions.nat, _lib.dptr(pos), spec.ctypes.data_as(_lib._PI))
-            if rc != _lib.OK:
-                lib.ofdft_pseudo_destroy(ptr)
-                _lib.check(rc)
             h = _PseudoHandle(lib, ptr, (gps, vps))
+            self._set_ions(h)
             self._native[dtype] = h
         return h.ptr
+
+    def _set_ions(self, h):
+        ions, keys = self.ions, self.species_keys
+        pos = np.ascontiguousarray(ions.positions, dtype=np.float64)
+        index = {k: i for i, k in enumerate(keys)}
+        spec = np.ascontiguousarray([index[s] for s in ions.symbols], dtype=np.int32)
+        _lib.check(h.lib.ofdft_pseudo_set_ions(h.ptr, ions.nat, _lib.dptr(pos), spec.ctypes.data_as(_lib._PI)))
 
     def vreal_for(self, dtype=torch.float64):
         """v_loc on the real-space grid (local_PP, :237-246), cached per precision."""
@@ -241,10 +242,15 @@ class LocalPseudo(NativeFunctional):
     def configure(self, cfg):
         cfg.pseudo = 1
 
+    def config_state(self):
+        return ()
+
     def prepare(self, ev, grid, dtype):
         if grid is not self.grid and not (grid == self.grid):
             raise ValueError("density grid differs from the pseudopotential grid")
-        ev.set_vloc(self.vreal_for(dtype), token=(self._version, dtype))
+        v = self.vreal_for(dtype)
+        # an inference-mode tensor keeps no in-place version: it is copied every time
+        ev.set_vloc(v, token=None if v.is_inference() else (self._version, dtype, v._version))
 
     def forces(self, rho):
         """LocalPseudo.forces (:260-270): PME or exact structure factor."""
@@ -298,9 +304,16 @@ class LocalPseudo(NativeFunctional):
         self._native, self._vreal, self._version = {}, {}, object()
 
     def set_positions(self, positions):
-        """Move the ions (Bohr); drops cached v_loc and the Ewald object."""
+        """Move the ions (Bohr); drops cached v_loc and the Ewald object.  The native handles
+        stay, with their radial tables on the grid."""
         self._ions.positions = np.array(positions, dtype=np.float64).reshape(self._ions.nat, 3)
-        self._native, self._vreal, self._version = {}, {}, object()
+        self._vreal, self._version = {}, object()
+        try:
+            for h in self._native.values():
+                self._set_ions(h)
+        except Exception:
+            self._native = {}
+            raise
         self.ewald = None
 
     def get_ewald(self, PME=None):

@@ -36,6 +36,9 @@ class XC(NativeFunctional):
     def configure(self, cfg):
         cfg.xc_lda = 1
 
+    def config_state(self):
+        return ()
+
     def compute(self, density, calcType={"E", "V"}, **kwargs):
         out = NativeFunctional.compute(self, density, calcType)
         if "E" in calcType:
@@ -94,6 +97,9 @@ class Hartree(NativeFunctional):
 
     def configure(self, cfg):
         cfg.hartree = 1
+
+    def config_state(self):
+        return ()
 
     @_ClassOrInstance
     def compute(self, density, calcType={"E", "V"}, **kwargs):

@@ -9,8 +9,7 @@ import torch
 
 from .. import _lib
 from ..field import DirectField, as_field
-from .abstract_functional import AbstractFunctional, NativeEval, NativeFunctional, calc_bits, config_key, \
-    empty_config
+from .abstract_functional import AbstractFunctional, ConfigCache, NativeEval, NativeFunctional, calc_bits
 from .functional_output import FunctionalOutput
 
 __all__ = ["TotalFunctional"]
@@ -43,6 +42,7 @@ class TotalFunctional(AbstractFunctional):
             self.name += f.name + " "
             self.type += f.type + " "
         self._evals = {}
+        self._config_cache = ConfigCache()
 
     def UpdateFunctional(self, keysToRemove=[], newFuncDict={}):
         for key in keysToRemove:
@@ -63,28 +63,19 @@ class TotalFunctional(AbstractFunctional):
         return None
 
     # -------------------------------------------------------- fused path
+    def _config(self):
+        return self._config_cache.update(list(self.funcDict.values()))
+
     def _fusable(self):
-        if not all(isinstance(f, NativeFunctional) for f in self.funcDict.values()):
-            return False
-        seen = 0
-        for f in self.funcDict.values():
-            cfg = empty_config()
-            f.configure(cfg)
-            bits = cfg.kedf_terms | (cfg.xc_lda << 8) | (cfg.hartree << 9) | (cfg.pseudo << 10) | (cfg.external << 11)
-            if bits & seen:
-                return False  # a term configured twice: evaluate separately and sum
-            seen |= bits
-        return True
+        return all(isinstance(f, NativeFunctional) for f in self.funcDict.values()) and self._config().fusable
 
     def evaluator(self, grid, dtype):
         """The fused native evaluator of this total functional on (grid, dtype)."""
-        cfg = empty_config()
-        for f in self.funcDict.values():
-            f.configure(cfg)
-        key = (id(grid), dtype, config_key(cfg))
+        c = self._config()
+        key = (id(grid), dtype, c.key)
         ev = self._evals.get(key)
         if ev is None:
-            ev = NativeEval(grid, dtype, cfg)
+            ev = NativeEval(grid, dtype, c.cfg)
             self._evals[key] = ev
         return ev
 

@@ -152,3 +152,39 @@ def test_calculator_matches_reference(tmp_path):
     for k, de, df, ds, dn in diffs:
         assert de <= 1e-10 and df <= 5e-6 and ds <= 2e-7 and dn <= 1e-10, diffs
     assert calc.nsteps == 3
+
+
+def test_moved_ions_and_changed_options_reach_the_evaluation():
+    """What a call must notice although the handle, the configuration and the copied
+    potential are kept: moved ions (also twice without waiting), a changed option, an
+    in-place change of v_loc."""
+    from dftpy_gb300 import synthetic as syn
+    lat, pos = syn.fcc_cell(7.6)
+    nr = (24, 20, 18)
+    g, v = syn.analytic_vloc(3.0, 1.0)
+    rho_np = syn.smooth_density(lat, nr, 12.0, seed=2, amp=0.4)
+
+    def build(p, x=1.0):
+        grid = D.DirectGrid(lat, nr)
+        pp = D.LocalPseudo(grid=grid, ions=D.Ions(symbols=["Al"] * 4, positions=p, cell=lat),
+                           PP_list={"Al": D.functional.RECPOT(r=g, v=v, zval=3)}, PME=True)
+        ke = D.Functional(type="KEDF", name="TFVW", x=x)
+        return D.DirectField(grid, data=rho_np), pp, ke, D.TotalFunctional(KE=ke, HARTREE=D.Functional(type="HARTREE"),
+                                                                           PSEUDO=pp)
+
+    rho, pp, ke, total = build(pos)
+    total(rho)
+    rng = np.random.default_rng(3)
+    moved = [pos + rng.normal(0, 0.2, pos.shape) for _ in range(3)]
+    for p in moved:
+        pp.set_positions(p)
+        pp.vreal  # enqueued; the next geometry must wait for it
+    ke.options["x"] = 0.7
+    out, F = total(rho), total.get_forces(rho)
+    rho2, _, _, fresh = build(moved[-1], x=0.7)
+    ref = fresh(rho2)
+    assert out.energy == ref.energy and np.array_equal(out.potential.numpy(), ref.potential.numpy())
+    assert np.allclose(F, fresh.get_forces(rho2), rtol=0, atol=1e-13)
+    pp.vreal.add_(0.5)
+    shifted = total(rho)
+    assert abs(shifted.energy - out.energy - 0.5 * 12.0) < 1e-9
