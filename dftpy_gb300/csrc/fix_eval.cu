@@ -176,68 +176,120 @@ __device__ __noinline__ double wt_build(const MulArgs& a, double gg) {
     return lindhard_dev(sqrt(gg) / a.state[2], a.wt_x, 1.0) * a.state[3];
 }
 
+// The last pass of a forward transform, the factor, and the first pass of the inverse with
+// the radices in reverse order: that one takes exactly the elements that this one leaves in
+// a thread's registers, so they are not exchanged in between.
+template <int R, class Factor>
+__device__ __forceinline__ void turn(const I2* src, I2* dst, const Plan& p, int lb, LineSm& sm, Factor factor) {
+    const int L = 1 << lb, m = p.n / R, l = threadIdx.x & (L - 1), j = threadIdx.x >> lb;
+    const bool on = j < m;
+    I2 u[R];
+    double2 v[R];
+    if (on) {
+        gather<R>(u, src, p.n, lb, m, j, l, pass_shift(sm.ds[l], p.np - 1, p.np, p.r[1]), p.tw);
+        Dft<R>::run(u);
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const double2 z = from_fix(u[q], sm, l);
+            const double f = factor(j + q * m);
+            v[q] = make_double2(z.y * f, z.x * f);  // parts exchanged: the inverse
+        }
+    }
+    __syncthreads();  // the buffer and the scales are read
+    reset(sm);
+    __syncthreads();
+    agree<R>(v, u, on, j, l, sm, p.np);
+    if (on) {
+        Dft<R>::run(u);
+#pragma unroll
+        for (int q = 0; q < R; ++q) dst[(j * R + q) * (L + 1) + l] = u[q];
+    }
+}
+
 // Axis 0 forward, the field's factor, axis 0 inverse.  |G|^2 = A f0^2 + B f0 + C along a
 // line (f0 the axis-0 frequency), so a point pays two operations for it.
-__global__ void __launch_bounds__(kThreads, 3) k_cols_mul(MulArgs a) {
+__global__ void __launch_bounds__(kThreads, kBlocks) k_cols_mul(MulArgs a) {
     extern __shared__ __align__(16) unsigned char fix_smem[];
     __shared__ LineSm sm;
     const Plan& p = a.c.g.p0;
-    const int n = p.n, lb = a.c.lb, L = 1 << lb, LP = L + 1;
+    const int n = p.n, lb = a.c.lb, L = 1 << lb;
     I2* b0 = reinterpret_cast<I2*>(fix_smem);
-    I2* b1 = b0 + n * LP;
-    double2* fq = reinterpret_cast<double2*>(b1 + n * LP);  // f0 and A f0^2
-    const int k1 = blockIdx.x / a.c.ktiles, k2 = (blockIdx.x % a.c.ktiles) * L;
-    const int nl = min(L, a.c.g.n2h - k2), l = threadIdx.x & (L - 1);
-    const long long stride = (long long)a.c.g.n1 * a.c.g.n2h;
-    const long long off = (long long)k1 * a.c.g.n2h + k2;
-    double2* base = a.c.sp[blockIdx.y] + off;
+    I2* b1 = b0 + (p.np == 3 ? n * (L + 1) : 0);
+    double2* fq = reinterpret_cast<double2*>(b1 + n * (L + 1));  // f0 and A f0^2
+    const int line = (blockIdx.x << lb) + (threadIdx.x & (L - 1));
+    const bool in = line < col_lines<0>(a.c.g);
+    const int k1 = line / a.c.g.n2h, k2 = line - k1 * a.c.g.n2h;
+    const long long stride = col_stride<0>(a.c.g);
+    double2* base = a.c.sp[blockIdx.y] + (in ? line : 0);
     const int kind = a.kind[blockIdx.y];
     const Geo& g = a.geo;
-    const double f1 = (double)freq_index(k1, g.n1) * g.fv[1], f2 = (double)(k2 + l) * g.fv[2];
+    const double f1 = (double)freq_index(k1, g.n1) * g.fv[1], f2 = (double)k2 * g.fv[2];
     const double ax = g.b[0] * g.fv[0], ay = g.b[1] * g.fv[0], az = g.b[2] * g.fv[0];
     const double cx = f1 * g.b[3] + f2 * g.b[6], cy = f1 * g.b[4] + f2 * g.b[7], cz = f1 * g.b[5] + f2 * g.b[8];
     const double A = ax * ax + ay * ay + az * az, B = 2.0 * (ax * cx + ay * cy + az * cz), C = cx * cx + cy * cy + cz * cz;
-    for (int i = threadIdx.x; i < n; i += kThreads) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const double f = (double)freq_index(i, n);
         fq[i] = make_double2(f, A * f * f);
     }
-    const I2* z = tile_fft(b0, b1, p, lb, sm, [&](int i, int q) {
-        return q < nl ? base[i * stride + q] : make_double2(0.0, 0.0);
-    });
-    const Scale c = sm.c[l];
-    const int ds = sm.ds[l];
-    __syncthreads();  // every thread has its line's scale before the next transform resets them
     const bool build = kind == F_WT && a.state[1] != 0.0;
     const double hart = 4.0 * M_PI * a.invN, half = 0.5 * a.invN;
-    const I2* y = tile_fft(b0, b1, p, lb, sm, [&](int i, int q) {
-        if (q >= nl) return make_double2(0.0, 0.0);
-        double f;
+    auto factor = [&](int i) -> double {
+        if (!in) return 0.0;
         if (kind == F_WT) {
-            const long long at = off + i * stride + q;
-            double K;
-            if (build) {
-                const double2 t = fq[i];
-                K = wt_build(a, fma(t.x, B, t.y) + C);
-                a.K[at] = K;
-            } else {
-                K = a.K[at];
-            }
-            f = K * a.invN;
-        } else {
+            const long long at = line + i * stride;
+            if (!build) return a.K[at] * a.invN;
             const double2 t = fq[i];
-            const double gg = fma(t.x, B, t.y) + C;
-            if (kind == F_VW) f = gg * half;
-            else f = i == 0 && off + q == 0 ? 0.0 : (ordinary(gg) ? recip(gg) : 1.0 / gg) * hart;
+            const double K = wt_build(a, fma(t.x, B, t.y) + C);
+            a.K[at] = K;
+            return K * a.invN;
         }
-        const I2 v = z[i * LP + q];
-        return make_double2(to_dbl(v.y, c, ds) * f, to_dbl(v.x, c, ds) * f);
-    });
-    for (int e = threadIdx.x; e < n * L; e += kThreads) {
-        const int q = e & (L - 1), i = e >> lb;
-        if (q >= nl) continue;
-        const Scale d = sm.c[q];
-        const I2 v = y[i * LP + q];
-        base[i * stride + q] = make_double2(to_dbl(v.y, d, sm.ds[q]), to_dbl(v.x, d, sm.ds[q]));
+        const double2 t = fq[i];
+        const double gg = fma(t.x, B, t.y) + C;
+        if (kind == F_VW) return gg * half;
+        return i == 0 && line == 0 ? 0.0 : (ordinary(gg) ? recip(gg) : 1.0 / gg) * hart;
+    };
+    auto get = [&](int i, int) { return in ? base[i * stride] : make_double2(0.0, 0.0); };
+    auto put = [&](int i, int l, I2 z) {
+        if (in) base[i * stride] = swapped(from_fix(z, sm, l));
+    };
+    reset(sm);
+    __syncthreads();
+    switch (p.r[0]) {
+#define FIX_CASE(R) \
+    case R: pass0<R>(b0, n, lb, sm, p.np, get); break;
+        FIX_RADICES(FIX_CASE)
+#undef FIX_CASE
+    }
+    __syncthreads();
+    if (p.np == 1) {  // one pass: the transform's outputs are in the buffer
+        const int l = threadIdx.x & (L - 1), k = sm.ds[l] - sm.k[l];
+        const bool nan = sm.emax[l] == kNonFinite;
+        __syncthreads();
+        tile_fft_out(
+            b0, b1, p, lb, sm,
+            [&](int i, int q) {
+                const I2 z = b0[i * (L + 1) + q];
+                const double f = factor(i);
+                return make_double2(to_dbl(z.y, k, nan) * f, to_dbl(z.x, k, nan) * f);
+            },
+            put);
+        return;
+    }
+    const I2* z = middle(b0, b1, p, lb, sm, p.np - 1, false);
+    I2* y = z == b0 ? b0 : b1;
+    switch (p.r[p.np - 1]) {
+#define FIX_CASE(R) \
+    case R: turn<R>(z, y, p, lb, sm, factor); break;
+        FIX_RADICES(FIX_CASE)
+#undef FIX_CASE
+    }
+    __syncthreads();
+    z = middle(y, y == b0 ? b1 : b0, p, lb, sm, p.np - 1, true);
+    switch (p.r[0]) {
+#define FIX_CASE(R) \
+    case R: pass_out<R>(z, n, lb, p.tw, sm, p.np - 1, p.np, p.r[p.np - 2], put); break;
+        FIX_RADICES(FIX_CASE)
+#undef FIX_CASE
     }
 }
 
@@ -303,7 +355,7 @@ namespace fix {
 
 struct GridPlans {
     Grid3 g;
-    I2* tw = nullptr;
+    Tw* tw = nullptr;
     bool ok = false;
 };
 
@@ -325,20 +377,20 @@ const Grid3* grid_plans(ofdft_grid* g) {
         }
         if (ok) {
             // twiddles at scale 2^61 from long double trigonometry
-            std::vector<I2> tw(total);
+            std::vector<Tw> tw(total);
             size_t off = 0;
             const long double pi = 3.14159265358979323846264338327950288L;
             for (int d = 0; d < 3; ++d) {
                 const int n = g->nr[d];
                 for (int k = 0; k < n; ++k) {
                     const long double t = -2.0L * pi * (long double)k / (long double)n;
-                    tw[off + k] = I2{(long long)std::llroundl(std::cos(t) * (long double)kOne),
-                                     (long long)std::llroundl(std::sin(t) * (long double)kOne)};
+                    tw[off + k] = tw_of((long long)std::llroundl(std::cos(t) * (long double)kOne),
+                                        (long long)std::llroundl(std::sin(t) * (long double)kOne));
                 }
                 off += n;
             }
-            OFDFT_CK(cudaMalloc(&h->tw, total * sizeof(I2)));
-            upload_now(h->tw, tw.data(), total * sizeof(I2));
+            OFDFT_CK(cudaMalloc(&h->tw, total * sizeof(Tw)));
+            upload_now(h->tw, tw.data(), total * sizeof(Tw));
             off = 0;
             for (int d = 0; d < 3; ++d) {
                 p[d]->tw = h->tw + off;
@@ -432,16 +484,18 @@ int local_enqueue(ofdft_grid* g, Scratch& sc, const LocalArgs& a, cudaStream_t s
     if (nf > 0) {
         rows_r2c(p, sms, in, sp, nf, st);
         cols<1>(p, sms, sp, nf, false, st);
-        m.c = col_args(p, 0, sms);
+        const Shape s = shape_of(p.p0, col_lines<0>(p), sms, true);
+        m.c.g = p;
+        m.c.lb = s.lb;
         for (int f = 0; f < nf; ++f) m.c.sp[f] = sp[f];
         m.geo = g->geo;
         m.K = a.wtK;
         m.state = a.wtstate;
         m.wt_x = a.wt_x;
         m.invN = 1.0 / (double)N;
-        const size_t smem = tile_smem(p.p0, 1 << m.c.lb) + (size_t)p.n0 * sizeof(double2);
+        const size_t smem = tile_smem(p.p0, s.lb, 1) + (size_t)p.n0 * sizeof(double2);
         smem_optin(k_cols_mul, smem);
-        k_cols_mul<<<dim3(col_blocks(m.c, 0), nf), kThreads, smem, st>>>(m);
+        k_cols_mul<<<dim3(col_blocks(col_lines<0>(p), s.lb), nf), s.threads, smem, st>>>(m);
         OFDFT_LAUNCH_CHECK();
         cols<1>(p, sms, sp, nf, true, st);
         rows_c2r(p, sms, sp, out, nf, st);

@@ -8,8 +8,8 @@
 //
 // Precision.  With R the first pass's radix, the scale maps the largest 1-norm
 // sum |re| + |im| of the subsets that the first pass transforms (every (n/R)-th
-// element; bounds taken from the leading 21 bits of every element) to at most 2^61,
-// and after the first pass the line's whole 1-norm to at most 2^61.  Every
+// element; a bound taken from every element's exponent) to at most 2^61,
+// and the later passes' sums, up to the line's whole 1-norm, to at most 2^61 as well.  Every
 // intermediate of an FFT is a sum of the inputs with weights of modulus one, so none
 // exceeds these bounds: nothing overflows, and no bits are given up that the line's
 // own values do not need.  For flat lines of up to 1024 elements the unit is 2^-56 of
@@ -51,10 +51,15 @@ FIX_HD I2 mulr(I2 a, long long c) { return I2{mulc(a.x, c), mulc(a.y, c)}; }
 FIX_HD I2 half(I2 a) { return I2{a.x >> 1, a.y >> 1}; }
 FIX_HD I2 quarter(I2 a) { return I2{a.x >> 2, a.y >> 2}; }
 
-// x w with w at scale 2^61
-FIX_HD I2 cmul(I2 x, I2 w) {
+// a twiddle at scale 2^61 in 31-bit limbs: real part high, low, imaginary part high, low
+struct __align__(16) Tw {
+    int ch, cl, dh, dl;
+};
+FIX_HD Tw tw_of(long long re, long long im) { return Tw{hi31(re), lo31(re), hi31(im), lo31(im)}; }
+
+FIX_HD I2 cmul(I2 x, Tw w) {
     const int ah = hi31(x.x), al = lo31(x.x), bh = hi31(x.y), bl = lo31(x.y);
-    const int ch = hi31(w.x), cl = lo31(w.x), dh = hi31(w.y), dl = lo31(w.y);
+    const int ch = w.ch, cl = w.cl, dh = w.dh, dl = w.dl;
     const long long ac = (long long)ah * cl + (long long)al * ch, bd = (long long)bh * dl + (long long)bl * dh;
     const long long x2 = (long long)ah * dl + (long long)al * dh + (long long)bh * cl + (long long)bl * ch;
     const long long re = (long long)ah * ch - (long long)bh * dh;
@@ -176,10 +181,10 @@ struct Dft<9> {
             for (int r = 0; r < 3; ++r) a[j][r] = u[j + 3 * r];
             Dft<3>::run(a[j]);
         }
-        a[1][1] = cmul(a[1][1], I2{kC91, -kS91});
-        a[1][2] = cmul(a[1][2], I2{kC92, -kS92});
-        a[2][1] = cmul(a[2][1], I2{kC92, -kS92});
-        a[2][2] = cmul(a[2][2], I2{kC94, -kS94});
+        a[1][1] = cmul(a[1][1], tw_of(kC91, -kS91));
+        a[1][2] = cmul(a[1][2], tw_of(kC92, -kS92));
+        a[2][1] = cmul(a[2][1], tw_of(kC92, -kS92));
+        a[2][2] = cmul(a[2][2], tw_of(kC94, -kS94));
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             I2 b[3] = {a[0][k], a[1][k], a[2][k]};
@@ -199,7 +204,7 @@ struct Dft<16> {
             for (int r = 0; r < 4; ++r) a[j][r] = u[j + 4 * r];
             Dft<4>::run(a[j]);
         }
-        const I2 w1{kC161, -kS161}, w3{kS161, -kC161}, w9{-kC161, kS161};
+        const Tw w1 = tw_of(kC161, -kS161), w3 = tw_of(kS161, -kC161), w9 = tw_of(-kC161, kS161);
         auto w2 = [](I2 v) { return I2{mulc(v.x + v.y, kH), mulc(v.y - v.x, kH)}; };
         auto w6 = [](I2 v) { return I2{mulc(v.y - v.x, kH), mulc(-(v.x + v.y), kH)}; };
         a[1][1] = cmul(a[1][1], w1);
@@ -288,11 +293,10 @@ FIX_HD double of_bits(unsigned long long b) {
 #endif
 }
 FIX_HD int expo(double v) { return (int)((unsigned)(bits_of(v) >> 52) & 0x7ffu); }  // biased exponent
-// the leading 21 bits of |v| at the scale of biased exponent emax (rounded down)
-FIX_HD unsigned lead(double v, int emax) {
-    const unsigned hi = (unsigned)(bits_of(v) >> 32) & 0x7fffffffu;
-    const int d = emax - (int)(hi >> 20);
-    return (hi >> 20) == 0u || d > 20 ? 0u : ((hi & 0xfffffu) | 0x100000u) >> d;
+// a bound of |v| in units of 2^(emax - 20), from its biased exponent e
+FIX_HD unsigned bound(int e, int emax) {
+    const int d = emax - e;
+    return 0x200000u >> (d < 31 ? d : 31);
 }
 // The scale of a line: emax, the largest biased exponent, and sh, the bit length of a
 // bound of the 1-norm in units of 2^(emax - 20).  x becomes x 2^(81 - sh) 2^-emax.
@@ -300,6 +304,13 @@ constexpr int kNonFinite = 0x7ff;
 struct Scale {
     int emax, sh;
 };
+// The shift in front of pass q >= 1 when the whole line needs ds: what the pass can grow
+// by (ceil log2 of its radix), or what is left
+FIX_HD int pass_shift(int ds, int q, int np, int r1) {
+    const int grow = r1 > 8 ? 4 : (r1 > 4 ? 3 : (r1 > 2 ? 2 : 1));
+    const int first = np == 2 || ds < grow ? ds : grow;
+    return q == 1 ? first : ds - first;
+}
 // v 2^-d, rounded
 FIX_HD long long shr(long long v, int d) { return (v + ((1LL << d) >> 1)) >> d; }
 // 64-bit roundings between integers and float64
@@ -310,38 +321,40 @@ FIX_HD long long rint64(double v) {
     return __builtin_llrint(v);
 #endif
 }
-// v 2^k by the exponent field: 0 on underflow, infinite on overflow (v normal or zero)
-FIX_HD double scaled(double v, int k) {
+// v at the line's scale: k = fix_shift is added to the exponent field (|v| 2^k' is below
+// 2^62); a zero, subnormal or wrapping element becomes a tiny value, which rounds to 0
+FIX_HD int fix_shift(Scale s) { return 81 - s.sh - s.emax + 1023; }
+FIX_HD long long to_fix(double v, int k) {
     const unsigned long long b = bits_of(v);
-    const int e = (int)((unsigned)(b >> 52) & 0x7ffu);
-    double r = of_bits(b + ((unsigned long long)(long long)k << 52));
-    if (e == 0 || e + k <= 0) r = 0.0;
-    if (e != 0 && e + k >= 0x7ff) r = of_bits((b & 0x8000000000000000ULL) | 0x7ff0000000000000ULL);
-    return r;
+    const int hi = (int)(b >> 32), e = (hi >> 20) & 0x7ff;
+    const unsigned t = e == 0 || e + k <= 0 ? 0u : (unsigned)(hi + (k << 20));
+    return rint64(of_bits(((unsigned long long)t << 32) | (b & 0xffffffffULL)));
 }
-FIX_HD long long to_fix(double v, Scale s) {
-    // |v| 2^(81 - sh - (emax - 1023)) is below 2^62
-    const unsigned long long b = bits_of(v);
-    const int e = (int)((unsigned)(b >> 52) & 0x7ffu), k = 81 - s.sh - s.emax + 1023;
-    const double t = of_bits(b + ((unsigned long long)(long long)k << 52));
-    return e == 0 || e + k <= 0 ? 0 : rint64(t);
-}
-// v 2^(emax + sh - 81 - 1023 + adj), rounded to nearest
-FIX_HD double to_dbl(long long v, Scale s, int adj) {
-    const double r = scaled((double)v, s.emax + s.sh - 81 - 1023 + adj);
-    return s.emax == kNonFinite ? of_bits(0x7ff8000000000000ULL) : r;
+// v 2^(k - 1023 + ...) for an output of the line: k = shift after the first pass - fix_shift;
+// 0 on underflow, infinite on overflow, NaN in a line that was not finite
+FIX_HD double to_dbl(long long v, int k, bool nan) {
+    const unsigned long long b = bits_of((double)v);
+    const int hi = (int)(b >> 32), e = ((hi >> 20) & 0x7ff) + k;
+    unsigned t = (unsigned)(hi + (k << 20)), lo = (unsigned)b;
+    if (v == 0 || e <= 0) t = lo = 0u;
+    if (v != 0 && e >= 0x7ff) {
+        t = (hi & 0x80000000u) | 0x7ff00000u;
+        lo = 0u;
+    }
+    if (nan) t = 0x7ff80000u;
+    return of_bits(((unsigned long long)t << 32) | lo);
 }
 
 // ---- plans: radices of a length, largest first where twiddles are fewest
-constexpr int kMaxPass = 4;
+constexpr int kMaxPass = 3;
 constexpr int kMaxLen = 1024;
 // Axes the three-dimensional transforms take: a tile of at least two lines of two
 // exchange buffers fits in shared memory.
 constexpr int kMaxAxis = 512;
 struct Plan {
     int n = 0, np = 0;
-    int r[kMaxPass] = {0, 0, 0, 0};
-    const I2* tw = nullptr;  // exp(-2 pi i k/n), k < n, at scale 2^61
+    int r[kMaxPass] = {0, 0, 0};
+    const Tw* tw = nullptr;  // exp(-2 pi i k/n), k < n
 };
 
 // false when n has a prime factor above 7, or is too long
@@ -362,6 +375,7 @@ inline bool plan_radices(int n, Plan& p) {
         for (int b : radix)
             if (a >= b && a * b == n && (!best || a < best)) best = a;
     if (best) {
+        // the larger radix first: the units of the second pass then grow by the smaller one
         p.np = 2;
         p.r[0] = best;
         p.r[1] = n / best;

@@ -24,11 +24,12 @@ static void dft(int R, I2* u) {
 extern "C" int line_fft(int n, const double* in, double* out) {  // 0 when n has no plan
     Plan p;
     if (!plan_radices(n, p)) return 0;
-    std::vector<I2> tw(n), a(n), b(n);
+    std::vector<I2> a(n), b(n);
+    std::vector<Tw> tw(n);
     for (int k = 0; k < n; ++k) {
         const long double t = -2.0L * 3.14159265358979323846264338327950288L * k / n;
-        tw[k] = I2{(long long)std::llroundl(std::cos(t) * (long double)kOne),
-                   (long long)std::llroundl(std::sin(t) * (long double)kOne)};
+        tw[k] = tw_of((long long)std::llroundl(std::cos(t) * (long double)kOne),
+                      (long long)std::llroundl(std::sin(t) * (long double)kOne));
     }
     int em = 0;
     for (int i = 0; i < 2 * n; ++i) em = std::max(em, expo(in[i]));
@@ -37,14 +38,15 @@ extern "C" int line_fft(int n, const double* in, double* out) {  // 0 when n has
         unsigned s = 2 * p.r[0];
         for (int q = 0; q < p.r[0]; ++q) {
             const double* v = in + 2 * (j + q * (n / p.r[0]));
-            s += lead(v[0], em) + lead(v[1], em);
+            s += bound(expo(v[0]), em) + bound(expo(v[1]), em);
         }
         most = std::max(most, s);
         sum += s;
     }
     const Scale c{em, 32 - __builtin_clz(most)};
     const int ds = p.np > 1 ? 32 - __builtin_clz(sum) - c.sh : 0;
-    for (int i = 0; i < n; ++i) a[i] = I2{to_fix(in[2 * i], c), to_fix(in[2 * i + 1], c)};
+    const int k = fix_shift(c);
+    for (int i = 0; i < n; ++i) a[i] = I2{to_fix(in[2 * i], k), to_fix(in[2 * i + 1], k)};
     int Ns = 1;
     for (int q = 0; q < p.np; ++q) {
         const int R = p.r[q], m = n / R, step = n / (Ns * R);
@@ -54,7 +56,10 @@ extern "C" int line_fft(int n, const double* in, double* out) {  // 0 when n has
             for (int r = 0; r < R; ++r) {
                 u[r] = a[j + r * m];
                 if (r && q) u[r] = cmul(u[r], tw[k * r * step]);
-                if (q == 1) u[r] = I2{shr(u[r].x, ds), shr(u[r].y, ds)};
+                if (q) {
+                    const int d = pass_shift(ds, q, p.np, p.r[1]);
+                    u[r] = I2{shr(u[r].x, d), shr(u[r].y, d)};
+                }
             }
             dft(R, u);
             for (int r = 0; r < R; ++r) b[(j / Ns) * Ns * R + k + r * Ns] = u[r];
@@ -63,8 +68,8 @@ extern "C" int line_fft(int n, const double* in, double* out) {  // 0 when n has
         Ns *= R;
     }
     for (int i = 0; i < n; ++i) {
-        out[2 * i] = to_dbl(a[i].x, c, ds);
-        out[2 * i + 1] = to_dbl(a[i].y, c, ds);
+        out[2 * i] = to_dbl(a[i].x, ds - k, em == kNonFinite);
+        out[2 * i + 1] = to_dbl(a[i].y, ds - k, em == kNonFinite);
     }
     return 1;
 }
