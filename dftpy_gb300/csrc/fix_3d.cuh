@@ -63,33 +63,29 @@ __device__ __forceinline__ double2 from_fix(I2 v, const LineSm& sm, int l, int a
 template <int R>
 __device__ __forceinline__ void agree(const double2 (&v)[R], I2 (&u)[R], bool on, int j, int l, LineSm& sm, int np) {
     int em = 0;
-    if (on) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) em = max(em, max(expo(v[q].x), expo(v[q].y)));
-        atomicMax(&sm.emax[l], em);
-    }
+    for (int q = 0; q < R; ++q) em = max(em, max(expo(v[q].x), expo(v[q].y)));
+    if (on) atomicMax(&sm.emax[l], em);
     __syncthreads();
-    if (on) {
-        em = sm.emax[l];
-        unsigned s = 0;
+    em = sm.emax[l];
+    unsigned s = 0;
 #pragma unroll
-        for (int q = 0; q < R; ++q) s += bound(expo(v[q].x), em) + bound(expo(v[q].y), em);
+    for (int q = 0; q < R; ++q) s += bound(expo(v[q].x), em) + bound(expo(v[q].y), em);
+    if (on) {
         atomicMax(&sm.most[l], s);
         atomicAdd(&sm.sum[l], s);
     }
     __syncthreads();
-    if (on) {
-        Scale c;
-        c.emax = em;
-        c.sh = 32 - __clz((int)(sm.most[l] | 1u));
-        const int k = fix_shift(c);
-        if (j == 0) {
-            sm.k[l] = k;
-            sm.ds[l] = np > 1 ? (32 - __clz((int)(sm.sum[l] | 1u))) - c.sh : 0;
-        }
-#pragma unroll
-        for (int q = 0; q < R; ++q) u[q] = I2{to_fix(v[q].x, k), to_fix(v[q].y, k)};
+    Scale c;
+    c.emax = em;
+    c.sh = 32 - __clz((int)(sm.most[l] | 1u));
+    const int k = fix_shift(c);
+    if (j == 0) {
+        sm.k[l] = k;
+        sm.ds[l] = np > 1 ? (32 - __clz((int)(sm.sum[l] | 1u))) - c.sh : 0;
     }
+#pragma unroll
+    for (int q = 0; q < R; ++q) u[q] = I2{to_fix(v[q].x, k), to_fix(v[q].y, k)};
 }
 
 __device__ __forceinline__ void reset(LineSm& sm) {
@@ -105,15 +101,16 @@ template <int R, class Get>
 __device__ __forceinline__ void pass0(I2* buf, int n, int lb, LineSm& sm, int np, Get get) {
     const int m = n / R, L = 1 << lb, l = threadIdx.x & (L - 1), j = threadIdx.x >> lb;
     const bool on = j < m;
+    // a thread without a butterfly repeats butterfly 0 and stores nothing: with the elements
+    // defined on some paths only, they are live around a caller's loop over tiles, and spilled
+    const int i = on ? j : 0;
     double2 v[R];
     I2 u[R];
-    if (on) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = get(j + q * m, l);
-    }
+    for (int q = 0; q < R; ++q) v[q] = get(i + q * m, l);
     agree<R>(v, u, on, j, l, sm, np);
+    Dft<R>::run(u);
     if (on) {
-        Dft<R>::run(u);
 #pragma unroll
         for (int q = 0; q < R; ++q) buf[(j * R + q) * (L + 1) + l] = u[q];
     }

@@ -86,18 +86,22 @@ struct PreK {
     double* sq;
     double* rb;
     double* ra;
+    double* kf;
     long long N;
     int tf, xc;
     int b56, a53;  // beta = 5/6; alpha + beta = 5/3 to rounding
-    double tf_x, alpha, beta, cE, cV;
+    double tf_x, alpha, beta, cE, cV, threepi2;
     LdaRoots lda;
 };
 
 // Pointwise pre-pass: bound by the float64 pipe (about 70 operations per point with
 // TF, LDA, PP and vW).  rho^(5/6) = rho^(1/2) rho^(1/3) and, when the exponents add up
 // to 5/3, rho^alpha = rho^(5/3) / rho^beta need no pow().
+// LWT: also k_F and its range (three more slots, after all blocks' sums), and LWT's clamp.
+template <bool LWT>
 __global__ void __launch_bounds__(RED_THREADS) k_pre(PreK a, double* partials) {
     double s[4] = {0.0, 0.0, 0.0, 0.0};
+    double mm[3] = {INFINITY, -INFINITY, -INFINITY};
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
         const double r = a.rho[i];
@@ -123,14 +127,28 @@ __global__ void __launch_bounds__(RED_THREADS) k_pre(PreK a, double* partials) {
         if (a.sq) a.sq[i] = sq;
         if (a.rb) {
             const bool ord = ordinary(r);
-            const double rc = r < kZERO ? kZERO : r;  // wt.py:15-18
+            // wt.py:15-18; lwt.py:206-221
+            const double rc = LWT ? (r > 0.0 ? r : 1e-30) : (r < kZERO ? kZERO : r);
             const double pb = a.b56 && ord ? sq * cb : pow(rc, a.beta);
             a.rb[i] = pb;
             if (a.ra) a.ra[i] = a.a53 && ord ? r * c2 / pb : pow(rc, a.alpha);
         }
+        if (LWT) {
+            // lwt.py:106.  To the last bit as the general path has it: a point at a node's k_F is
+            // inside an interval or, at the last node, outside every one
+            const double kf = 2.0 * cbrt(a.threepi2 * r);
+            a.kf[i] = kf;
+            mm[0] = fmin(mm[0], kf);
+            mm[1] = fmax(mm[1], kf);
+            mm[2] = fmax(mm[2], r);
+        }
         if (a.V) a.V[i] = v;
     }
     block_sums<4>(s, partials);
+    if (LWT) {
+        const int kinds[3] = {1, 2, 2};
+        block_reduce_store<3>(mm, kinds, partials + 4 * (long long)gridDim.x);
+    }
 }
 
 // Block sums of ns slots into out[0..ns), in a fixed order, and (plan != 0) the
@@ -305,6 +323,12 @@ struct PostK {
     const double* ra;
     long long N;
     double vw_y, alpha, beta, half_alpha;  // 0.5 / alpha
+    // density-dependent kernel
+    const double* kf;
+    const double* pot1[4];
+    const double* pot2;
+    const double* pot3[4];
+    double rhomax, ld, kfclip;
 };
 
 // Pointwise post-pass: vW and Hartree potentials, the Wang-Teter potential
@@ -341,6 +365,27 @@ __global__ void __launch_bounds__(RED_THREADS) k_post(PostK a, double* partials)
                 const double pa = a.ra[i];
                 s[2] += c1 * pa;
                 if (a.V) v += a.alpha * (pa * ri) * c1 + a.beta * (pb * ri) * a.nl2[i];
+            }
+        }
+        if (a.pot1[0]) {
+            auto parts = [&](const double* const (&p)[4]) {  // null: no part
+                double x = 0.0;
+                for (int k = 0; k < 4; ++k)
+                    if (p[k]) x += p[k][i];
+                return x;
+            };
+            // low-density factor (lwt.py:315-322) and the combination (:324-339)
+            double f = 1.0;
+            if (r < 1e-6) f = pow(fabs(r), a.ld) / pow(a.rhomax, a.ld);
+            if (r < 0.0) f = 0.0;
+            const double rc = ord ? ri : 1.0 / (r > 0.0 ? r : tiny);
+            const double pa = a.ra ? a.ra[i] : a.rb[i], p1 = parts(a.pot1) * f;
+            s[2] += pa * p1;
+            if (a.V) {
+                const double p2 = a.pot2 ? a.pot2[i] * f : p1;
+                const double p3 = parts(a.pot3) * f;
+                const double kf = fmin(a.kf[i], a.kfclip);
+                v += a.alpha * (pa * rc) * p1 + (a.beta * (a.rb[i] * rc) * p2 + kf * (1.0 / 3.0) * (pa * rc) * p3);
             }
         }
         if (a.V) a.V[i] = v;
@@ -425,43 +470,59 @@ void c2r(ofdft_grid* g, double2* const* in, double* const* out, int nf, cudaStre
     rows_c2r(p, g->sms, in, out, nf, st);
 }
 
-int local_enqueue(ofdft_grid* g, Scratch& sc, const LocalArgs& a, cudaStream_t st) {
+static int point_blocks(const ofdft_grid* g) {
+    return (int)std::max(1LL, std::min((long long)g->sms * 8, (g->N + RED_THREADS - 1) / RED_THREADS));
+}
+
+int local_begin(ofdft_grid* g, Scratch& sc, const LocalArgs& a, Fields& f, cudaEvent_t copied, cudaStream_t st) {
     const Grid3& p = *grid_plans(g);
     const long long N = g->N;
     const size_t rb = g->real_bytes(), cb = g->cplx_bytes();
     const int sms = g->sms;
-    const bool same = std::fabs(a.wt_beta - a.wt_alpha) < 1e-9;
-    double* sq = a.vw ? (double*)sc.get("sq", rb) : nullptr;
-    double* rbp = a.wt ? (double*)sc.get("rb", rb) : nullptr;
-    double* rap = a.wt && !same ? (double*)sc.get("ra", rb) : nullptr;
-    const int blocks = (int)std::max(1LL, std::min((long long)sms * 8, (N + RED_THREADS - 1) / RED_THREADS));
-    double* part = (double*)sc.get("fix_part", (size_t)blocks * 4 * sizeof(double));
+    const bool nl = a.wt || a.lwt, same = std::fabs(a.beta - a.alpha) < (a.wt ? 1e-9 : 1e-8);
+    f.sq = a.vw ? (double*)sc.get("sq", rb) : nullptr;
+    f.rb = nl ? (double*)sc.get("rb", rb) : nullptr;
+    f.ra = nl && !same ? (double*)sc.get("ra", rb) : nullptr;
+    f.kf = a.lwt ? (double*)sc.get("kf", rb) : nullptr;
+    const int blocks = point_blocks(g);
+    double* part = (double*)sc.get("fix_part", (size_t)blocks * 7 * sizeof(double));
     const Consts k = make_consts();
 
     PreK pk{};
     pk.rho = a.rho;
     pk.vloc = a.vloc;
     pk.V = a.V;
-    pk.sq = sq;
-    pk.rb = rbp;
-    pk.ra = rap;
+    pk.sq = f.sq;
+    pk.rb = f.rb;
+    pk.ra = f.ra;
+    pk.kf = f.kf;
     pk.N = N;
     pk.tf = a.tf;
     pk.xc = a.xc;
-    pk.b56 = a.wt_beta == 5.0 / 6.0;
-    pk.a53 = std::fabs(a.wt_alpha + a.wt_beta - 5.0 / 3.0) < 4e-16;
+    pk.b56 = a.beta == 5.0 / 6.0;
+    pk.a53 = std::fabs(a.alpha + a.beta - 5.0 / 3.0) < 4e-16;
     pk.tf_x = a.tf_x;
-    pk.alpha = a.wt_alpha;
-    pk.beta = a.wt_beta;
+    pk.alpha = a.alpha;
+    pk.beta = a.beta;
     pk.cE = k.cTF_E;
     pk.cV = k.cTF_V;
+    pk.threepi2 = k.threepi2;
     pk.lda = LdaRoots{k.lda_rs, std::sqrt(k.lda_rs), k.lda_ex, k.lda_vx};
-    k_pre<<<blocks, RED_THREADS, 0, st>>>(pk, part);
+    if (a.lwt) k_pre<true><<<blocks, RED_THREADS, 0, st>>>(pk, part);
+    else k_pre<false><<<blocks, RED_THREADS, 0, st>>>(pk, part);
     OFDFT_LAUNCH_CHECK();
-    k_sums<<<1, 128, 0, st>>>(part, blocks, 4, g->d_results, a.wt, a.wtstate, a.wt_rho0, 1.0 / (double)N, a.wt_alpha,
-                              a.wt_beta, a.cTF_wt);
+    k_sums<<<1, 128, 0, st>>>(part, blocks, 4, g->d_results, a.wt, a.wtstate, a.wt_rho0, 1.0 / (double)N, a.alpha,
+                              a.beta, a.cTF_wt);
     OFDFT_LAUNCH_CHECK();
-    int launches = 4;
+    int launches = 2;
+    if (a.lwt) {
+        reduce_finalize<<<3, RED_THREADS, 0, st>>>(part + 4 * (size_t)blocks, blocks, 3, 1ull | (2ull << 2) | (2ull << 4),
+                                                   g->d_results + 4);
+        OFDFT_LAUNCH_CHECK();
+        OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 7 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        OFDFT_CK(cudaEventRecord(copied, st));
+        ++launches;
+    }
 
     // fields to transform, their factors and what they become
     const double* in[4];
@@ -476,18 +537,29 @@ int local_enqueue(ofdft_grid* g, Scratch& sc, const LocalArgs& a, cudaStream_t s
         m.kind[nf] = kind;
         return out[nf++];
     };
-    PostK q{};
-    if (a.h) q.vH = field(a.rho, "rhoG", "vH", F_HARTREE);
-    if (a.vw) q.lap = field(sq, "sqG", "lap", F_VW);
-    if (a.wt) q.nl1 = field(rbp, "rbG", "nl1", F_WT);
-    if (rap) q.nl2 = field(rap, "raG", "nl2", F_WT);
+    if (a.h) f.vH = field(a.rho, "rhoG", "vH", F_HARTREE);
+    if (a.vw) f.lap = field(f.sq, "sqG", "lap", F_VW);
+    if (a.wt) f.nl1 = field(f.rb, "rbG", "nl1", F_WT);
+    if (a.wt && f.ra) f.nl2 = field(f.ra, "raG", "nl2", F_WT);
+    const int back = nf;  // fields that are transformed back
+    if (a.lwt) {
+        in[nf] = f.rb;
+        f.rbG = sp[nf++] = (double2*)sc.get("rbG", cb);
+    }
     if (nf > 0) {
         rows_r2c(p, sms, in, sp, nf, st);
         cols<1>(p, sms, sp, nf, false, st);
+        launches += 2;
+    }
+    if (a.lwt) {
+        cols<0>(p, sms, &f.rbG, 1, false, st);
+        ++launches;
+    }
+    if (back > 0) {
         const Shape s = shape_of(p.p0, col_lines<0>(p), sms, true);
         m.c.g = p;
         m.c.lb = s.lb;
-        for (int f = 0; f < nf; ++f) m.c.sp[f] = sp[f];
+        for (int i = 0; i < back; ++i) m.c.sp[i] = sp[i];
         m.geo = g->geo;
         m.K = a.wtK;
         m.state = a.wtstate;
@@ -495,27 +567,44 @@ int local_enqueue(ofdft_grid* g, Scratch& sc, const LocalArgs& a, cudaStream_t s
         m.invN = 1.0 / (double)N;
         const size_t smem = tile_smem(p.p0, s.lb, 1) + (size_t)p.n0 * sizeof(double2);
         smem_optin(k_cols_mul, smem);
-        k_cols_mul<<<dim3(col_blocks(col_lines<0>(p), s.lb), nf), s.threads, smem, st>>>(m);
+        k_cols_mul<<<dim3(col_blocks(col_lines<0>(p), s.lb), back), s.threads, smem, st>>>(m);
         OFDFT_LAUNCH_CHECK();
-        cols<1>(p, sms, sp, nf, true, st);
-        rows_c2r(p, sms, sp, out, nf, st);
-        launches += 5;
+        cols<1>(p, sms, sp, back, true, st);
+        rows_c2r(p, sms, sp, out, back, st);
+        launches += 3;
     }
+    return launches;
+}
+
+int local_finish(ofdft_grid* g, Scratch& sc, const LocalArgs& a, const Fields& f, const LwtPost& w, cudaStream_t st) {
+    const int blocks = point_blocks(g);
+    double* part = (double*)sc.get("fix_part", (size_t)blocks * 7 * sizeof(double));
+    PostK q{};
     q.rho = a.rho;
     q.V = a.V;
-    q.sq = sq;
-    q.rb = rbp;
-    q.ra = rap;
-    q.N = N;
+    q.sq = f.sq;
+    q.lap = f.lap;
+    q.vH = f.vH;
+    q.nl1 = f.nl1;
+    q.nl2 = f.nl2;
+    q.rb = f.rb;
+    q.ra = f.ra;
+    q.N = g->N;
     q.vw_y = a.vw_y;
-    q.alpha = a.wt_alpha;
-    q.beta = a.wt_beta;
-    q.half_alpha = 0.5 / a.wt_alpha;
+    q.alpha = a.alpha;
+    q.beta = a.beta;
+    q.half_alpha = 0.5 / a.alpha;
+    q.kf = f.kf;
+    q.pot2 = w.pot2;
+    for (int i = 0; i < 4; ++i) q.pot1[i] = w.pot1[i], q.pot3[i] = w.pot3[i];
+    q.rhomax = w.rhomax;
+    q.ld = w.ld;
+    q.kfclip = w.kfclip;
     k_post<<<blocks, RED_THREADS, 0, st>>>(q, part);
     OFDFT_LAUNCH_CHECK();
     k_sums<<<1, 128, 0, st>>>(part, blocks, 3, g->d_results + 16, 0, nullptr, 0.0, 0.0, 0.0, 0.0, 0.0);
     OFDFT_LAUNCH_CHECK();
-    return launches;
+    return 2;
 }
 
 }  // namespace fix

@@ -790,6 +790,7 @@ struct ofdft_eval {
     // density-dependent kernel
     void* tab_c = nullptr;
     void* tab_cd = nullptr;
+    double* tab_x = nullptr;  // its knots (float64 node kernels)
     int tab_nint = 0;
     double tab_step = 0, tab_limit = 0, tab_limitd = 0;
     double* d_nodes = nullptr;  // [k (kMaxNodes), 1/k, k+1e-18]
@@ -997,6 +998,35 @@ struct LwtPlan {
     double kfclip = INFINITY;
 };
 
+// The nodes of an evaluation from the density's k_F range (lwt.py:115-190), uploaded
+LwtPlan plan_lwt(ofdft_eval* e, double kf_l, double kf_r, cudaStream_t st) {
+    const ofdft_config& c = e->cfg;
+    LwtPlan lp;
+    if (std::fabs(kf_r - kf_l) >= 1e-8) {  // lwt.py:115-124
+        lp.active = true;
+        const bool fmin_ = !std::isnan(c.lwt_kfmin), fmax_ = !std::isnan(c.lwt_kfmax);
+        double b0, b1;
+        guess_kf_bound(kf_l, kf_r, fmin_, c.lwt_kfmin, fmax_, c.lwt_kfmax, e->kf_set_min, e->kf_st_min, e->kf_set_max,
+                       e->kf_st_max, b0, b1);
+        lp.kfclip = b1;
+        double kmin_c = std::min(kf_l, b1), kmax_c = std::min(kf_r, b1);
+        double kfMin = fmin_ ? c.lwt_kfmin : std::max(kmin_c, b0);
+        double kfMax = fmax_ ? c.lwt_kfmax : kmax_c;
+        lp.nodes = kf_nodes(kfMin, kfMax, c.lwt_nsp, c.lwt_delta, c.lwt_ratio);
+        OFDFT_REQUIRE((int)lp.nodes.size() <= kMaxNodes && lp.nodes.size() >= 2,
+                      "density-dependent kernel: %zu nodes (max %d)", lp.nodes.size(), kMaxNodes);
+        const int m = (int)lp.nodes.size();
+        for (int i = 0; i < m; ++i) {
+            e->h_nodes[i] = lp.nodes[i];
+            e->h_nodes[kMaxNodes + i] = 1.0 / lp.nodes[i];
+            e->h_nodes[2 * kMaxNodes + i] = lp.nodes[i] + 1e-18;
+        }
+        OFDFT_CK(cudaMemcpyAsync(e->d_nodes, e->h_nodes, 3 * kMaxNodes * sizeof(double), cudaMemcpyHostToDevice, st));
+    }
+    e->last_nsp = lp.active ? (int)lp.nodes.size() : 0;
+    return lp;
+}
+
 // ------------------------------------------------ fused k_F-node pipeline (host)
 constexpr int kFzMaxNodes = 1024;  // node bounds (6 floats each) staged in shared memory
 
@@ -1056,7 +1086,7 @@ void fz_tables(ofdft_eval* e) {
     *e->h_fz_err = 0;
     upload_now(e->d_fz_err, e->h_fz_err, sizeof(unsigned));
     OFDFT_CK(cudaStreamCreateWithFlags(&e->fz_st2, cudaStreamNonBlocking));
-    OFDFT_CK(cudaEventCreateWithFlags(&e->fz_fork, cudaEventDisableTiming));
+    if (!e->fz_fork) OFDFT_CK(cudaEventCreateWithFlags(&e->fz_fork, cudaEventDisableTiming));
     OFDFT_CK(cudaEventCreateWithFlags(&e->fz_join, cudaEventDisableTiming));
 }
 
@@ -1492,31 +1522,8 @@ void compute_t(ofdft_eval* e, const T* rho, T* V, unsigned calc, double* energie
     } else if (lwt) {
         OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, PRE_NS * sizeof(double), cudaMemcpyDeviceToHost, st));
         OFDFT_CK(cudaStreamSynchronize(st));
-        const double kf_l = g->h_results[4], kf_r = g->h_results[5];
         rhomax = g->h_results[6];
-        if (std::fabs(kf_r - kf_l) >= 1e-8) {  // lwt.py:115-124
-            lp.active = true;
-            const bool fmin_ = !std::isnan(c.lwt_kfmin), fmax_ = !std::isnan(c.lwt_kfmax);
-            double b0, b1;
-            guess_kf_bound(kf_l, kf_r, fmin_, c.lwt_kfmin, fmax_, c.lwt_kfmax, e->kf_set_min, e->kf_st_min,
-                           e->kf_set_max, e->kf_st_max, b0, b1);
-            lp.kfclip = b1;
-            double kmin_c = std::min(kf_l, b1), kmax_c = std::min(kf_r, b1);
-            double kfMin = fmin_ ? c.lwt_kfmin : std::max(kmin_c, b0);
-            double kfMax = fmax_ ? c.lwt_kfmax : kmax_c;
-            lp.nodes = kf_nodes(kfMin, kfMax, c.lwt_nsp, c.lwt_delta, c.lwt_ratio);
-            OFDFT_REQUIRE((int)lp.nodes.size() <= kMaxNodes && lp.nodes.size() >= 2,
-                          "density-dependent kernel: %zu nodes (max %d)", lp.nodes.size(), kMaxNodes);
-            const int m = (int)lp.nodes.size();
-            for (int i = 0; i < m; ++i) {
-                e->h_nodes[i] = lp.nodes[i];
-                e->h_nodes[kMaxNodes + i] = 1.0 / lp.nodes[i];
-                e->h_nodes[2 * kMaxNodes + i] = lp.nodes[i] + 1e-18;
-            }
-            OFDFT_CK(cudaMemcpyAsync(e->d_nodes, e->h_nodes, 3 * kMaxNodes * sizeof(double), cudaMemcpyHostToDevice,
-                                     st));
-        }
-        e->last_nsp = lp.active ? (int)lp.nodes.size() : 0;
+        lp = plan_lwt(e, g->h_results[4], g->h_results[5], st);
     }
 
     // ---- forward transforms
@@ -1806,24 +1813,42 @@ void collect_energies(ofdft_eval* e, double* energies) {
 }
 
 // Whether ofdft_eval_compute takes the float64 evaluation on integer-pipe transforms
-// (fix_eval.cu): TF, vW, LDA, Hartree, PP and the Wang-Teter kernel without smoothing
-// or corrections, on axes the plans cover.  It is 2 to 8 times faster than the general
-// path, whose float64 transforms and powers saturate the slow float64 pipe.
+// (fix_eval.cu, fix_lwt.cu): TF, vW, LDA, Hartree, PP, the Wang-Teter kernel and the
+// density-dependent kernel without smoothing or corrections, on axes the plans cover.  It is
+// 2 to 8 times faster than the general path, whose float64 transforms and powers saturate
+// the slow float64 pipe.  An explicit CUFFT pipeline and per-kernel profiling stay with the
+// general path.
 bool fix_applies(ofdft_eval* e) {
     const ofdft_config& c = e->cfg;
-    const int known = OFDFT_KE_TF | OFDFT_KE_VW | OFDFT_KE_WT;
-    return e->g->prec == OFDFT_F64 && !(c.kedf_terms & ~known) && !(c.vw_sigma > 0.0) && !c.wte && !c.external &&
-           !((c.kedf_terms & OFDFT_KE_WT) && c.wt_kernel != OFDFT_LWT_KERNEL_WT) && !e->prof &&
-           fix::grid_plans(e->g) != nullptr;
+    const int known = OFDFT_KE_TF | OFDFT_KE_VW | OFDFT_KE_WT | OFDFT_KE_LWT;
+    if (e->g->prec != OFDFT_F64 || (c.kedf_terms & ~known) || c.vw_sigma > 0.0 || c.wte || c.external || e->prof)
+        return false;
+    if ((c.kedf_terms & OFDFT_KE_WT) && c.wt_kernel != OFDFT_LWT_KERNEL_WT) return false;
+    if ((c.kedf_terms & OFDFT_KE_LWT) &&
+        (c.lwt_family != OFDFT_LWT_FAMILY_LWT || c.lwt_pipeline != OFDFT_LWT_PIPE_AUTO))
+        return false;
+    return fix::grid_plans(e->g) != nullptr;
+}
+
+// The kernel table's knots l step, for the float64 node kernels
+const double* table_knots(ofdft_eval* e) {
+    if (!e->tab_x) {
+        std::vector<double> x(e->tab_nint + 1);
+        for (int l = 0; l <= e->tab_nint; ++l) x[l] = (double)l * e->tab_step;
+        OFDFT_CK(cudaMalloc(&e->tab_x, x.size() * sizeof(double)));
+        upload_now(e->tab_x, x.data(), x.size() * sizeof(double));
+    }
+    return e->tab_x;
 }
 
 void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, double* energies, cudaStream_t st) {
     ofdft_grid* g = e->g;
     const ofdft_config& c = e->cfg;
     const bool wantV = (calc & OFDFT_CALC_V) != 0;
+    const bool wt = c.kedf_terms & OFDFT_KE_WT, lwt = c.kedf_terms & OFDFT_KE_LWT;
+    OFDFT_REQUIRE(!lwt || e->tab_set, "k_F-node kernel: no table set (ofdft_eval_set_lwt_table)");
     OFDFT_REQUIRE(!(c.pseudo && !e->have_vloc), "ofdft_eval_compute: pseudo enabled but no v_loc set");
     OFDFT_REQUIRE(!(wantV && !V), "ofdft_eval_compute: V requested but v_out is NULL");
-    const bool wt = c.kedf_terms & OFDFT_KE_WT;
     fix::LocalArgs a{};
     a.rho = rho;
     a.vloc = c.pseudo ? (const double*)e->vloc : nullptr;
@@ -1831,23 +1856,71 @@ void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, dou
     a.tf = (c.kedf_terms & OFDFT_KE_TF) != 0;
     a.vw = (c.kedf_terms & OFDFT_KE_VW) != 0;
     a.wt = wt;
+    a.lwt = lwt;
     a.xc = c.xc_lda != 0;
     a.h = c.hartree != 0;
     a.tf_x = c.tf_x;
     a.vw_y = c.vw_y;
-    a.wt_alpha = c.wt_alpha;
-    a.wt_beta = c.wt_beta;
+    a.alpha = lwt ? c.lwt_alpha : c.wt_alpha;
+    a.beta = lwt ? c.lwt_beta : c.wt_beta;
     a.wt_x = c.wt_x;
     a.wt_rho0 = c.wt_rho0;
     a.wtstate = e->wtstate;
     a.wtK = wt ? (double*)e->sc.get("wtK", (size_t)g->Nc * sizeof(double)) : nullptr;
     a.cTF_wt = e->k.cTF_wt;
-    const int launches = fix::local_enqueue(g, e->sc, a, st);
+    if (lwt && !e->fz_fork) OFDFT_CK(cudaEventCreateWithFlags(&e->fz_fork, cudaEventDisableTiming));
+    fix::Fields f;
+    int launches = fix::local_begin(g, e->sc, a, f, e->fz_fork, st);
+    fix::LwtPost q;
+    bool active = false;
+    if (lwt) {
+        OFDFT_CK(cudaEventSynchronize(e->fz_fork));  // the k_F range; the local transforms go on
+        const LwtPlan lp = plan_lwt(e, g->h_results[4], g->h_results[5], st);
+        active = lp.active;
+        if (active) {
+            const size_t rb = g->real_bytes();
+            fix::LwtArgs r{};
+            r.kdd = wantV ? c.lwt_kdd : 1;
+            r.kf = f.kf;
+            r.rA = f.ra ? f.ra : f.rb;
+            r.rbG = f.rbG;
+            r.hermite = c.lwt_interp == OFDFT_INTERP_HERMITE;
+            const char* names[2][4] = {{"fx_p1a", "fx_p1b", "fx_p1c", "fx_p1d"}, {"fx_p3a", "fx_p3b", "fx_p3c", "fx_p3d"}};
+            for (int i = 0; i < 4; ++i) {
+                if (fix::lwt_has(1, i, r.hermite)) q.pot1[i] = r.pot1[i] = (double*)e->sc.get(names[0][i], rb);
+                if (r.kdd == 3 && fix::lwt_has(3, i, r.hermite))
+                    q.pot3[i] = r.pot3[i] = (double*)e->sc.get(names[1][i], rb);
+            }
+            r.pot2 = r.kdd > 1 ? (double*)e->sc.get("pot2", rb) : nullptr;
+            r.tab_c = (const double*)e->tab_c;
+            r.tab_cd = (const double*)e->tab_cd;
+            r.tab_x = table_knots(e);
+            r.nint = e->tab_nint;
+            r.step = e->tab_step;
+            r.etamax = c.lwt_etamax;
+            r.limit = e->tab_limit;
+            r.limitd = e->tab_limitd;
+            r.kn = e->d_nodes;
+            r.invk = e->d_nodes + kMaxNodes;
+            r.kup = e->d_nodes + 2 * kMaxNodes;
+            r.m = (int)lp.nodes.size();
+            r.max_batch = c.lwt_max_batch;
+            r.kfclip = lp.kfclip;
+            launches += fix::lwt_enqueue(g, e->sc, r, st);
+            q.pot2 = r.pot2;
+            q.rhomax = g->h_results[6];
+            q.ld = std::max(0.1, c.lwt_ldw);
+            q.kfclip = lp.kfclip;
+        }
+    }
+    launches += fix::local_finish(g, e->sc, a, f, q, st);
     OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 24 * sizeof(double), cudaMemcpyDeviceToHost, st));
     e->pend = {};
     e->pend.tf = a.tf;
     e->pend.vw = a.vw;
     e->pend.wt = wt;
+    e->pend.lwt = lwt;
+    e->pend.lp_active = active;
     e->pend.xc = a.xc;
     e->pend.h = a.h;
     e->pend.pp = a.vloc != nullptr;
@@ -2264,6 +2337,7 @@ void ofdft_eval_destroy(ofdft_eval* e) {
     if (e->wtstate) cudaFree(e->wtstate);
     if (e->tab_c) cudaFree(e->tab_c);
     if (e->tab_cd) cudaFree(e->tab_cd);
+    if (e->tab_x) cudaFree(e->tab_x);
     if (e->d_nodes) cudaFree(e->d_nodes);
     if (e->h_nodes) cudaFreeHost(e->h_nodes);
     if (e->fz_tw) cudaFree(e->fz_tw);
