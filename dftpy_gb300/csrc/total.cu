@@ -41,6 +41,8 @@ struct PreArgs {
     T* rb;
     T* ra;
     T* kf;
+    T* c5;  // split pre-pass: (rho^5)^(1/3) and the XC energy density, for the sums
+    T* ex;
     long long N;
     int tf, vw, xc, pp, ext, nl, lwt, same_ab, wantV;
     int tf_v;       // add the TF potential (off under WTE, which scales it afterwards)
@@ -56,8 +58,9 @@ struct PreArgs {
 constexpr int PRE_NS = 9;
 
 // Pointwise pre-pass.  All arithmetic runs in the grid precision T; sums run
-// per thread in RunSum<T> and across threads in float64.
-template <typename T>
+// per thread in RunSum<T> and across threads in float64.  SPLIT leaves the sums to
+// k_prepass_sums, so that any number of blocks may share the points.
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(RED_THREADS) k_prepass(PreArgs<T> a, double* partials) {
     using M = T;
     RunSum<M> sum[6];
@@ -72,29 +75,34 @@ __global__ void __launch_bounds__(RED_THREADS) k_prepass(PreArgs<T> a, double* p
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
         const M r = a.rho[i];
         M v = (M)0;
-        sum[3].add(r);
-        rmax = r > rmax ? r : rmax;
+        if (!SPLIT) {
+            sum[3].add(r);
+            rmax = r > rmax ? r : rmax;
+        }
         if (a.tf) {
             // PowerInt(rho, 5, 3): repeated products then cbrt (math_utils.py:158-176)
             M r5 = r * r;
             r5 *= r;
             r5 *= r;
             r5 *= r;
-            sum[0].add(mcbrt(r5) * cTF_E);
+            const M c5 = mcbrt(r5);
+            if (SPLIT) a.c5[i] = c5;
+            else sum[0].add(c5 * cTF_E);
             if (a.wantV && a.tf_v) v += cTF_V * mcbrt(r * r) * tf_x;
         }
         if (a.xc) {
             M ex, vx;
             lda_point(r, lc, ex, vx);
-            sum[1].add(ex * r);
+            if (SPLIT) a.ex[i] = ex;
+            else sum[1].add(ex * r);
             v += vx;
         }
         if (a.pp) {
             const M vl = a.vloc[i];
-            sum[2].add(vl * r);
+            if (!SPLIT) sum[2].add(vl * r);
             v += vl;
         }
-        if (a.dttf) {  // TTF - TF (tf.py:101-204): theta = T / v_TF, fitted forms below/above 1.36
+        if (!SPLIT && a.dttf) {  // TTF - TF (tf.py:101-204): theta = T / v_TF, fitted forms below/above 1.36
             const M T = (M)a.temp, vtf = cTF_V * mcbrt(r * r), th = T / vtf, cc = (M)0.752252778063675;
             const M r2 = sqrt((M)2), r23 = (M)2 * r2;  // 2^0.5, 2^1.5
             const M tf_ed = mcbrt(r * r * r * r * r) * cTF_E;
@@ -126,7 +134,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_prepass(PreArgs<T> a, double* p
         }
         if (a.ext) {  // external_potential.py:30-35
             const M ve = a.vext[i];
-            sum[4].add(ve * r);
+            if (!SPLIT) sum[4].add(ve * r);
             v += ve;
         }
         if (a.vw) a.sq[i] = msqrt(r > (M)0 ? r : tiny);  // kedf/vw.py:34-44
@@ -138,13 +146,46 @@ __global__ void __launch_bounds__(RED_THREADS) k_prepass(PreArgs<T> a, double* p
         if (a.lwt) {
             const M kf = (M)2 * mcbrt(threepi2 * r);  // kedf/lwt.py:106
             a.kf[i] = kf;
-            kfmin = kf < kfmin ? kf : kfmin;
-            kfmax = kf > kfmax ? kf : kfmax;
+            if (!SPLIT) {
+                kfmin = kf < kfmin ? kf : kfmin;
+                kfmax = kf > kfmax ? kf : kfmax;
+            }
         }
         if (a.wantV) a.V[i] = v;
     }
+    if (SPLIT) return;
     double acc[PRE_NS] = {sum[0].get(), sum[1].get(), sum[2].get(), sum[3].get(), (double)kfmin, (double)kfmax,
                           (double)rmax, sum[4].get(), sum[5].get()};
+    block_reduce_store<PRE_NS>(acc, kinds, partials);
+}
+
+// The sums of a split pre-pass: the threads, points and orders of the other one, so the same
+// bits (a density optimisation amplifies a changed last bit of an energy 1e7 times)
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS) k_prepass_sums(PreArgs<T> a, double* partials) {
+    using M = T;
+    RunSum<M> sum[5];
+    M kfmin = (M)INFINITY, kfmax = -(M)INFINITY, rmax = -(M)INFINITY;
+    const int kinds[PRE_NS] = {0, 0, 0, 0, 1, 2, 2, 0, 0};
+    const M cTF_E = (M)a.k.cTF_E;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
+        const M r = a.rho[i];
+        sum[3].add(r);
+        rmax = r > rmax ? r : rmax;
+        if (a.tf) sum[0].add(a.c5[i] * cTF_E);
+        if (a.xc) sum[1].add(a.ex[i] * r);
+        if (a.pp) sum[2].add(a.vloc[i] * r);
+        if (a.ext) sum[4].add(a.vext[i] * r);
+        if (a.lwt) {
+            const M kf = a.kf[i];
+            kfmin = kf < kfmin ? kf : kfmin;
+            kfmax = kf > kfmax ? kf : kfmax;
+        }
+    }
+    double acc[PRE_NS] = {sum[0].get(), sum[1].get(), sum[2].get(), sum[3].get(), (double)kfmin, (double)kfmax,
+                          (double)rmax, sum[4].get(), 0.0};
     block_reduce_store<PRE_NS>(acc, kinds, partials);
 }
 
@@ -1423,7 +1464,24 @@ void compute_t(ofdft_eval* e, const T* rho, T* V, unsigned calc, double* energie
     {
         // algorithmic bytes: read rho (+ v_loc); write V, sqrt(rho), rho^beta (+ rho^alpha), k_F as active
         double b = Nd * s * (1 + pp + ext + wantV + vw + nl + (nl && !same_ab) + lwt);
-        timed(e, P_PREPASS, b, st, [&] { k_prepass<T><<<g->red_blocks, RED_THREADS, 0, st>>>(pa, g->d_partials); });
+        // The order of the sums fixes red_blocks blocks with 16 points per thread: on 53 of 152
+        // SMs at 60^3, where the float64 pipe is the bound.  Up to the size that gives every SM
+        // eight such blocks the points take a block per 256 of them, and the sums a pass of
+        // their own (60^3 with TF, WT, LDA and PP: 232 us, now 87 and 16).
+        const bool split = std::is_same<T, double>::value && !pa.dttf && g->red_blocks < 8 * g->sms;
+        if (split) {
+            pa.c5 = pa.tf ? (T*)e->sc.get("pre_c5", rb) : nullptr;
+            pa.ex = pa.xc ? (T*)e->sc.get("pre_ex", rb) : nullptr;
+        }
+        timed(e, P_PREPASS, b, st, [&] {
+            if (split) {
+                k_prepass<T, true><<<blocks_for(N, RED_THREADS, 1 << 20), RED_THREADS, 0, st>>>(pa, nullptr);
+                k_prepass_sums<T><<<g->red_blocks, RED_THREADS, 0, st>>>(pa, g->d_partials);
+            } else {
+                k_prepass<T, false><<<g->red_blocks, RED_THREADS, 0, st>>>(pa, g->d_partials);
+            }
+        });
+        launches += split;
     }
     OFDFT_LAUNCH_CHECK();
     unsigned long long kinds = (1ull << (2 * 4)) | (2ull << (2 * 5)) | (2ull << (2 * 6));
