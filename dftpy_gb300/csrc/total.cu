@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_prepass_sums(PreArgs<T> a, doub
     const int kinds[PRE_NS] = {0, 0, 0, 0, 1, 2, 2, 0, 0};
     const M cTF_E = (M)a.k.cTF_E;
     const long long stride = (long long)gridDim.x * blockDim.x;
-#pragma unroll 4
+#pragma unroll 8
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
         const M r = a.rho[i];
         sum[3].add(r);
@@ -692,6 +692,8 @@ struct PostArgs {
     int hc;
     const T* hc_c1;
     const T* hc_q;
+    T* pw;   // split post-pass, for the sums: the vW potential and the WT energy density
+    T* enl;
     long long N;
     int vw, h, wt, lwt, same_ab, wantV, kdd;
     double vw_y;
@@ -702,7 +704,8 @@ struct PostArgs {
 // slots: 0 vW, 1 Hartree, 2 NL
 constexpr int POST_NS = 3;
 
-template <typename T>
+// SPLIT: as k_prepass; without the density-dependent kernel
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(RED_THREADS) k_postpass(PostArgs<T> a, double* partials) {
     using M = T;  // working precision; sums run in RunSum<T>, then float64
     RunSum<M> sum[POST_NS];
@@ -717,12 +720,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_postpass(PostArgs<T> a, double*
             M s = a.sq[i];
             if (fabs(s) < tiny) s = tiny;
             const M pw = a.lap[i] / s;
-            if (r > (M)0) sum[0].add(r * pw);
+            if (SPLIT) a.pw[i] = pw;
+            else if (r > (M)0) sum[0].add(r * pw);
             v += pw * vw_y;
         }
         if (a.h) {
             const M vh = a.vH[i];
-            sum[1].add(vh * r);
+            if (!SPLIT) sum[1].add(vh * r);
             v += vh;
         }
         if (a.wt) {
@@ -733,14 +737,16 @@ __global__ void __launch_bounds__(RED_THREADS) k_postpass(PostArgs<T> a, double*
             if (a.same_ab) {
                 const M pot = (M)2 * alpha * (pb / rc) * c1;  // wt.py:19-23
                 if (a.wantV) {
-                    sum[2].add(pot * r / ((M)2 * alpha));  // wt.py:124-125
+                    const M enl = pot * r / ((M)2 * alpha);  // wt.py:124-125
+                    if (SPLIT) a.enl[i] = enl;
+                    else sum[2].add(enl);
                     vnl = pot;
-                } else {
+                } else if (!SPLIT) {
                     sum[2].add(c1 * pb);  // wt.py:44-56
                 }
             } else {
                 const M pa = a.ra[i];
-                sum[2].add(c1 * pa);
+                if (!SPLIT) sum[2].add(c1 * pa);
                 if (a.wantV) vnl = alpha * (pa / rc) * c1 + beta * (pb / rc) * a.nl2[i];
             }
             if (a.wantV) {
@@ -750,7 +756,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_postpass(PostArgs<T> a, double*
                     v += vnl;
             }
         }
-        if (a.lwt && a.hc) {
+        if (!SPLIT && a.lwt && a.hc) {
             // HC (hc.py:294-330): the energy without the low-density factor, the potential
             // factor * (alpha rho^(alpha-1) pot1 + beta rho^(beta-1) pot2 + c1 rho^alpha pot3 - div)
             const M rc = r < zero_clamp ? zero_clamp : r;
@@ -763,7 +769,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_postpass(PostArgs<T> a, double*
                 v += f * (alpha * (pa / rc) * a.pot1[i] + beta * (pb / rc) * a.pot2[i] + a.hc_c1[i] * pa * a.pot3[i] -
                           a.hc_q[i]);
             }
-        } else if (a.lwt) {
+        } else if (!SPLIT && a.lwt) {
             // low-density factor (lwt.py:315-322) and the final combination (:324-339)
             M f = (M)1;
             if (r < (M)1e-6) f = mpow(fabs(r), ld) / mpow(rhomax, ld);
@@ -782,6 +788,30 @@ __global__ void __launch_bounds__(RED_THREADS) k_postpass(PostArgs<T> a, double*
             }
         }
         if (a.wantV) a.V[i] = v;
+    }
+    if (SPLIT) return;
+    double acc[POST_NS] = {sum[0].get(), sum[1].get(), sum[2].get()};
+    block_sum_store<POST_NS>(acc, partials);
+}
+
+// The sums of a split post-pass, as k_prepass_sums
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS) k_postpass_sums(PostArgs<T> a, double* partials) {
+    using M = T;
+    RunSum<M> sum[POST_NS];
+    const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 8
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
+        const M r = a.rho[i];
+        if (a.vw) {
+            const M pw = a.pw[i];
+            if (r > (M)0) sum[0].add(r * pw);
+        }
+        if (a.h) sum[1].add(a.vH[i] * r);
+        if (a.wt) {
+            if (a.same_ab && a.wantV) sum[2].add(a.enl[i]);
+            else sum[2].add(a.nl1[i] * (a.same_ab ? a.rb[i] : a.ra[i]));
+        }
     }
     double acc[POST_NS] = {sum[0].get(), sum[1].get(), sum[2].get()};
     block_sum_store<POST_NS>(acc, partials);
@@ -1789,8 +1819,21 @@ void compute_t(ofdft_eval* e, const T* rho, T* V, unsigned calc, double* energie
         int reads = 1 + wantV + 2 * vw + h + (wt ? 2 + !same_ab * 2 : 0) +
                     (lw ? 1 + 1 + !same_ab + 1 + (kdd > 1) + (kdd == 3) : 0);
         double b = Nd * s * (reads + wantV);
-        timed(e, P_POSTPASS, b, st,
-              [&] { k_postpass<T><<<g->red_blocks, RED_THREADS, 0, st>>>(qa, g->d_partials); });
+        // by the pre-pass's rule (60^3 with vW, WT and Hartree: 48 us, now 16 and 12)
+        const bool split = std::is_same<T, double>::value && !qa.lwt && g->red_blocks < 8 * g->sms;
+        if (split) {
+            qa.pw = qa.vw ? (T*)e->sc.get("post_pw", rb) : nullptr;
+            qa.enl = qa.wt && same_ab && wantV ? (T*)e->sc.get("post_enl", rb) : nullptr;
+        }
+        timed(e, P_POSTPASS, b, st, [&] {
+            if (split) {
+                k_postpass<T, true><<<blocks_for(N, RED_THREADS, 1 << 20), RED_THREADS, 0, st>>>(qa, nullptr);
+                k_postpass_sums<T><<<g->red_blocks, RED_THREADS, 0, st>>>(qa, g->d_partials);
+            } else {
+                k_postpass<T, false><<<g->red_blocks, RED_THREADS, 0, st>>>(qa, g->d_partials);
+            }
+        });
+        launches += split;
     }
     OFDFT_LAUNCH_CHECK();
     timed(e, P_REDUCE, (double)g->red_blocks * POST_NS * 8, st, [&] {

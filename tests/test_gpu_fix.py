@@ -36,6 +36,12 @@ def test_evaluation(nr, kedf):
     assert abs(only.energy - ref["E"]) <= E_RTOL * max(1.0, abs(ref["E"]))
 
 
+@pytest.mark.parametrize("nr", [(11, 13, 2), (22, 23, 26)])  # one block of the sums; a partial last one
+@pytest.mark.parametrize("kedf", ["TFVW", "WT", "WT-ab"])
+def test_general_path_in_split_passes(nr, kedf):
+    test_evaluation(nr, kedf)
+
+
 @pytest.mark.parametrize("nr,opts", [
     ((2, 3, 4), dict(nsp=3)),
     ((16, 15, 14), dict(nsp=8, max_batch=3)),  # several batches of nodes, the last one short
