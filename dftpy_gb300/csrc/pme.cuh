@@ -50,15 +50,17 @@ __device__ __forceinline__ double bspline_mn_lane(double x, int order, int n, do
 }
 
 // ---------------------------------------------------------------------------
-// Deterministic spreading.  The grid is cut into 8^3 tiles, one block each, one thread per
-// grid point.  The block goes through the atoms in list order, 512 at a time: every thread
-// tests one atom's order^3 stencil against the tile, the hits are compacted in order into
-// shared memory, and every thread sums their contributions in that order in float64 and
-// stores its point once.  The sum at every point has a fixed order, so Q is the same bits on
-// every run (a per-atom scatter with global atomics sums in arrival order).  The test costs
-// tiles x atoms comparisons, 67 million for 2048 atoms on 256^3 (about 30 us); lists built
-// and sorted on the host took 2.5 ms there.
+// Deterministic spreading.  The grid is cut into 8 x 8 x 32 tiles, one block each, four grid
+// points (8 apart on axis 2) per thread.  The block goes through the atoms in list order, 512
+// at a time: every thread tests one atom's order^3 stencil against the tile, the hits are
+// compacted in order into shared memory, and every thread sums their contributions in that
+// order in float64 and stores its points once.  The sum at every point has a fixed order, so Q
+// is the same bits on every run (a per-atom scatter with global atomics sums in arrival order).
+// The test costs tiles x atoms comparisons and bounds the kernel, hence the long tiles (2048
+// atoms on 256^3: 149 us; 8^3 tiles: 404 us); lists built and sorted on the host took 2.5 ms
+// there.
 constexpr int kPmeTile = 8;
+constexpr int kPmeLong = 4;  // 8-point pieces of a tile along axis 2
 constexpr int kPmeThreads = kPmeTile * kPmeTile * kPmeTile;
 
 // Stencil base and B-spline weights of every list position: 16 lanes per atom and axis
@@ -91,13 +93,15 @@ __global__ void __launch_bounds__(kPmeThreads)
     __shared__ int hit[kPmeThreads];
     __shared__ int off[kPmeThreads][3];  // (1 + base - first point of the tile) mod n per axis
     __shared__ int count[kPmeThreads / 32];
-    const int T1 = (geo.n1 + kPmeTile - 1) / kPmeTile, T2 = (geo.n2 + kPmeTile - 1) / kPmeTile;
+    const int T1 = (geo.n1 + kPmeTile - 1) / kPmeTile;
+    constexpr int wide = kPmeTile * kPmeLong;
+    const int T2 = (geo.n2 + wide - 1) / wide;
     const int tid = blockIdx.x, nr[3] = {geo.n0, geo.n1, geo.n2};
-    const int lo[3] = {(tid / (T1 * T2)) * kPmeTile, ((tid / T2) % T1) * kPmeTile, (tid % T2) * kPmeTile};
+    const int lo[3] = {(tid / (T1 * T2)) * kPmeTile, ((tid / T2) % T1) * kPmeTile, (tid % T2) * wide};
     const int p[3] = {(int)(threadIdx.x >> 6), (int)((threadIdx.x >> 3) & 7), (int)(threadIdx.x & 7)};
     const bool in = lo[0] + p[0] < nr[0] && lo[1] + p[1] < nr[1] && lo[2] + p[2] < nr[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o1 = order + 1;
-    double v = 0.0;
+    double v[kPmeLong] = {};
     for (int q0 = 0; q0 < nlist; q0 += kPmeThreads) {
         const int q = q0 + threadIdx.x;
         int o[3] = {0, 0, 0};
@@ -108,7 +112,7 @@ __global__ void __launch_bounds__(kPmeThreads)
                 int t = 1 + base[3 * q + d] - lo[d];  // base in [0, n): t in (-n, n]
                 t = t < 0 ? t + nr[d] : (t >= nr[d] ? t - nr[d] : t);
                 o[d] = t;
-                on = on && t <= order + min(kPmeTile, nr[d] - lo[d]) - 2;
+                on = on && t <= order + min(d == 2 ? wide : kPmeTile, nr[d] - lo[d]) - 2;
             }
         }
         const unsigned b = __ballot_sync(0xffffffffu, on);
@@ -132,23 +136,34 @@ __global__ void __launch_bounds__(kPmeThreads)
         __syncthreads();
         if (!in) continue;
         for (int h = 0; h < total; ++h) {
-            int i0 = off[h][0] - p[0], j0 = off[h][1] - p[1], k0 = off[h][2] - p[2];
+            int i0 = off[h][0] - p[0], j0 = off[h][1] - p[1];
             i0 += i0 < 0 ? nr[0] : 0;
             j0 += j0 < 0 ? nr[1] : 0;
-            k0 += k0 < 0 ? nr[2] : 0;
-            if (i0 >= order || j0 >= order || k0 >= order) continue;
+            if (i0 >= order || j0 >= order) continue;
             const int a = hit[h];
             const double* M0 = M + (3 * (size_t)a) * o1;
             const double* M1 = M0 + o1;
             const double* M2 = M1 + o1;
             const double wa = w ? w[list ? list[a] : a] : 1.0;
-            // n >= order in practice; the loops also cover a stencil that wraps onto itself
-            for (int i = i0; i < order; i += nr[0])
-                for (int j = j0; j < order; j += nr[1])
-                    for (int k = k0; k < order; k += nr[2]) v += wa * M0[i + 1] * M1[j + 1] * M2[k + 1];
+#pragma unroll
+            for (int s = 0; s < kPmeLong; ++s) {
+                int k0 = off[h][2] - p[2] - s * kPmeTile;
+                k0 += k0 < 0 ? nr[2] : 0;
+                // n >= order in practice; the loops also cover a stencil that wraps onto itself
+                if (k0 >= 0 && k0 < order)
+                    for (int i = i0; i < order; i += nr[0])
+                        for (int j = j0; j < order; j += nr[1])
+                            for (int k = k0; k < order; k += nr[2]) v[s] += wa * M0[i + 1] * M1[j + 1] * M2[k + 1];
+            }
         }
     }
-    if (in) Q[((long long)(lo[0] + p[0]) * geo.n1 + lo[1] + p[1]) * geo.n2 + lo[2] + p[2]] = (T)v;
+    if (!in) return;
+    T* out = Q + ((long long)(lo[0] + p[0]) * geo.n1 + lo[1] + p[1]) * geo.n2;
+#pragma unroll
+    for (int s = 0; s < kPmeLong; ++s) {
+        const int k = lo[2] + p[2] + s * kPmeTile;
+        if (k < nr[2]) out[k] = (T)v[s];
+    }
 }
 
 // Q = the spread of the list's atoms with weights w (null: 1).  d_frac, d_list and d_w on
@@ -167,7 +182,7 @@ void pme_spread(Scratch& sc, const std::string& prefix, int nlist, int order, co
     k_pme_prep<<<(groups + 7) / 8, 128, 0, st>>>(d_frac, d_list, nlist, order, geo, base, M);
     OFDFT_LAUNCH_CHECK();
     auto tiles = [](int n) { return (n + kPmeTile - 1) / kPmeTile; };
-    const unsigned nt = (unsigned)tiles(geo.n0) * tiles(geo.n1) * tiles(geo.n2);
+    const unsigned nt = (unsigned)tiles(geo.n0) * tiles(geo.n1) * ((geo.n2 + kPmeTile * kPmeLong - 1) / (kPmeTile * kPmeLong));
     k_pme_tiles<T><<<nt, kPmeThreads, 0, st>>>(nlist, order, base, M, d_w, d_list, geo, Q);
     OFDFT_LAUNCH_CHECK();
 }
