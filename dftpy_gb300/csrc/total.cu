@@ -1234,7 +1234,8 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
     const double* knode = r.nd.k;
     const double* invk = r.nd.invk;
     int launches = 0;
-    // the rows that each node needs
+    // the rows that each node needs; their share of all rows, for the profile's byte counts
+    double share = 1.0;
     FzNeed need{};
     if (!split) {
         const int words = n1 / 32;
@@ -1254,6 +1255,14 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
         timed(e, P_LWT_INTERP, Nd * 4.0, st, [&] { k_fz_need<<<n0 * words, kFzRowThreads, smem, st>>>(na, bits); });
         OFDFT_LAUNCH_CHECK();
         ++launches;
+        if (e->prof) {
+            std::vector<unsigned> h((size_t)n0 * r.m * words);
+            OFDFT_CK(cudaMemcpyAsync(h.data(), bits, h.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+            OFDFT_CK(cudaStreamSynchronize(st));
+            long long on = 0;
+            for (unsigned b : h) on += __builtin_popcount(b);
+            share = (double)on / ((double)n0 * n1 * r.m);
+        }
     }
     if (two) {
         OFDFT_CK(cudaEventRecord(e->fz_fork, st));
@@ -1304,7 +1313,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
             const int grid = n0 * 8;
             auto launch = [&](auto kern, int plane0, float* pot) {
                 fz_smem_optin(kern, smem);
-                timed(e, P_LWT_INTERP, Ncd * 8.0 * nb + Nd * 4.0 * (1 + (first ? 1 : 2)), st,
+                timed(e, P_LWT_INTERP, Ncd * 8.0 * nb * share + Nd * 4.0 * (1 + (first ? 1 : 2)), st,
                       [&] { kern<<<grid, kS8RowThreads, smem, st>>>(ra, plane0, pot); });
                 OFDFT_LAUNCH_CHECK();
             };
@@ -1330,7 +1339,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
         if (!split) with_col(n1, [&](auto c1) {
             constexpr int N1 = decltype(c1)::value;
             const size_t smem = std::max(fz::col_slots(N1), kFzLines * fz::row_slots(N1)) * sizeof(float2);
-            timed(e, P_FZ_AXIS1, Ncd * 16.0 * nplanes, st,
+            timed(e, P_FZ_AXIS1, Ncd * 8.0 * nplanes * (1.0 + share), st,
                   [&] { k_fz_axis1<N1, +1><<<tiles1 * nplanes, N1, smem, st>>>(XY, d, tw.t1, need, j0, nb); });
         });
         OFDFT_LAUNCH_CHECK();
@@ -1342,7 +1351,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
             const int grid = (int)((long long)n0 * n1 / ROWS);
             auto launch = [&](auto kern, int plane0, float* pot) {
                 fz_smem_optin(kern, smem);
-                timed(e, P_LWT_INTERP, Ncd * 8.0 * nb + Nd * 4.0 * (1 + (first ? 1 : 2)), st,
+                timed(e, P_LWT_INTERP, Ncd * 8.0 * nb * share + Nd * 4.0 * (1 + (first ? 1 : 2)), st,
                       [&] { kern<<<grid, kFzRowThreads, smem, st>>>(ra, plane0, pot); });
                 OFDFT_LAUNCH_CHECK();
             };
@@ -1366,7 +1375,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
                 // radix-8 stage, axis 0 and the sum into pot2(G)
                 const size_t smem = fz8_row_smem(r.m, 1);
                 fz_smem_optin(k_fz_r2c_s8, smem);
-                timed(e, P_FZ_HAT, Nd * 8.0 + Ncd * 8.0 * nb, st2,
+                timed(e, P_FZ_HAT, Nd * 8.0 + Ncd * 8.0 * nb * share, st2,
                       [&] { k_fz_r2c_s8<<<n0 * 8, kS8RowThreads, smem, st2>>>(ra2); });
                 OFDFT_LAUNCH_CHECK();
                 with_col(n0, [&](auto c0) {
@@ -1388,7 +1397,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
                 const int grid = (int)((long long)n0 * n1 / ROWS);
                 auto hat = [&](auto kern) {
                     fz_smem_optin(kern, smem);
-                    timed(e, P_FZ_HAT, Nd * 8.0 + Ncd * 8.0 * hp * nb, st2,
+                    timed(e, P_FZ_HAT, Nd * 8.0 + Ncd * 8.0 * hp * nb * share, st2,
                           [&] { kern<<<grid, kFzRowThreads, smem, st2>>>(ra2); });
                 };
                 if (r.hermite) hat(k_fz_r2c_rows<HH, true>);
@@ -1398,7 +1407,7 @@ int fz_run(ofdft_eval* e, const FzRun& r, cudaStream_t st) {
             if (!split) with_col(n1, [&](auto c1) {
                 constexpr int N1 = decltype(c1)::value;
                 const size_t smem = std::max(fz::col_slots(N1), kFzLines * fz::row_slots(N1)) * sizeof(float2);
-                timed(e, P_FZ_AXIS1, Ncd * 16.0 * hp * nb, st2,
+                timed(e, P_FZ_AXIS1, Ncd * 8.0 * hp * nb * (1.0 + share), st2,
                       [&] { k_fz_axis1<N1, -1><<<tiles1 * hp * nb, N1, smem, st2>>>(XY2, d, tw.t1, need, j0, nb); });
             });
             OFDFT_LAUNCH_CHECK();

@@ -110,7 +110,9 @@ enum { OFDFT_GGA_LKT = 0, OFDFT_GGA_LKTVW, OFDFT_GGA_DK, OFDFT_GGA_LLP, OFDFT_GG
 enum { OFDFT_INTERP_LINEAR = 0, OFDFT_INTERP_HERMITE = 1 };
 /* k_F-node kernel pipeline: AUTO takes FUSED where it applies (float32 grid,
  * the LWT family, every axis a power of two in 32..256, the last axis up to
- * 512; linear or cubic Hermite interpolation) and CUFFT otherwise; FUSED fails
+ * 512; linear or cubic Hermite interpolation), in ofdft_eval_compute on a float64
+ * grid with 2, 3, 5, 7-smooth axes up to 512 the same arrangement on integer-pipe
+ * transforms, and CUFFT otherwise; FUSED fails
  * with OFDFT_EINVAL where it does not apply.  FUSED folds the node kernel, the
  * interpolation and the pot2 sum into the library's own tile FFTs; CUFFT runs
  * them as separate passes around batched cuFFT transforms.  Both compute the
