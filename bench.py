@@ -1185,7 +1185,9 @@ def c2_workload(args, emit=True):
     ew = D.ewald(ions=ions, grid=grid, PME=True)
     F_gpu = ew.forces
     t_ew = time.perf_counter() - t0
-    # stress of every term at the same density (warm once: plans, v_loc)
+    # stress of every term at the same density (warm once: plans, v_loc); the Hartree term
+    # takes the energy that the class cached at the last evaluation
+    tot(rho)
     tot.get_stress(rho)
     torch.cuda.synchronize()
     t0 = time.perf_counter()
