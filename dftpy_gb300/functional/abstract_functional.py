@@ -45,7 +45,6 @@ class NativeEval:
         h = _lib.C.c_void_p()
         _lib.check(self.lib.ofdft_eval_create(grid.native_for(dtype), _lib.C.byref(cfg), _lib.C.byref(h)))
         self.h = h
-        self.vloc_token = None
         self._E = np.zeros(_lib.NE, dtype=np.float64)
 
     def __del__(self):
@@ -56,14 +55,12 @@ class NativeEval:
         except Exception:
             pass
 
-    def set_vloc(self, vloc, token):
-        """Copy a local potential in, unless the evaluator holds it already: ``token``
-        names its geometry, precision and in-place version (None: always copied)."""
-        if token is not None and self.vloc_token == token:
-            return
+    def set_vloc(self, vloc):
+        """Copy a local potential in.  Every evaluation copies: nothing tells whether the tensor
+        was written to since (.data, DLPack and raw pointers leave PyTorch's version counter
+        alone), or whether the handle was given another one."""
         t = vloc.as_subclass(torch.Tensor).contiguous()
         _lib.check(self.lib.ofdft_eval_set_vloc(self.h, _lib.C.c_void_p(t.data_ptr()), stream_ptr()))
-        self.vloc_token = token
 
     def set_external(self, v):
         """Copy a frozen external potential (device tensor of the evaluator dtype) in."""

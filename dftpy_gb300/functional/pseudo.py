@@ -142,7 +142,6 @@ class LocalPseudo(NativeFunctional):
                                   BsplineOrder=self.BsplineOrder)
         self._native = {}
         self._vreal = {}
-        self._version = object()
         self.ewald = None
         self._ions = None
         self._grid = None
@@ -160,7 +159,7 @@ class LocalPseudo(NativeFunctional):
     @grid.setter
     def grid(self, value):
         self._grid = value.get_direct() if hasattr(value, "get_direct") else value
-        self._native, self._vreal, self._version = {}, {}, object()
+        self._native, self._vreal = {}, {}
 
     @property
     def ions(self):
@@ -181,7 +180,7 @@ class LocalPseudo(NativeFunctional):
             except Exception:
                 pass
         self._ions = ions
-        self._native, self._vreal, self._version = {}, {}, object()
+        self._native, self._vreal = {}, {}
 
     @property
     def zval(self):
@@ -248,9 +247,7 @@ class LocalPseudo(NativeFunctional):
     def prepare(self, ev, grid, dtype):
         if grid is not self.grid and not (grid == self.grid):
             raise ValueError("density grid differs from the pseudopotential grid")
-        v = self.vreal_for(dtype)
-        # an inference-mode tensor keeps no in-place version: it is copied every time
-        ev.set_vloc(v, token=None if v.is_inference() else (self._version, dtype, v._version))
+        ev.set_vloc(self.vreal_for(dtype))
 
     def forces(self, rho):
         """LocalPseudo.forces (:260-270): PME or exact structure factor."""
@@ -301,13 +298,13 @@ class LocalPseudo(NativeFunctional):
             if v.shape != self.readpp.vp[k].shape:
                 raise ValueError("table of %s must keep its %d points" % (k, len(self.readpp.vp[k])))
             self.readpp._vp[k] = v.copy()
-        self._native, self._vreal, self._version = {}, {}, object()
+        self._native, self._vreal = {}, {}
 
     def set_positions(self, positions):
         """Move the ions (Bohr); drops cached v_loc and the Ewald object.  The native handles
         stay, with their radial tables on the grid."""
         self._ions.positions = np.array(positions, dtype=np.float64).reshape(self._ions.nat, 3)
-        self._vreal, self._version = {}, object()
+        self._vreal = {}
         try:
             for h in self._native.values():
                 self._set_ions(h)
