@@ -184,14 +184,17 @@ class ConfigCache:
         self.cfg = self.key = None
         self.fusable = False
 
+    def _holds(self, functionals):
+        if self._states is None or len(self._states) != len(functionals):
+            return False
+        for f, (g, old) in zip(functionals, self._states):
+            if f is not g or old is None or not _same(f.config_state(), old):
+                return False
+        return True
+
     def update(self, functionals):
-        states = [(f, f.config_state()) for f in functionals]
-        try:
-            same = self._states is not None and len(states) == len(self._states) and all(
-                f is g and a is not None and bool(a == b) for (f, a), (g, b) in zip(states, self._states))
-        except (ValueError, TypeError, RuntimeError):  # option values that do not compare to a truth value
-            same = False
-        if not same:
+        if not self._holds(functionals):
+            states = [(f, _copied(f.config_state())) for f in functionals]
             cfg, seen, fusable = empty_config(), 0, True
             for f in functionals:
                 one = empty_config()
@@ -201,8 +204,33 @@ class ConfigCache:
                 seen |= bits
                 f.configure(cfg)
             self.cfg, self.key, self.fusable = cfg, config_key(cfg), fusable
-            self._states = [(f, copy.deepcopy(a)) for f, a in states]
+            self._states = states
         return self
+
+
+def _copied(state):
+    """A copy of a configuration state that later changes do not reach, or None."""
+    try:
+        return copy.deepcopy(state)
+    except Exception:  # option values that cannot be copied
+        return None
+
+
+def _same(a, b):
+    """Equal in value and type throughout (configure() tells 2 from np.int64(2)).  b is a copy:
+    where it is a itself, a cannot change."""
+    if a is b:
+        return True
+    if type(a) is not type(b):
+        return False
+    if isinstance(a, dict):
+        return len(a) == len(b) and all(k in b and _same(v, b[k]) for k, v in a.items())
+    if isinstance(a, (list, tuple)):
+        return len(a) == len(b) and all(map(_same, a, b))
+    try:
+        return bool(a == b)
+    except Exception:  # values that do not compare to a truth value
+        return False
 
 
 class NativeFunctional(AbstractFunctional):
@@ -214,8 +242,18 @@ class NativeFunctional(AbstractFunctional):
     def configure(self, cfg):  # fill this functional's part of the evaluator config
         raise NotImplementedError
 
-    def config_state(self):  # what configure() depends on, comparable with ==; None: not known
+    def config_state(self):
+        """What configure() depends on, for ``ConfigCache``; None: not known, so the functional
+        is configured on every call.  A built-in class answers with ``_plain_state``."""
         return None
+
+    def _plain_state(self, cls, *values):
+        """The methods that configure an object of exactly the class ``cls``, and ``values``;
+        None for a derived class, whose configure() may depend on anything."""
+        own = self.__dict__
+        if type(self) is not cls or "configure" in own or "engines" in own:
+            return None
+        return (cls.configure,) + values
 
     def prepare(self, ev, grid, dtype):  # bind per-grid data (v_loc, k_F state) before a compute
         pass

@@ -226,7 +226,7 @@ class KEDF(NativeFunctional):
         return KEDFEngines[(name or self.name).upper()]
 
     def config_state(self):
-        return self.name, self.options
+        return self._plain_state(KEDF, self.name, self.engines(), self.options)
 
     def configure(self, cfg, engines=None):
         o = self.options

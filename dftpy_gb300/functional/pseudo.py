@@ -242,7 +242,7 @@ class LocalPseudo(NativeFunctional):
         cfg.pseudo = 1
 
     def config_state(self):
-        return ()
+        return self._plain_state(LocalPseudo)
 
     def prepare(self, ev, grid, dtype):
         if grid is not self.grid and not (grid == self.grid):

@@ -37,7 +37,7 @@ class XC(NativeFunctional):
         cfg.xc_lda = 1
 
     def config_state(self):
-        return ()
+        return self._plain_state(XC)
 
     def compute(self, density, calcType={"E", "V"}, **kwargs):
         out = NativeFunctional.compute(self, density, calcType)
@@ -99,7 +99,7 @@ class Hartree(NativeFunctional):
         cfg.hartree = 1
 
     def config_state(self):
-        return ()
+        return self._plain_state(Hartree)
 
     @_ClassOrInstance
     def compute(self, density, calcType={"E", "V"}, **kwargs):
