@@ -198,19 +198,26 @@ class LocalPseudo(NativeFunctional):
         h = self._native.get(dtype)
         if h is None:
             lib = _lib.load()
-            keys = self.species_keys
-            gps = [np.ascontiguousarray(self.readpp.gp[k]) for k in keys]
-            vps = [np.ascontiguousarray(self.readpp.vp[k]) for k in keys]
+            made = self._settings()
+            _, pme, order, keys, gps, vps = made
             npts = (_lib.C.c_int * len(keys))(*[len(g) for g in gps])
             gpp = (_lib._PD * len(keys))(*[_lib.dptr(g) for g in gps])
             vpp = (_lib._PD * len(keys))(*[_lib.dptr(v) for v in vps])
             ptr = _lib.C.c_void_p()
-            _lib.check(lib.ofdft_pseudo_create(self.grid.native_for(dtype), len(keys), npts, gpp, vpp,
-                                               1 if self.PME else 0, int(self.BsplineOrder), _lib.C.byref(ptr)))
-            h = _PseudoHandle(lib, ptr, (gps, vps))
+            _lib.check(lib.ofdft_pseudo_create(self.grid.native_for(dtype), len(keys), npts, gpp, vpp, pme, order,
+                                               _lib.C.byref(ptr)))
+            h = _PseudoHandle(lib, ptr, made)
             self._set_ions(h)
             self._native[dtype] = h
         return h.ptr
+
+    def _settings(self):
+        """What a native handle is made from, besides the ions: copies, so that a later
+        change of an attribute or of a table's values shows."""
+        keys = self.species_keys
+        return (self.grid, 1 if self.PME else 0, int(self.BsplineOrder), keys,
+                [np.array(self.readpp.gp[k], dtype=np.float64) for k in keys],
+                [np.array(self.readpp.vp[k], dtype=np.float64) for k in keys])
 
     def _set_ions(self, h):
         ions, keys = self.ions, self.species_keys
@@ -301,17 +308,16 @@ class LocalPseudo(NativeFunctional):
         self._native, self._vreal = {}, {}
 
     def set_positions(self, positions):
-        """Move the ions (Bohr); drops cached v_loc and the Ewald object.  The native handles
-        stay, with their radial tables on the grid."""
+        """Move the ions (Bohr); drops cached v_loc and the Ewald object.  Native handles that
+        were made with the present settings (PME, BsplineOrder, grid, tables) stay, with their
+        radial tables on the grid."""
         self._ions.positions = np.array(positions, dtype=np.float64).reshape(self._ions.nat, 3)
-        self._vreal = {}
-        try:
-            for h in self._native.values():
+        self._vreal, self.ewald = {}, None
+        handles, self._native = self._native, {}
+        for dtype, h in handles.items():
+            if h.made_with(self._settings()):
                 self._set_ions(h)
-        except Exception:
-            self._native = {}
-            raise
-        self.ewald = None
+                self._native[dtype] = h
 
     def get_ewald(self, PME=None):
         if self.ewald is None:
@@ -323,8 +329,13 @@ class LocalPseudo(NativeFunctional):
 
 
 class _PseudoHandle:
-    def __init__(self, lib, ptr, keep):
-        self.lib, self.ptr, self.keep = lib, ptr, keep
+    def __init__(self, lib, ptr, made):
+        self.lib, self.ptr, self.made = lib, ptr, made
+
+    def made_with(self, now):
+        (grid, *a), (grid_now, *b) = self.made, now
+        same = lambda x, y: len(x) == len(y) and all(map(np.array_equal, x, y))
+        return grid is grid_now and a[:3] == b[:3] and same(a[3], b[3]) and same(a[4], b[4])
 
     def __del__(self):
         try:
