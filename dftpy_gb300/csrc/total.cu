@@ -857,7 +857,12 @@ struct ofdft_eval {
     double* mgp_c = nullptr;  // 4 per interval
     int mgp_n = 0;
     bool tab_set = false;  // the k_F-node kernel table is on the device
-    double* wtstate = nullptr;  // device [rho0, flag, tkf, factor, init]
+    // Device [rho0, flag, tkf, factor, init] of the kept Wang-Teter kernel: eight values of the
+    // general path, whose kernel is "wtK", and kFixState on those of fix_compute ("wtK_fix").  The
+    // two form |G|^2 and rho0 with other roundings, so neither takes the other's kernel: an
+    // optimisation gives the same bits with and without an evaluation before it.
+    static constexpr int kFixState = 8;
+    double* wtstate = nullptr;
     // density-dependent kernel
     void* tab_c = nullptr;
     void* tab_cd = nullptr;
@@ -1975,8 +1980,8 @@ void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, dou
     a.beta = lwt ? c.lwt_beta : c.wt_beta;
     a.wt_x = c.wt_x;
     a.wt_rho0 = c.wt_rho0;
-    a.wtstate = e->wtstate;
-    a.wtK = wt ? (double*)e->sc.get("wtK", (size_t)g->Nc * sizeof(double)) : nullptr;
+    a.wtstate = e->wtstate + ofdft_eval::kFixState;
+    a.wtK = wt ? (double*)e->sc.get("wtK_fix", (size_t)g->Nc * sizeof(double)) : nullptr;
     a.cTF_wt = e->k.cTF_wt;
     if (lwt && !e->fz_fork) OFDFT_CK(cudaEventCreateWithFlags(&e->fz_fork, cudaEventDisableTiming));
     fix::Fields f;
@@ -2403,8 +2408,8 @@ int ofdft_eval_create(ofdft_grid* g, const ofdft_config* cfg, ofdft_eval** out) 
         e->cfg = c;
         e->k = make_consts();
         try {
-            OFDFT_CK(cudaMalloc(&e->wtstate, 8 * sizeof(double)));
-            zero_now(e->wtstate, 8 * sizeof(double));
+            OFDFT_CK(cudaMalloc(&e->wtstate, 2 * ofdft_eval::kFixState * sizeof(double)));
+            zero_now(e->wtstate, 2 * ofdft_eval::kFixState * sizeof(double));
             if ((c.kedf_terms & OFDFT_KE_WT) && c.wt_kernel != OFDFT_LWT_KERNEL_WT) {
                 // MGPKernelTable (kernel.py:281-292): splrep of LindhardFunction(eta, 1, 1) on
                 // logspace(log10(1e-4), log10(52), 10000)
