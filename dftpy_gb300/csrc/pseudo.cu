@@ -379,13 +379,27 @@ struct ofdft_pseudo {
     double* d_scale = nullptr;    // per-atom gather scale
     bool have_vl = false;         // sc "vl<s>" holds the radial values on the half grid
     // recorded after the kernels that a call leaves running: moved ions wait for them on the
-    // host, other streams on the device
+    // host, other streams on the device.  A call under stream capture neither waits (an event
+    // from outside would end the capture) nor records; moved ions then wait for the whole
+    // device, as nothing here knows of a replay.
     cudaEvent_t busy = nullptr;
-    bool running = false;
+    bool running = false, captured = false;
+    static bool capturing(cudaStream_t st) {
+        cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {  // the default stream beside a capture
+            cudaGetLastError();
+            return false;
+        }
+        return s != cudaStreamCaptureStatusNone;
+    }
     void follow(cudaStream_t st) {
-        if (running) OFDFT_CK(cudaStreamWaitEvent(st, busy, 0));
+        if (running && !capturing(st)) OFDFT_CK(cudaStreamWaitEvent(st, busy, 0));
     }
     void mark(cudaStream_t st) {
+        if (capturing(st)) {
+            captured = true;
+            return;
+        }
         if (!busy) OFDFT_CK(cudaEventCreateWithFlags(&busy, cudaEventDisableTiming));
         OFDFT_CK(cudaEventRecord(busy, st));
         running = true;
@@ -520,7 +534,7 @@ void vloc_t(ofdft_pseudo* p, T* out, cudaStream_t st) {
             OFDFT_LAUNCH_CHECK();
             first = false;
         }
-        p->have_vl = true;
+        if (!p->capturing(st)) p->have_vl = true;  // captured: not there before a replay
     } else {
         k_pp_exact<T><<<gblk, 256, 0, st>>>(vG, p->lines(), p->d_pos, p->d_spec, p->nat, g->geo, scale);
         OFDFT_LAUNCH_CHECK();
@@ -784,7 +798,9 @@ int ofdft_pseudo_set_ions(ofdft_pseudo* p, int nat, const double* pos, const int
         for (int a = 0; a < nat; ++a)
             OFDFT_REQUIRE(species[a] >= 0 && species[a] < p->ns, "atom %d has species %d outside 0..%d", a,
                           species[a], p->ns - 1);
-        if (p->running) OFDFT_CK(cudaEventSynchronize(p->busy));  // they read the ions that move
+        // what runs reads the ions that move
+        if (p->captured) OFDFT_CK(cudaDeviceSynchronize());
+        else if (p->running) OFDFT_CK(cudaEventSynchronize(p->busy));
         p->running = false;
         p->nat = nat;
         p->pos.assign(pos, pos + 3 * (size_t)nat);
