@@ -226,7 +226,11 @@ class KEDF(NativeFunctional):
         return KEDFEngines[(name or self.name).upper()]
 
     def config_state(self):
-        return self._plain_state(KEDF, self.name, self.engines(), self.options)
+        own, o = self.__dict__, self.options
+        if type(self) is not KEDF or "configure" in own or "engines" in own:
+            return None
+        # with the options' types: configure() tells 2 from np.int64(2)
+        return KEDF.configure, self.name, self.engines(), o, tuple(map(type, o.values()))
 
     def configure(self, cfg, engines=None):
         o = self.options

@@ -249,7 +249,7 @@ class LocalPseudo(NativeFunctional):
         cfg.pseudo = 1
 
     def config_state(self):
-        return self._plain_state(LocalPseudo)
+        return LocalPseudo.configure if type(self) is LocalPseudo and "configure" not in self.__dict__ else None
 
     def prepare(self, ev, grid, dtype):
         if grid is not self.grid and not (grid == self.grid):

@@ -37,7 +37,7 @@ class XC(NativeFunctional):
         cfg.xc_lda = 1
 
     def config_state(self):
-        return self._plain_state(XC)
+        return XC.configure if type(self) is XC and "configure" not in self.__dict__ else None
 
     def compute(self, density, calcType={"E", "V"}, **kwargs):
         out = NativeFunctional.compute(self, density, calcType)
@@ -99,7 +99,7 @@ class Hartree(NativeFunctional):
         cfg.hartree = 1
 
     def config_state(self):
-        return self._plain_state(Hartree)
+        return Hartree.configure if type(self) is Hartree and "configure" not in self.__dict__ else None
 
     @_ClassOrInstance
     def compute(self, density, calcType={"E", "V"}, **kwargs):
