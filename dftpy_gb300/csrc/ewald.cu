@@ -145,15 +145,15 @@ __global__ void __launch_bounds__(RED_THREADS) k_ewald_real_sum(const double* __
     block_sum_store<7>(acc, partials);
 }
 
-// PME reciprocal energy and the force convolution input:
+// PME reciprocal energy and (conv) the force convolution's input, over QG in place:
 // E = 4 pi/V sum_mask |Q(G) B(G)|^2 exp(-G^2/4 eta)/G^2 (raw FFT, dV factors cancel);
 // X = Q(G) |B(G)|^2 exp(-G^2/4 eta)/G^2 / N.  The factors of the energy's terms go to
 // terms (zero outside the mask) and are summed by k_ewald_rec_sum, whose order of the
 // points does not depend on how this pass walks the rows.
 template <typename T>
 __global__ void __launch_bounds__(32 * kRowWarps)
-    k_ewald_rec_pme(const typename Cplx<T>::type* __restrict__ QG, typename Cplx<T>::type* X, const double* bre,
-                    const double* bim, Geo geo, double eta, double2* __restrict__ terms) {
+    k_ewald_rec_pme(typename Cplx<T>::type* __restrict__ QG, bool conv, const double* bre, const double* bim, Geo geo,
+                    double eta, double2* __restrict__ terms) {
     const int rows = geo.n0 * geo.n1;
     const double invN = 1.0 / (double)geo.N;
     for (int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kRowWarps) {
@@ -168,10 +168,10 @@ __global__ void __launch_bounds__(32 * kRowWarps)
             const double inv = (i == 0) ? 0.0 : 1.0 / gg;
             const double w = exp(-gg / (4.0 * eta)) * inv;
             terms[i] = half_mask(geo, i) ? make_double2(sr * sr + si * si, w) : make_double2(0.0, 0.0);
-            if (X) {
+            if (conv) {
                 const double f = (br * br + bi * bi) * w * invN;
-                X[i].x = (T)(qr * f);
-                X[i].y = (T)(qi * f);
+                QG[i].x = (T)(qr * f);
+                QG[i].y = (T)(qi * f);
             }
         }
     }
@@ -361,8 +361,13 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
         std::vector<int> fill(start.begin(), start.end() - 1);
         for (int a = 0; a < nat; ++a) order_atoms[fill[cellof[a]]++] = a;
     }
-    // Device buffers live in the grid's scratch; what the host prepares goes up in one copy
+    // Device buffers live in the grid's scratch; what the host prepares goes up in one copy.
+    // Meshes above kKeep bytes are the call's own and are freed with it, as large grids need the
+    // memory for node planes.  Allocating and freeing two of 135 MB (256^3; kept) takes 0.3 ms of
+    // a 6.5 ms ion step, two of 540 MB 1.0 ms.
+    constexpr size_t kKeep = (size_t)320 << 20;
     Scratch& sc = g->scratch;
+    Scratch own;
     const size_t n = (size_t)nat;
     double cinv[9];
     lattice_inverse(g->lattice, cinv);
@@ -415,18 +420,15 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
         double* bre = (double*)sc.get("ew_b", bm.size() * sizeof(double));
         double* bim = bre + nb;
         OFDFT_CK(cudaMemcpyAsync(bre, bm.data(), bm.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-        T* Q = (T*)sc.get("ew_Q", rb);
-        C* QG = (C*)sc.get("ew_QG", cb);
-        C* X = forces ? (C*)sc.get("ew_X", cb) : nullptr;
+        // two meshes: the charges, then the energy's terms, then the convolution; and their
+        // transform, which becomes the convolution's in place
+        const size_t mesh = std::max(rb, (size_t)g->Nc * sizeof(double2));
+        Scratch& big = mesh + cb > kKeep ? own : sc;
+        T* Q = (T*)big.get("ew_Q", mesh);
+        C* QG = (C*)big.get("ew_QG", cb);
+        double2* terms = reinterpret_cast<double2*>(Q);
         pme_spread<T>(sc, "ew_", nat, order, d_frac, nullptr, d_q, g->geo, Q, st);
         g->exec_r2c(Q, QG, 1, st);
-        double2* terms = (double2*)sc.get("ew_terms", (size_t)g->Nc * sizeof(double2));
-        k_ewald_rec_pme<T><<<row_grid(g->geo, g->sms), 32 * kRowWarps, 0, st>>>(QG, X, bre, bim, g->geo, eta, terms);
-        OFDFT_LAUNCH_CHECK();
-        k_ewald_rec_sum<<<g->red_blocks, RED_THREADS, 0, st>>>(terms, g->Nc, d_part);
-        OFDFT_LAUNCH_CHECK();
-        reduce_finalize<<<1, RED_THREADS, 0, st>>>(d_part, g->red_blocks, 1, 0ull, g->d_results + 7);
-        OFDFT_LAUNCH_CHECK();
         if (stress) {
             k_ewald_stress_rec<T><<<g->red_blocks, RED_THREADS, 0, st>>>(QG, nullptr, bre, bim, g->geo, eta,
                                                                          g->d_partials);
@@ -434,14 +436,21 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
             reduce_finalize<<<6, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 6, 0ull, g->d_results + 8);
             OFDFT_LAUNCH_CHECK();
         }
+        k_ewald_rec_pme<T><<<row_grid(g->geo, g->sms), 32 * kRowWarps, 0, st>>>(QG, forces != nullptr, bre, bim, g->geo,
+                                                                                eta, terms);
+        OFDFT_LAUNCH_CHECK();
+        k_ewald_rec_sum<<<g->red_blocks, RED_THREADS, 0, st>>>(terms, g->Nc, d_part);
+        OFDFT_LAUNCH_CHECK();
+        reduce_finalize<<<1, RED_THREADS, 0, st>>>(d_part, g->red_blocks, 1, 0ull, g->d_results + 7);
+        OFDFT_LAUNCH_CHECK();
         if (forces) {
-            T* conv = Q;  // the mesh charges are done with
+            T* conv = Q;  // charges and terms are done with
             if (sizeof(T) == 8 && fix::grid_plans(g)) {
-                double2* in = (double2*)X;
+                double2* in = (double2*)QG;
                 double* out = (double*)conv;
                 fix::c2r(g, &in, &out, 1, st);
             } else {
-                g->exec_c2r(X, conv, 1, st);
+                g->exec_c2r(QG, conv, 1, st);
             }
             k_pme_gather<T><<<nat, kGatherThreads, 0, st>>>(d_frac, nullptr, order, g->geo, conv, d_cinv, d_scale,
                                                             d_F + 3 * n);
@@ -455,7 +464,8 @@ void ewald_t(ofdft_grid* g, int nat, const double* pos, const double* charges, d
         for (int k = 0; k < 6; ++k) s_rec[k] = stress ? g->h_results[8 + k] : 0.0;
     } else {
         OFDFT_CK(cudaMemcpyAsync(Fall.data(), d_F, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, st));
-        double* S = (double*)sc.get("ew_S", (size_t)g->Nc * 2 * sizeof(double));
+        const size_t sb = (size_t)g->Nc * 2 * sizeof(double);
+        double* S = (double*)(sb > kKeep / 2 ? own : sc).get("ew_S", sb);
         k_ewald_rec_exact<T><<<g->red_blocks, RED_THREADS, 0, st>>>(d_pos, d_q, nat, g->geo, eta, S, g->d_partials);
         OFDFT_LAUNCH_CHECK();
         reduce_finalize<<<1, RED_THREADS, 0, st>>>(g->d_partials, g->red_blocks, 1, 0ull, g->d_results + 7);
