@@ -6,34 +6,21 @@
 #pragma once
 #include "common.cuh"
 
+#include <algorithm>
 #include <string>
 
 namespace ofdft {
 
 constexpr int kMaxOrder = 16;
 
-// out[n] = M_order(x + n - 1), n = 1..order; out[0] = 0 (ewald.py:63-82)
-__device__ inline void bspline_mn_dev(double x, int order, double* Mn) {
-    for (int i = 0; i <= order; ++i) Mn[i] = 0.0;
-    Mn[1] = x;
-    Mn[2] = 1.0 - x;
-    for (int i = 3; i <= order; ++i) {
-        for (int j = 0; j < i; ++j) {
-            int n = i - j;
-            Mn[n] = (x + n - 1) * Mn[n] + (j + 1 - x) * Mn[n - 1];
-            Mn[n] /= (double)(i - 1);
-        }
-    }
-}
-
 __device__ inline int pmod(long long a, int n) {
     long long r = a % n;
     return (int)(r < 0 ? r + n : r);
 }
 
-// B-spline values with one lane per n: lane n - 1 of a group of 16 holds M_i(x + n - 1)
-// after step i, the same recursion step by step (and the same roundings).  before: the
-// values of order - 1 (what the derivatives need).
+// B-spline values M_order(x + n - 1), n = 1..order (ewald.py:63-82), with one lane per n: lane
+// n - 1 of a group of 16 holds M_i(x + n - 1) after step i.  before: the values of order - 1
+// (what the derivatives need).
 __device__ __forceinline__ double bspline_mn_lane(double x, int order, int n, double& before) {
     double v = n == 1 ? x : (n == 2 ? 1.0 - x : 0.0);
     before = v;
@@ -58,10 +45,14 @@ __device__ __forceinline__ double bspline_mn_lane(double x, int order, int n, do
 // is the same bits on every run (a per-atom scatter with global atomics sums in arrival order).
 // The test costs tiles x atoms comparisons and bounds the kernel, hence the long tiles (2048
 // atoms on 256^3: 149 us; 8^3 tiles: 404 us); lists built and sorted on the host took 2.5 ms
-// there.
+// there.  From kPmeSlabAtoms atoms on, every slab of 8 points along axis 0 first gets the list of
+// the atoms that touch it (the same order), and its tiles test those.  v_loc without and with the
+// lists, ms: 108 atoms on 64^3 0.13 and 0.14; 4000 on 96^3 0.31 and 0.32, on 256^3 0.89 and 0.78;
+// 16384 on 128^3 0.89 and 0.85, on 512^3 10.1 and 5.3; 131072 on 1024^3 378 and 43.
 constexpr int kPmeTile = 8;
 constexpr int kPmeLong = 4;  // 8-point pieces of a tile along axis 2
 constexpr int kPmeThreads = kPmeTile * kPmeTile * kPmeTile;
+constexpr int kPmeSlabAtoms = 4096;
 
 // Stencil base and B-spline weights of every list position: 16 lanes per atom and axis
 static __global__ void k_pme_prep(const double* __restrict__ frac, const int* __restrict__ list, int nlist, int order,
@@ -84,12 +75,65 @@ static __global__ void k_pme_prep(const double* __restrict__ frac, const int* __
     }
 }
 
+// Whether the order points of an atom's stencil with base b along an axis of n points touch the
+// `wide` points from lo on; t = (1 + b - lo) mod n
+__device__ __forceinline__ bool pme_touches(int b, int lo, int n, int wide, int order, int& t) {
+    t = 1 + b - lo;  // base in [0, n): t in (-n, n]
+    t = t < 0 ? t + n : (t >= n ? t - n : t);
+    return t <= order + min(wide, n - lo) - 2;
+}
+
+// Ordered lists of the atoms that touch each slab of 8 points along axis 0, one block per slab:
+// counts, then (FILL) the lists one after another, with their starts.  An atom's points lie in
+// at most pme_slabs_of(order) slabs: a run of them, cut where it wraps around or meets the axis's
+// partial slab.
+inline int pme_slabs_of(int order) { return order / kPmeTile + 4; }
+template <bool FILL>
+static __global__ void __launch_bounds__(kPmeThreads)
+    k_pme_slabs(int nlist, int order, const int* __restrict__ base, int n0, int* __restrict__ counts,
+                int* __restrict__ starts, int* __restrict__ lists, long long room) {
+    __shared__ int part[kPmeThreads / 32];
+    __shared__ int from;
+    const int lo = blockIdx.x * kPmeTile, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) from = 0;
+    __syncthreads();
+    if (FILL) {
+        int before = 0;
+        for (int s = threadIdx.x; s < (int)blockIdx.x; s += kPmeThreads) before += counts[s];
+        if (before) atomicAdd(&from, before);
+        __syncthreads();
+        if (threadIdx.x == 0) starts[blockIdx.x] = from;
+    }
+    int found = FILL ? from : 0;
+    for (int q0 = 0; q0 < nlist; q0 += kPmeThreads) {
+        const int q = q0 + threadIdx.x;
+        int t;
+        const bool on = q < nlist && pme_touches(base[3 * q], lo, n0, kPmeTile, order, t);
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        __syncthreads();  // part is read
+        if (lane == 0) part[warp] = __popc(b);
+        __syncthreads();
+        int at = found;
+        for (int k = 0; k < kPmeThreads / 32; ++k) {
+            at += k < warp ? part[k] : 0;
+            found += part[k];
+        }
+        if (FILL && on) {
+            at += __popc(b & ((1u << lane) - 1u));
+            if (at < room) lists[at] = q;
+        }
+    }
+    if (!FILL && threadIdx.x == 0) counts[blockIdx.x] = found;
+}
+
 // Q at every point of a tile: sum over the atoms that touch it, in list order, of
-// w_a M0(i) M1(j) M2(k) with i = (1 + base_0 - l0) mod n0 (< order), etc.
+// w_a M0(i) M1(j) M2(k) with i = (1 + base_0 - l0) mod n0 (< order), etc.  counts, starts,
+// lists: of k_pme_slabs, or null
 template <typename T>
 __global__ void __launch_bounds__(kPmeThreads)
     k_pme_tiles(int nlist, int order, const int* __restrict__ base, const double* __restrict__ M,
-                const double* __restrict__ w, const int* __restrict__ list, Geo geo, T* Q) {
+                const double* __restrict__ w, const int* __restrict__ list, Geo geo, T* Q,
+                const int* __restrict__ counts, const int* __restrict__ starts, const int* __restrict__ lists) {
     __shared__ int hit[kPmeThreads];
     __shared__ int off[kPmeThreads][3];  // (1 + base - first point of the tile) mod n per axis
     __shared__ int count[kPmeThreads / 32];
@@ -102,18 +146,17 @@ __global__ void __launch_bounds__(kPmeThreads)
     const bool in = lo[0] + p[0] < nr[0] && lo[1] + p[1] < nr[1] && lo[2] + p[2] < nr[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o1 = order + 1;
     double v[kPmeLong] = {};
-    for (int q0 = 0; q0 < nlist; q0 += kPmeThreads) {
-        const int q = q0 + threadIdx.x;
+    const int slab = tid / (T1 * T2), atoms = lists ? counts[slab] : nlist;
+    const int* mine = lists ? lists + starts[slab] : nullptr;
+    for (int q0 = 0; q0 < atoms; q0 += kPmeThreads) {
+        int q = q0 + threadIdx.x;
         int o[3] = {0, 0, 0};
-        bool on = q < nlist;
+        bool on = q < atoms;
         if (on) {
+            if (mine) q = mine[q];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                int t = 1 + base[3 * q + d] - lo[d];  // base in [0, n): t in (-n, n]
-                t = t < 0 ? t + nr[d] : (t >= nr[d] ? t - nr[d] : t);
-                o[d] = t;
-                on = on && t <= order + min(d == 2 ? wide : kPmeTile, nr[d] - lo[d]) - 2;
-            }
+            for (int d = 0; d < 3; ++d)
+                on = pme_touches(base[3 * q + d], lo[d], nr[d], d == 2 ? wide : kPmeTile, order, o[d]) && on;
         }
         const unsigned b = __ballot_sync(0xffffffffu, on);
         __syncthreads();  // the previous chunk's list is done with
@@ -183,7 +226,19 @@ void pme_spread(Scratch& sc, const std::string& prefix, int nlist, int order, co
     OFDFT_LAUNCH_CHECK();
     auto tiles = [](int n) { return (n + kPmeTile - 1) / kPmeTile; };
     const unsigned nt = (unsigned)tiles(geo.n0) * tiles(geo.n1) * ((geo.n2 + kPmeTile * kPmeLong - 1) / (kPmeTile * kPmeLong));
-    k_pme_tiles<T><<<nt, kPmeThreads, 0, st>>>(nlist, order, base, M, d_w, d_list, geo, Q);
+    int *counts = nullptr, *starts = nullptr, *lists = nullptr;
+    if (nlist >= kPmeSlabAtoms) {
+        const int slabs = tiles(geo.n0);
+        const long long room = (long long)nlist * std::min(slabs, pme_slabs_of(order));
+        counts = (int*)sc.get(prefix + "slabs", 2 * (size_t)slabs * sizeof(int));
+        starts = counts + slabs;
+        lists = (int*)sc.get(prefix + "lists", (size_t)room * sizeof(int));
+        k_pme_slabs<false><<<slabs, kPmeThreads, 0, st>>>(nlist, order, base, geo.n0, counts, starts, lists, room);
+        OFDFT_LAUNCH_CHECK();
+        k_pme_slabs<true><<<slabs, kPmeThreads, 0, st>>>(nlist, order, base, geo.n0, counts, starts, lists, room);
+        OFDFT_LAUNCH_CHECK();
+    }
+    k_pme_tiles<T><<<nt, kPmeThreads, 0, st>>>(nlist, order, base, M, d_w, d_list, geo, Q, counts, starts, lists);
     OFDFT_LAUNCH_CHECK();
 }
 

@@ -31,3 +31,24 @@ def test_local_potential_and_ewald(nr):
     assert float(np.abs(out.potential.numpy() - ref["V"]).max()) <= V_ATOL
     ew, oew = pp.get_ewald(), O.Ewald(og, pos, np.full(len(pos), 3.0), PME=True)
     assert abs(ew.energy - oew.energy()) <= E_RTOL * max(len(pos), abs(oew.energy()))
+
+
+@pytest.mark.parametrize("nr", [(20, 12, 34), (17, 13, 16)])  # a partial slab of four points, of one
+def test_many_atoms(nr):
+    """From 4096 atoms on the tiles take their atoms from lists of the slabs along axis 0."""
+    lat = np.array([[8.0, 0.2, 0.0], [0.0, 9.0, 0.3], [0.5, 0.0, 10.0]])
+    pos = np.random.default_rng(7).uniform(0, 1, (4100, 3)) @ lat
+    gp, vp = syn.analytic_vloc(3.0, 1.0)
+    grid = D.DirectGrid(lat, nr)
+    ions = D.Ions(symbols=["Al"] * len(pos), positions=pos, cell=lat)
+    pp = D.LocalPseudo(grid=grid, ions=ions, PP_list={"Al": D.functional.RECPOT(r=gp, v=vp, zval=3)}, PME=True)
+    og = O.Grid(lat, nr)
+    rho_np = syn.smooth_density(lat, nr, 9.0, seed=5, amp=0.5, kmax=1)
+    ref = O.LocalPseudo(og, pos, np.zeros(len(pos), dtype=int), [(gp, vp)], PME=True)(rho_np, ("E", "V"))
+    out = pp(D.DirectField(grid, data=rho_np))
+    assert abs(out.energy - ref["E"]) <= E_RTOL * max(len(pos), abs(ref["E"]))
+    # a potential that grows with the atoms: the bar is relative to its range
+    assert float(np.abs(out.potential.numpy() - ref["V"]).max()) <= V_ATOL * max(1.0, float(np.abs(ref["V"]).max()))
+    again = pp.vreal.numpy().copy()
+    pp.set_positions(pos)
+    assert np.array_equal(pp.vreal.numpy(), again)
