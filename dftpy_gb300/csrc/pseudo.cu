@@ -199,8 +199,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_pp_force_exact(const typename C
 // the spline interval holding |G|; the host applies the spline adjoint.
 // The moments of the intervals are summed in shared memory, `copies` of them so that the
 // lanes of a warp rarely meet in one (range intervals can hold a |G|), and added to the
-// result once per block; range = 0: straight into the result, for tables too fine to fit.
-// 160^3 with 256 table points: 1.48 ms per species with every point's atomics in global memory.
+// result once per block; range = 0: straight into the result.
 template <typename T>
 __global__ void __launch_bounds__(32 * kRowWarps)
     k_pp_grad_moments(const typename Cplx<T>::type* __restrict__ rhoG, const typename Cplx<T>::type* __restrict__ QG,
@@ -676,18 +675,24 @@ void vloc_grad_t(ofdft_pseudo* p, const T* rho, double* grad, cudaStream_t st) {
                 k_strf_species<T><<<gblk, 256, 0, st>>>(SG, p->d_pos, p->d_sel + p->sel_off[s], n_s, g->geo);
                 OFDFT_LAUNCH_CHECK();
             }
-            // intervals a |G| can fall in; up to 16 copies of their moments in 160 KB
+            // Intervals a |G| can fall in; up to 16 copies of their moments in 160 KB.  Shared copies
+            // pay where many points meet in an interval; with few of them the blocks spend longer
+            // clearing and adding up their copies.  float64, us, global and shared: 252 intervals
+            // (16 copies) at 32^3 20 and 20, 64^3 102 and 53, 160^3 1387 and 285; 1014 (5) at 64^3 43
+            // and 57, 96^3 102 and 94, 160^3 418 and 293; 4062 (1) at 128^3 158 and 209, 256^3 940
+            // and 1148.
             const std::vector<double>& x = p->spl[s].x;
             int range = (int)(std::upper_bound(x.begin(), x.end(), 1.000001 * gmax) - x.begin());
             range = std::min(nint, std::max(1, range));
             const size_t one = (4 * (size_t)range + 3) * sizeof(double), most = 160 * 1024;
-            const int copies = (int)std::min<size_t>(16, most / one);
-            if (copies == 0) range = 0;
+            int copies = (int)std::min<size_t>(16, most / one);
+            if ((double)copies * (double)g->Nc < 2100.0 * range) copies = 0;
+            if (copies == 0) range = 0;  // together: without copies the kernel has no shared memory
             const size_t smem = copies * one;
             if (smem > 40 * 1024)
                 OFDFT_CK(cudaFuncSetAttribute(k_pp_grad_moments<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)most));
-            const int grid = std::min(row_grid(g->geo, g->sms), 2 * g->sms);
+            const int rows = row_grid(g->geo, g->sms), grid = copies ? std::min(rows, 2 * g->sms) : rows;
             k_pp_grad_moments<T><<<grid, 32 * kRowWarps, smem, st>>>(rhoG, SG, p->pme ? p->d_bre : nullptr,
                                                                      p->pme ? p->d_bim : nullptr, p->line(s), g->geo,
                                                                      scale, range, copies, mom, mom + 4 * (size_t)nint);
