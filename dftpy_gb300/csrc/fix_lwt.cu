@@ -236,8 +236,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_axis1(Lwt a) {
         });
 }
 
-// The row passes: a block has two rows (one complex line) and transforms them for the planes
-// that they need, as many at a time as the tile has lines.  One row pair per tile keeps the
+// The row passes: a block has two rows (one complex line) and transforms them for its part of
+// the planes that they need, as many at a time as the tile has lines.  One row pair per tile keeps the
 // list short (a warp with eight rows to a node transformed 1.5 times as much), and warps that
 // run the same passes together share the instruction cache (one-warp blocks: 60% of the stalls
 // were fetches).  In shared memory: the codes of the points and the planes' list (2 node + plane).
@@ -247,7 +247,7 @@ struct RowPair {
     short2* code;           // of point i in both rows
     unsigned short* list;
     unsigned char* both;    // rows that need the plane: 1, 2 or both
-    int c;
+    int from, to;           // the block's part of the list (blockIdx.y), whole tiles
 };
 __device__ __forceinline__ RowPair stage_rows(const Lwt& a, void* at, int* counter) {
     RowPair s;
@@ -283,7 +283,9 @@ __device__ __forceinline__ RowPair stage_rows(const Lwt& a, void* at, int* count
     for (int i = threadIdx.x; i < n; i += T)
         s.code[i] = make_short2(a.code[s.row0 * n + i], s.two == 2 ? a.code[(s.row0 + 1) * n + i] : (short)-2);
     __syncthreads();
-    s.c = *counter;
+    const int c = *counter, per = (((c + (1 << a.lb) - 1) >> a.lb) + gridDim.y - 1) / gridDim.y << a.lb;
+    s.from = min(c, (int)blockIdx.y * per);
+    s.to = min(c, s.from + per);
     return s;
 }
 inline size_t rows_smem(int n, int planes) { return (size_t)n * sizeof(short2) + (size_t)planes * 3 + 16; }
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_rows(Lwt a) {
     I2* b0 = reinterpret_cast<I2*>(fix_smem);
     I2* b1 = b0 + (p.np == 3 ? n * LP : 0);
     const RowPair s = stage_rows(a, b1 + n * LP, &count);
-    if (a.first) {  // ends that no plane writes
+    if (a.first && blockIdx.y == 0) {  // ends that no plane writes
         for (int e = threadIdx.x; e < s.two * n; e += T) {
             const int i = a.dn.div(e) ? e - n : e, cd = e < n ? s.code[i].x : s.code[i].y;
             if (cd >= 0) continue;
@@ -325,12 +327,12 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_rows(Lwt a) {
         }
     }
     double2* raw = reinterpret_cast<double2*>(b0);
-    for (int q0 = 0; q0 < s.c; q0 += L) {
+    for (int q0 = s.from; q0 < s.to; q0 += L) {
         __syncthreads();  // the buffer and the scales are free
         for (int e = threadIdx.x; e < L * h; e += T) {
             const int l = a.dh.div(e), k = e - l * h, q = q0 + l;
             double2 A = make_double2(0.0, 0.0), B = A;
-            if (q < s.c) {
+            if (q < s.to) {
                 const int it = s.list[q], on = s.both[q];  // a row that the node does not need holds no values
                 const double2* in = a.XY + (long long)((it & 1) * a.nb + (it >> 1)) * a.plane + s.row0 * h + k;
                 if (on & 1) A = __ldcs(in);
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_rows(Lwt a) {
         tile_fft_out(
             b0, b1, p, a.lb, sm, [&](int i, int l) { return raw[i * LP + l]; },
             [&](int i, int l, I2 v) {
-                if (q0 + l >= s.c) return;
+                if (q0 + l >= s.to) return;
                 const int it = s.list[q0 + l], j = a.j0 + (it >> 1), d = it & 1;
                 const short2 two = s.code[i];
                 for (int b = 0; b < 2; ++b) {
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_hats(Lwt a) {
     I2* b0 = reinterpret_cast<I2*>(fix_smem);
     I2* b1 = b0 + n * LP;
     const RowPair s = stage_rows(a, b1 + n * LP, &count);
-    for (int q0 = 0; q0 < s.c; q0 += L) {
+    for (int q0 = s.from; q0 < s.to; q0 += L) {
         auto hat = [&](int cd, int j, int d, long long o) {
             const int il = cd >> 1;
             const bool small = cd == -4 && j == 0 && d == 0, here = cd >= 0 && (il == j || il == j - 1);
@@ -401,7 +403,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_hats(Lwt a) {
         __syncthreads();  // the buffers and the scales are free
         const I2* z = tile_fft(b0, b1, p, a.lb, sm, [&](int i, int l) {
             double2 v = make_double2(0.0, 0.0);
-            if (q0 + l < s.c) {
+            if (q0 + l < s.to) {
                 const int it = s.list[q0 + l], j = a.j0 + (it >> 1), d = it & 1;
                 const short2 two = s.code[i];
                 v.x = hat(two.x, j, d, s.row0 * n + i);
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_hats(Lwt a) {
         });
         for (int e = threadIdx.x; e < L * h; e += T) {
             const int l = a.dh.div(e), k = e - l * h, q = q0 + l;
-            if (q >= s.c) break;
+            if (q >= s.to) break;
             const int it = s.list[q], on = s.both[q];
             const I2 Z = z[k * LP + l], Y = z[(k ? n - k : 0) * LP + l];
             double2* out = a.XY + (long long)((it & 1) * a.nb + (it >> 1)) * a.plane + s.row0 * h + k;
@@ -572,13 +574,24 @@ int lwt_enqueue(ofdft_grid* g, Scratch& sc, const LwtArgs& r, cudaStream_t st) {
     const Shape s0 = fit(p.p0, col_lines<0>(p), sms, (size_t)p.n0 * (sizeof(double2) + sizeof(double)));
     const int tiles0 = (int)col_blocks(col_lines<0>(p), s0.lb);
     const size_t smem0 = tile_smem(p.p0, s0.lb, 1) + (size_t)p.n0 * ((1 << s0.lb) + 1) * (sizeof(double2) + sizeof(double));
-    const int parts = shares(B, 8, tiles0, (long long)sms * resident(s0.threads, smem0));
+    const long long slots0 = (long long)sms * resident(s0.threads, smem0);
+    // k_fx_pot2's shares are partial spectra, so few; k_fx_nodes sums nothing, and splits further
+    // where eight shares leave the chip idle
+    const int parts = shares(B, 8, tiles0, slots0), nparts = 8 * tiles0 < slots0 ? shares(B, B, tiles0, slots0) : parts;
     const Shape s1 = shape_of(p.p1, col_lines<1>(p), sms);
     const size_t smem1 = tile_smem(p.p1, s1.lb, 1);
     const Shape s2 = shape_of(p.p2, 1LL << 40, sms);
     const size_t smemr = tile_smem(p.p2, s2.lb, 1) + rows_smem(p.n2, nc * B);
     const size_t smemh = tile_smem(p.p2, s2.lb, 2) + rows_smem(p.n2, std::max(nh, 1) * B);
     const unsigned b2 = (unsigned)(((long long)p.n0 * p.n1 + 1) / 2);
+    // Row pairs times parts of their planes' lists: as many parts as fill the chip once.  With a
+    // block per row pair a grid of few rows waited for lists of up to 128 planes: 64 nodes,
+    // Hermite, whole call: 16^3 789 us (568 in parts; general path 650), 4 x 4 x 512 2082 (456; 740),
+    // 32^3 792 (764; 1245), 64 x 72 x 80 in one part either way.
+    auto row_parts = [&](int planes, size_t smem) {
+        const long long slots = (long long)sms * resident(s2.threads, smem), tiles = (planes + (1 << s2.lb) - 1) >> s2.lb;
+        return (unsigned)std::max(1LL, std::min(tiles, slots / b2));
+    };
     double2* pot2 = hats ? (double2*)sc.get("fx_pot2", (size_t)parts * cb) : nullptr;
     smem_optin(k_fx_nodes, smem0);
     smem_optin(k_fx_pot2, smem0);
@@ -594,7 +607,7 @@ int lwt_enqueue(ofdft_grid* g, Scratch& sc, const LwtArgs& r, cudaStream_t st) {
         a.nm = nc;
         a.lb = s0.lb;
         a.lines = tiles0;
-        a.share = (a.nb + parts - 1) / parts;
+        a.share = (a.nb + nparts - 1) / nparts;
         k_fx_nodes<<<tiles0 * ((a.nb + a.share - 1) / a.share), s0.threads, smem0, st>>>(a);
         OFDFT_LAUNCH_CHECK();
         a.lb = s1.lb;
@@ -602,13 +615,13 @@ int lwt_enqueue(ofdft_grid* g, Scratch& sc, const LwtArgs& r, cudaStream_t st) {
         k_fx_axis1<true><<<dim3(b1, nc * a.nb), s1.threads, smem1, st>>>(a);
         OFDFT_LAUNCH_CHECK();
         a.lb = s2.lb;
-        k_fx_rows<<<b2, s2.threads, smemr, st>>>(a);
+        k_fx_rows<<<dim3(b2, row_parts(nc * a.nb, smemr)), s2.threads, smemr, st>>>(a);
         OFDFT_LAUNCH_CHECK();
         launches += 3;
         if (!hats) continue;
         a.XY = U;
         a.nm = nh;
-        k_fx_hats<<<b2, s2.threads, smemh, st>>>(a);
+        k_fx_hats<<<dim3(b2, row_parts(nh * a.nb, smemh)), s2.threads, smemh, st>>>(a);
         OFDFT_LAUNCH_CHECK();
         a.lb = s1.lb;
         k_fx_axis1<false><<<dim3(b1, nh * a.nb), s1.threads, smem1, st>>>(a);
