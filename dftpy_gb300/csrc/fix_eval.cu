@@ -224,8 +224,9 @@ __device__ __forceinline__ void turn(const I2* src, I2* dst, const Plan& p, int 
     }
 }
 
-// Axis 0 forward, the field's factor, axis 0 inverse.  |G|^2 = A f0^2 + B f0 + C along a
-// line (f0 the axis-0 frequency), so a point pays two operations for it.
+// Axis 0 forward, the field's factor, axis 0 inverse.  G = f0 b0 + c along a line (f0 the axis-0
+// frequency), |G|^2 the sum of its squares: six operations.  As a polynomial in f0, in two, it
+// lost up to 150 units in cells whose reciprocal vectors nearly cancel.
 __global__ void __launch_bounds__(kThreads, kBlocks) k_cols_mul(MulArgs a) {
     extern __shared__ __align__(16) unsigned char fix_smem[];
     __shared__ LineSm sm;
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_cols_mul(MulArgs a) {
     const int n = p.n, lb = a.c.lb, L = 1 << lb;
     I2* b0 = reinterpret_cast<I2*>(fix_smem);
     I2* b1 = b0 + (p.np == 3 ? n * (L + 1) : 0);
-    double2* fq = reinterpret_cast<double2*>(b1 + n * (L + 1));  // f0 and A f0^2
+    double* fq = reinterpret_cast<double*>(b1 + n * (L + 1));  // f0
     const int line = (blockIdx.x << lb) + (threadIdx.x & (L - 1));
     const bool in = line < col_lines<0>(a.c.g);
     const int k1 = line / a.c.g.n2h, k2 = line - k1 * a.c.g.n2h;
@@ -242,13 +243,12 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_cols_mul(MulArgs a) {
     const int kind = a.kind[blockIdx.y];
     const Geo& g = a.geo;
     const double f1 = (double)freq_index(k1, g.n1) * g.fv[1], f2 = (double)k2 * g.fv[2];
-    const double ax = g.b[0] * g.fv[0], ay = g.b[1] * g.fv[0], az = g.b[2] * g.fv[0];
     const double cx = f1 * g.b[3] + f2 * g.b[6], cy = f1 * g.b[4] + f2 * g.b[7], cz = f1 * g.b[5] + f2 * g.b[8];
-    const double A = ax * ax + ay * ay + az * az, B = 2.0 * (ax * cx + ay * cy + az * cz), C = cx * cx + cy * cy + cz * cz;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double f = (double)freq_index(i, n);
-        fq[i] = make_double2(f, A * f * f);
-    }
+    auto gsq_at = [&](int i) {
+        const double f = fq[i], gx = fma(f, g.b[0], cx), gy = fma(f, g.b[1], cy), gz = fma(f, g.b[2], cz);
+        return fma(gx, gx, fma(gy, gy, gz * gz));
+    };
+    for (int i = threadIdx.x; i < n; i += blockDim.x) fq[i] = (double)freq_index(i, n) * g.fv[0];
     const bool build = kind == F_WT && a.state[1] != 0.0;
     const double hart = 4.0 * M_PI * a.invN, half = 0.5 * a.invN;
     auto factor = [&](int i) -> double {
@@ -256,13 +256,11 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_cols_mul(MulArgs a) {
         if (kind == F_WT) {
             const long long at = line + i * stride;
             if (!build) return a.K[at] * a.invN;
-            const double2 t = fq[i];
-            const double K = wt_build(a, fma(t.x, B, t.y) + C);
+            const double K = wt_build(a, gsq_at(i));
             a.K[at] = K;
             return K * a.invN;
         }
-        const double2 t = fq[i];
-        const double gg = fma(t.x, B, t.y) + C;
+        const double gg = gsq_at(i);
         if (kind == F_VW) return gg * half;
         return i == 0 && line == 0 ? 0.0 : (ordinary(gg) ? recip(gg) : 1.0 / gg) * hart;
     };
@@ -565,7 +563,7 @@ int local_begin(ofdft_grid* g, Scratch& sc, const LocalArgs& a, Fields& f, cudaE
         m.state = a.wtstate;
         m.wt_x = a.wt_x;
         m.invN = 1.0 / (double)N;
-        const size_t smem = tile_smem(p.p0, s.lb, 1) + (size_t)p.n0 * sizeof(double2);
+        const size_t smem = tile_smem(p.p0, s.lb, 1) + (size_t)p.n0 * sizeof(double);
         smem_optin(k_cols_mul, smem);
         k_cols_mul<<<dim3(col_blocks(col_lines<0>(p), s.lb), back), s.threads, smem, st>>>(m);
         OFDFT_LAUNCH_CHECK();
