@@ -3,7 +3,7 @@
 //
 // The same quantities as the evaluator's general path (total.cu), arranged for a GPU
 // whose float64 pipe is the bound of everything:
-//   k_pre       every power of rho from one pair of roots and a square root
+//   k_pre       every power of rho from one sixth root
 //   rows, cols  the forward transforms of rho, sqrt(rho), rho^beta (rho^alpha) in
 //               one launch per axis
 //   k_cols_mul  axis 0 forward, 4 pi/G^2 | G^2/2 | K(G), axis 0 inverse in one launch
@@ -21,10 +21,14 @@ using namespace ofdft::fix;
 
 namespace {
 
-// The range where float32 seeds hold (also: not zero, negative or NaN).
-__device__ __forceinline__ bool ordinary(double x) { return x > 1e-30 && x < 1e30; }
+// The range where float32 seeds hold, 2^-99 to 2^99 (also: not zero, negative or NaN).  From the
+// high word: a float64 comparison takes a slot of the float64 pipe.
+__device__ __forceinline__ bool ordinary(double x) {
+    return (unsigned)(__double2hiint(x) - ((1023 - 99) << 20)) < (198u << 20);
+}
+__device__ __forceinline__ bool positive(double x) { return __double_as_longlong(x) > 0; }  // true for NaN, too
 
-// 1/x, 1e-30 < |x| < 1e30: a float32 seed y and one cubic Newton step
+// 1/x of an ordinary x: a float32 seed y and one cubic Newton step
 // y (1 + e + e^2), e = 1 - x y.  Two conversions and three float64 operations, where
 // the division takes about ten.
 __device__ __forceinline__ double recip(double x) {
@@ -33,20 +37,51 @@ __device__ __forceinline__ double recip(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
-// c = x^(1/3) and w = x^(-1/3): w from the float32 reciprocal cube root by one
-// Householder step (e = 1 - x w^3, w (1 + e/3 + 2 e^2/9)), c = x w^2 with one Newton
-// correction; 12 float64 operations for both, c within one unit in the last place.
-__device__ __forceinline__ void roots3(double x, double& c, double& w) {
+// The powers of a density that the pre-pass needs, every one within 0.51 units in the last place.
+// v = x^(-1/6) = v0 (1 + d) with a float32 seed v0, whose square is exact in float64: the power
+// x v0^k is taken as a sum of two float64 numbers, e = 1 - x v0^6 gives d by the binomial series
+// of (1 - e)^(-1/6) (|e| below 1e-6), and (1 + d)^k - 1 corrects the power before its only
+// rounding.  About 40 float64 operations for all of them; separate roots with products of them
+// took as many and were off by 2 to 8 units, as the factors' roundings add up.
+struct Roots {
+    double c, c2, w, v, sq;  // x^(1/3), x^(2/3), x^(-1/3), x^(-1/6), x^(1/2)
+    double r53;              // x^(5/3)
+    double p56;              // x to the float64 number nearest 5/6
+};
+__device__ __forceinline__ Roots roots_of(double x) {
+    Roots o;
     if (ordinary(x)) {
-        const double w0 = (double)rcbrtf((float)x);
-        const double e = fma(-(x * w0), w0 * w0, 1.0);
-        w = fma(w0 * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), w0);
-        const double u = w * w, c0 = x * u;
-        c = fma(fma(-(c0 * c0), c0, x) * u, 1.0 / 3.0, c0);
+        const float xf = (float)x;
+        const double v0 = (double)sqrtf(rcbrtf(xf)), a = v0 * v0;
+        const double y = x * a, yl = fma(x, a, -y);               // x v0^2
+        const double z = y * a, zl = fma(yl, a, fma(y, a, -z));   // x v0^4
+        const double s = y * v0, sl = fma(yl, v0, fma(y, v0, -s));  // x v0^3
+        const double p = x * v0, pl = fma(x, v0, -p);
+        const double e = fma(-zl, a, fma(-z, a, 1.0));
+        const double d = e * fma(e, 7.0 / 72.0, 1.0 / 6.0);
+        const double d2 = fma(d, d, d + d), d3 = fma(d2, d, d2 + d), d4 = fma(d2, d2, d2 + d2);
+        const double t = fma(y, d2, yl);
+        o.v = fma(v0, d, v0);
+        o.w = fma(a, d2, a);
+        o.c2 = y + t;
+        o.c = z + fma(z, d4, zl);
+        o.sq = s + fma(s, d3, sl);
+        const double h = x * y;
+        o.r53 = h + fma(x, t, fma(x, y, -h));
+        // the exponent is 3.7e-17 above 5/6
+        const double more = (double)(3.700743415417188e-17f * __logf(xf));
+        o.p56 = p + fma(p, d + more, pl);
     } else {
-        c = cbrt(x);
-        w = 1.0 / c;
+        o.c = cbrt(x);
+        if (o.c < 1e-30) o.c = 1e-30;  // for LDA (xc/semilocal_xc.py:283-319), which alone takes c, w and v
+        o.c2 = cbrt(x * x);
+        o.w = 1.0 / o.c;
+        o.v = sqrt(o.w);
+        o.sq = sqrt(x > 0.0 ? x : 1e-30);  // kedf/vw.py:34-44
+        o.r53 = x * o.c2;
+        o.p56 = 0.0;  // not used
     }
+    return o;
 }
 
 struct LdaRoots {
@@ -54,22 +89,19 @@ struct LdaRoots {
 };
 
 // Slater exchange + PZ81 correlation (xc/semilocal_xc.py:283-319) from the roots of r:
-// cb = r^(1/3), w = r^(-1/3), sq = sqrt(r); sqrt(Rs) = sqrt(rs) r^(1/2) r^(-2/3)
-__device__ __forceinline__ void lda_roots(double r, double cb, double w, double sq, const LdaRoots& k, double& ex,
-                                          double& vx) {
-    const double tiny = 1e-30;
+// sqrt(Rs) = sqrt(rs) r^(-1/6)
+__device__ __forceinline__ void lda_roots(const Roots& p, const LdaRoots& k, double& ex, double& vx) {
     const double a = 0.0311, b = -0.048, c = 0.0020, d = -0.0116, g = -0.1423, b1 = 1.0529, b2 = 0.3334;
-    const double rc = cb < tiny ? tiny : cb;
-    const double Rs = cb < tiny ? k.rs / tiny : k.rs * w;
-    if (Rs < 1.0) {
+    const double Rs = k.rs * p.w;
+    if (__double2hiint(Rs) < 0x3ff00000) {  // Rs < 1; NaN is not
         const double lr = log(Rs);
-        ex = k.ex * rc + (a * lr + b + c * Rs * lr + d * Rs);
-        vx = k.vx * rc + (lr * (a + (2.0 / 3) * c * Rs) + b - (1.0 / 3) * a + (1.0 / 3) * (2 * d - c) * Rs);
+        ex = k.ex * p.c + (a * lr + b + c * Rs * lr + d * Rs);
+        vx = k.vx * p.c + (lr * (a + (2.0 / 3) * c * Rs) + b - (1.0 / 3) * a + (1.0 / 3) * (2 * d - c) * Rs);
     } else {
-        const double sRs = ordinary(r) ? k.srs * (sq * (w * w)) : sqrt(Rs);
+        const double sRs = k.srs * p.v;
         const double inv = recip(1.0 + b1 * sRs + b2 * Rs);
-        ex = k.ex * rc + g * inv;
-        vx = k.vx * rc + (g + (7.0 / 6.0 * g * b1) * sRs + (4.0 / 3.0 * g * b2) * Rs) * (inv * inv);
+        ex = k.ex * p.c + g * inv;
+        vx = k.vx * p.c + (g + (7.0 / 6.0 * g * b1) * sRs + (4.0 / 3.0 * g * b2) * Rs) * (inv * inv);
     }
 }
 
@@ -89,14 +121,13 @@ struct PreK {
     double* kf;
     long long N;
     int tf, xc;
-    int b56, a53;  // beta = 5/6; alpha + beta = 5/3 to rounding
+    int b56;  // beta = 5/6
     double tf_x, alpha, beta, cE, cV, threepi2;
     LdaRoots lda;
 };
 
 // Pointwise pre-pass: bound by the float64 pipe (about 70 operations per point with
-// TF, LDA, PP and vW).  rho^(5/6) = rho^(1/2) rho^(1/3) and, when the exponents add up
-// to 5/3, rho^alpha = rho^(5/3) / rho^beta need no pow().
+// TF, LDA, PP, vW and rho^(5/6), which needs no pow()).
 // LWT: also k_F and its range (three more slots, after all blocks' sums), and LWT's clamp.
 template <bool LWT>
 __global__ void __launch_bounds__(RED_THREADS) k_pre(PreK a, double* partials) {
@@ -105,17 +136,16 @@ __global__ void __launch_bounds__(RED_THREADS) k_pre(PreK a, double* partials) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += stride) {
         const double r = a.rho[i];
-        double v = 0.0, cb, w;
+        double v = 0.0;
         s[3] += r;
-        roots3(r, cb, w);
-        const double c2 = cb * cb, sq = sqrt(r > 0.0 ? r : 1e-30);  // kedf/vw.py:34-44
+        const Roots p = roots_of(r);
         if (a.tf) {
-            s[0] += r * c2 * a.cE;
-            v = a.cV * c2 * a.tf_x;
+            s[0] += p.r53 * a.cE;
+            v = a.cV * p.c2 * a.tf_x;
         }
         if (a.xc) {
             double ex, vx;
-            lda_roots(r, cb, w, sq, a.lda, ex, vx);
+            lda_roots(p, a.lda, ex, vx);
             s[1] += ex * r;
             v += vx;
         }
@@ -124,14 +154,12 @@ __global__ void __launch_bounds__(RED_THREADS) k_pre(PreK a, double* partials) {
             s[2] += vl * r;
             v += vl;
         }
-        if (a.sq) a.sq[i] = sq;
+        if (a.sq) a.sq[i] = p.sq;
         if (a.rb) {
-            const bool ord = ordinary(r);
             // wt.py:15-18; lwt.py:206-221
             const double rc = LWT ? (r > 0.0 ? r : 1e-30) : (r < kZERO ? kZERO : r);
-            const double pb = a.b56 && ord ? sq * cb : pow(rc, a.beta);
-            a.rb[i] = pb;
-            if (a.ra) a.ra[i] = a.a53 && ord ? r * c2 / pb : pow(rc, a.alpha);
+            a.rb[i] = a.b56 && ordinary(r) ? p.p56 : pow(rc, a.beta);
+            if (a.ra) a.ra[i] = pow(rc, a.alpha);
         }
         if (LWT) {
             // lwt.py:106.  To the last bit as the general path has it: a point at a node's k_F is
@@ -342,9 +370,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_post(PostK a, double* partials)
         double v = a.V ? a.V[i] : 0.0;
         if (a.lap) {
             double q = a.sq[i];
-            if (fabs(q) < tiny) q = tiny;
+            if (!ord && fabs(q) < tiny) q = tiny;
             const double pw = a.lap[i] * (ord ? q * ri : 1.0 / q);
-            if (r > 0.0) s[0] += r * pw;
+            if (positive(r)) s[0] += r * pw;
             v += pw * a.vw_y;
         }
         if (a.vH) {
@@ -498,7 +526,6 @@ int local_begin(ofdft_grid* g, Scratch& sc, const LocalArgs& a, Fields& f, cudaE
     pk.tf = a.tf;
     pk.xc = a.xc;
     pk.b56 = a.beta == 5.0 / 6.0;
-    pk.a53 = std::fabs(a.alpha + a.beta - 5.0 / 3.0) < 4e-16;
     pk.tf_x = a.tf_x;
     pk.alpha = a.alpha;
     pk.beta = a.beta;
