@@ -491,20 +491,24 @@ def gpu_arm(args):
         k64 = min(5, max(2, args.steps // 3))
         t64 = run(torch.float64, k64, 1)
         ms64 = maxrank(t64["ms_total"]) / k64
-        # the general path (float64 library transforms), which profiling and the optimisers take
         r64 = run(torch.float64, k64, 1, profile=True)
-        ms64g = maxrank(r64["ms_total"]) / k64
         tot64 = sum(v["ms"] for v in r64["prof"].values())
+        # the general path (float64 library transforms), which the optimisers take
+        ke_g = D.Functional(type="KEDF", name="LWT", nsp=args.nsp, kdd=3, interp=args.interp, pipeline="cufft", **WGC)
+        g64 = run(torch.float64, k64, 1, profile=True,
+                  total=D.TotalFunctional(KineticEnergyFunctional=ke_g, XCFunctional=D.Functional(type="XC", name="LDA"),
+                                          HARTREE=D.Functional(type="HARTREE"), PSEUDO=pp))
+        ms64g = maxrank(g64["ms_total"]) / k64
         out["fp64"] = {"value": world * 1e3 / ms64, "unit": "evals/s", "ms_per_step": ms64, "steps": k64,
                        "energy": t64["E"], "general_path_ms_per_step": ms64g,
-                       "kernels_note": "of the general path",
+                       "kernels_note": "of a profiled run of the same evaluation",
                        "kernels": {k: {"share": v["ms"] / tot64 if tot64 else 0.0, "ms_per_step": v["ms"] / k64}
                                    for k, v in r64["prof"].items() if v["launches"] > 0}}
         # the general path is bound by GB300's float64 rate, not by HBM: the transforms'
         # flops (2.5 n log2 n per real transform of n points, the usual count)
         # over the cuFFT time, against a cuBLAS DGEMM measured here
         nfft = 198 if args.nsp == 64 else None  # 64 P + 64 M C2R, 64 hat R2C, 6 local transforms
-        cu = r64["prof"].get("cufft")
+        cu = g64["prof"].get("cufft")
         if nfft and cu and cu["ms"] > 0:
             peak64 = fp64_peak()
             fl = nfft * 2.5 * n3 * np.log2(n3)

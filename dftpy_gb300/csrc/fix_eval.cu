@@ -533,17 +533,21 @@ int local_begin(ofdft_grid* g, Scratch& sc, const LocalArgs& a, Fields& f, cudaE
     pk.cV = k.cTF_V;
     pk.threepi2 = k.threepi2;
     pk.lda = LdaRoots{k.lda_rs, std::sqrt(k.lda_rs), k.lda_ex, k.lda_vx};
-    if (a.lwt) k_pre<true><<<blocks, RED_THREADS, 0, st>>>(pk, part);
-    else k_pre<false><<<blocks, RED_THREADS, 0, st>>>(pk, part);
-    OFDFT_LAUNCH_CHECK();
-    k_sums<<<1, 128, 0, st>>>(part, blocks, 4, g->d_results, a.wt, a.wtstate, a.wt_rho0, 1.0 / (double)N, a.alpha,
-                              a.beta, a.cTF_wt);
-    OFDFT_LAUNCH_CHECK();
+    const double real = (double)rb, cplx = (double)cb;
+    a.time(PRE, real * (1 + (a.vloc != nullptr) + (a.V != nullptr) + a.vw + nl + (f.ra != nullptr) + a.lwt), st, [&] {
+        if (a.lwt) k_pre<true><<<blocks, RED_THREADS, 0, st>>>(pk, part);
+        else k_pre<false><<<blocks, RED_THREADS, 0, st>>>(pk, part);
+    });
+    a.time(SUMS, blocks * 4.0 * sizeof(double), st, [&] {
+        k_sums<<<1, 128, 0, st>>>(part, blocks, 4, g->d_results, a.wt, a.wtstate, a.wt_rho0, 1.0 / (double)N, a.alpha,
+                                  a.beta, a.cTF_wt);
+    });
     int launches = 2;
     if (a.lwt) {
-        reduce_finalize<<<3, RED_THREADS, 0, st>>>(part + 4 * (size_t)blocks, blocks, 3, 1ull | (2ull << 2) | (2ull << 4),
-                                                   g->d_results + 4);
-        OFDFT_LAUNCH_CHECK();
+        a.time(SUMS, blocks * 3.0 * sizeof(double), st, [&] {
+            reduce_finalize<<<3, RED_THREADS, 0, st>>>(part + 4 * (size_t)blocks, blocks, 3,
+                                                       1ull | (2ull << 2) | (2ull << 4), g->d_results + 4);
+        });
         OFDFT_CK(cudaMemcpyAsync(g->h_results, g->d_results, 7 * sizeof(double), cudaMemcpyDeviceToHost, st));
         OFDFT_CK(cudaEventRecord(copied, st));
         ++launches;
@@ -572,12 +576,12 @@ int local_begin(ofdft_grid* g, Scratch& sc, const LocalArgs& a, Fields& f, cudaE
         f.rbG = sp[nf++] = (double2*)sc.get("rbG", cb);
     }
     if (nf > 0) {
-        rows_r2c(p, sms, in, sp, nf, st);
-        cols<1>(p, sms, sp, nf, false, st);
+        a.time(FFT, nf * (real + cplx), st, [&] { rows_r2c(p, sms, in, sp, nf, st); });
+        a.time(FFT, nf * 2 * cplx, st, [&] { cols<1>(p, sms, sp, nf, false, st); });
         launches += 2;
     }
     if (a.lwt) {
-        cols<0>(p, sms, &f.rbG, 1, false, st);
+        a.time(FFT, 2 * cplx, st, [&] { cols<0>(p, sms, &f.rbG, 1, false, st); });
         ++launches;
     }
     if (back > 0) {
@@ -592,10 +596,11 @@ int local_begin(ofdft_grid* g, Scratch& sc, const LocalArgs& a, Fields& f, cudaE
         m.invN = 1.0 / (double)N;
         const size_t smem = tile_smem(p.p0, s.lb, 1) + (size_t)p.n0 * sizeof(double);
         smem_optin(k_cols_mul, smem);
-        k_cols_mul<<<dim3(col_blocks(col_lines<0>(p), s.lb), back), s.threads, smem, st>>>(m);
-        OFDFT_LAUNCH_CHECK();
-        cols<1>(p, sms, sp, back, true, st);
-        rows_c2r(p, sms, sp, out, back, st);
+        a.time(FFT, (back * 2 + (a.wt ? 0.5 : 0.0)) * cplx, st, [&] {
+            k_cols_mul<<<dim3(col_blocks(col_lines<0>(p), s.lb), back), s.threads, smem, st>>>(m);
+        });
+        a.time(FFT, back * 2 * cplx, st, [&] { cols<1>(p, sms, sp, back, true, st); });
+        a.time(FFT, back * (real + cplx), st, [&] { rows_c2r(p, sms, sp, out, back, st); });
         launches += 3;
     }
     return launches;
@@ -625,10 +630,16 @@ int local_finish(ofdft_grid* g, Scratch& sc, const LocalArgs& a, const Fields& f
     q.rhomax = w.rhomax;
     q.ld = w.ld;
     q.kfclip = w.kfclip;
-    k_post<<<blocks, RED_THREADS, 0, st>>>(q, part);
-    OFDFT_LAUNCH_CHECK();
-    k_sums<<<1, 128, 0, st>>>(part, blocks, 3, g->d_results + 16, 0, nullptr, 0.0, 0.0, 0.0, 0.0, 0.0);
-    OFDFT_LAUNCH_CHECK();
+    int fields = 1;  // read, and V written
+    for (const void* x : {(const void*)f.sq, (const void*)f.lap, (const void*)f.vH, (const void*)f.nl1, (const void*)f.nl2,
+                          (const void*)f.rb, (const void*)f.ra, (const void*)f.kf, (const void*)w.pot2})
+        fields += x != nullptr;
+    for (int i = 0; i < 4; ++i) fields += (w.pot1[i] != nullptr) + (w.pot3[i] != nullptr);
+    fields += a.V ? 2 : 0;
+    a.time(POST, (double)g->real_bytes() * fields, st, [&] { k_post<<<blocks, RED_THREADS, 0, st>>>(q, part); });
+    a.time(SUMS, blocks * 3.0 * sizeof(double), st, [&] {
+        k_sums<<<1, 128, 0, st>>>(part, blocks, 3, g->d_results + 16, 0, nullptr, 0.0, 0.0, 0.0, 0.0, 0.0);
+    });
     return 2;
 }
 

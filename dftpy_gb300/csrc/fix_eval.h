@@ -17,7 +17,24 @@ void free_plans(ofdft_grid* g);
 void r2c(ofdft_grid* g, const double* const* in, double2* const* out, int nf, cudaStream_t st);
 void c2r(ofdft_grid* g, double2* const* in, double* const* out, int nf, cudaStream_t st);
 
+// Kernel classes of these evaluations, and who times them (ofdft_eval_profile; owner null: nobody):
+// a launch, or a few of one class, between begin and end, with the bytes that it has to move
+enum Part { PRE, POST, SUMS, FFT, NODES, AXIS1, INTERP, HATS, POT2 };
+struct Timing {
+    void* owner = nullptr;
+    int (*begin)(void* owner, Part part, double bytes, cudaStream_t st) = nullptr;
+    void (*end)(void* owner, int at, cudaStream_t st) = nullptr;
+    template <class F>
+    void operator()(Part part, double bytes, cudaStream_t st, F&& f) const {
+        const int at = owner ? begin(owner, part, bytes, st) : -1;
+        f();
+        OFDFT_LAUNCH_CHECK();
+        if (owner) end(owner, at, st);
+    }
+};
+
 struct LocalArgs {
+    Timing time;
     const double* rho;
     const double* vloc;  // or null
     double* V;           // or null: energies only
@@ -32,6 +49,7 @@ struct LocalArgs {
 
 // The density-dependent kernel between the two halves of an evaluation (fix_lwt.cu)
 struct LwtArgs {
+    Timing time;
     const double* kf;
     const double* rA;
     const double2* rbG;  // FFT(rho^beta)

@@ -18,6 +18,7 @@
 #include "fix_3d.cuh"
 
 #include <algorithm>
+#include <vector>
 
 using namespace ofdft;
 using namespace ofdft::fix;
@@ -553,13 +554,24 @@ int lwt_enqueue(ofdft_grid* g, Scratch& sc, const LwtArgs& r, cudaStream_t st) {
     a.need = need;
     a.code = code;
     a.t = t;
+    double share = 1.0;  // of the rows that are needed: for the byte counts of a timed run
     {
         const size_t smem = (size_t)r.m * (2 * sizeof(double) + sizeof(unsigned));
         smem_optin(k_fx_need, smem);
-        k_fx_need<<<p.n0 * a.words, std::min(32, p.n1) * 32, smem, st>>>(a, need, code, t);
-        OFDFT_LAUNCH_CHECK();
+        r.time(INTERP, (double)g->N * (2 * sizeof(double) + sizeof(short)), st, [&] {
+            k_fx_need<<<p.n0 * a.words, std::min(32, p.n1) * 32, smem, st>>>(a, need, code, t);
+        });
         ++launches;
+        if (r.time.owner) {
+            std::vector<unsigned> bits((size_t)p.n0 * r.m * a.words);
+            OFDFT_CK(cudaMemcpyAsync(bits.data(), need, bits.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+            OFDFT_CK(cudaStreamSynchronize(st));
+            long long on = 0;
+            for (unsigned b : bits) on += __builtin_popcount(b);
+            share = (double)on / ((double)p.n0 * p.n1 * r.m);
+        }
     }
+    const double cplx = (double)cb, real = (double)g->real_bytes();
     const bool mc = r.kdd == 3 || r.hermite, hats = r.kdd > 1;
     const int nc = mc ? 2 : 1, nh = hats ? (r.hermite ? 2 : 1) : 0;
     size_t freeb = 0, totalb = 0;
@@ -608,42 +620,49 @@ int lwt_enqueue(ofdft_grid* g, Scratch& sc, const LwtArgs& r, cudaStream_t st) {
         a.lb = s0.lb;
         a.lines = tiles0;
         a.share = (a.nb + nparts - 1) / nparts;
-        k_fx_nodes<<<tiles0 * ((a.nb + a.share - 1) / a.share), s0.threads, smem0, st>>>(a);
-        OFDFT_LAUNCH_CHECK();
+        r.time(NODES, cplx * (1 + nc * a.nb), st, [&] {
+            k_fx_nodes<<<tiles0 * ((a.nb + a.share - 1) / a.share), s0.threads, smem0, st>>>(a);
+        });
         a.lb = s1.lb;
         const unsigned b1 = col_blocks(col_lines<1>(p), s1.lb);
-        k_fx_axis1<true><<<dim3(b1, nc * a.nb), s1.threads, smem1, st>>>(a);
-        OFDFT_LAUNCH_CHECK();
+        r.time(AXIS1, cplx * nc * a.nb * (1 + share), st, [&] {
+            k_fx_axis1<true><<<dim3(b1, nc * a.nb), s1.threads, smem1, st>>>(a);
+        });
         a.lb = s2.lb;
-        k_fx_rows<<<dim3(b2, row_parts(nc * a.nb, smemr)), s2.threads, smemr, st>>>(a);
-        OFDFT_LAUNCH_CHECK();
+        r.time(INTERP, cplx * nc * a.nb * share + real * 2, st, [&] {
+            k_fx_rows<<<dim3(b2, row_parts(nc * a.nb, smemr)), s2.threads, smemr, st>>>(a);
+        });
         launches += 3;
         if (!hats) continue;
         a.XY = U;
         a.nm = nh;
-        k_fx_hats<<<dim3(b2, row_parts(nh * a.nb, smemh)), s2.threads, smemh, st>>>(a);
-        OFDFT_LAUNCH_CHECK();
+        r.time(HATS, cplx * nh * a.nb * share + real * 2, st, [&] {
+            k_fx_hats<<<dim3(b2, row_parts(nh * a.nb, smemh)), s2.threads, smemh, st>>>(a);
+        });
         a.lb = s1.lb;
-        k_fx_axis1<false><<<dim3(b1, nh * a.nb), s1.threads, smem1, st>>>(a);
-        OFDFT_LAUNCH_CHECK();
+        r.time(AXIS1, cplx * nh * a.nb * (1 + share), st, [&] {
+            k_fx_axis1<false><<<dim3(b1, nh * a.nb), s1.threads, smem1, st>>>(a);
+        });
         a.lb = s0.lb;
         a.pot2G = pot2;
         a.share = (a.nb + parts - 1) / parts;
         const int used = (a.nb + a.share - 1) / a.share;
         if (a.first && used < parts)  // a later, fuller batch may use more partial spectra
             OFDFT_CK(cudaMemsetAsync(pot2 + (size_t)used * g->Nc, 0, (size_t)(parts - used) * cb, st));
-        k_fx_pot2<<<tiles0 * used, s0.threads, smem0, st>>>(a);
-        OFDFT_LAUNCH_CHECK();
+        r.time(POT2, cplx * (nh * a.nb + used), st, [&] {
+            k_fx_pot2<<<tiles0 * used, s0.threads, smem0, st>>>(a);
+        });
         launches += 3;
     }
     if (hats) {
         if (parts > 1) {
-            k_fx_join<<<blocks_for(g->Nc, 256, sms * 8), 256, 0, st>>>(pot2, g->Nc, parts);
-            OFDFT_LAUNCH_CHECK();
+            r.time(POT2, cplx * (parts + 1), st, [&] {
+                k_fx_join<<<blocks_for(g->Nc, 256, sms * 8), 256, 0, st>>>(pot2, g->Nc, parts);
+            });
             ++launches;
         }
         double* out = r.pot2;
-        c2r(g, &pot2, &out, 1, st);
+        r.time(FFT, 5 * cplx + real, st, [&] { c2r(g, &pot2, &out, 1, st); });
         launches += 3;
     }
     return launches;

@@ -886,7 +886,7 @@ struct ofdft_eval {
     double kf_st_min = 0, kf_st_max = 0;
     int last_nsp = 0, last_launches = 0;
     // per-kernel-class CUDA-event profiling
-    static constexpr int kClasses = 10;
+    static constexpr int kClasses = 11;
     bool prof = false;
     std::vector<cudaEvent_t> evs;   // pool, two per recorded launch
     std::vector<int> rec_cls;       // class of each recorded launch
@@ -937,10 +937,12 @@ enum ProfClass {
     P_REDUCE,
     P_CUFFT,
     P_FZ_AXIS1,
-    P_FZ_HAT
+    P_FZ_HAT,
+    P_FIX_FFT
 };
 const char* kProfNames[ofdft_eval::kClasses] = {"prepass", "gspace",   "lwt_nodes", "lwt_interp", "lwt_pot2",
-                                                 "postpass", "reduce", "cufft",     "fz_axis1",   "fz_hat"};
+                                                 "postpass", "reduce", "cufft",     "fz_axis1",   "fz_hat",
+                                                 "fix_fft"};
 
 // Record a start event for one launch of class cls moving `bytes` algorithmic bytes.
 int prof_begin(ofdft_eval* e, int cls, double bytes, cudaStream_t st) {
@@ -1930,13 +1932,13 @@ void collect_energies(ofdft_eval* e, double* energies) {
 // Whether ofdft_eval_compute takes the float64 evaluation on integer-pipe transforms
 // (fix_eval.cu, fix_lwt.cu): TF, vW, LDA, Hartree, PP, the Wang-Teter kernel and the
 // density-dependent kernel without smoothing or corrections, on axes the plans cover.  It is
-// 2 to 8 times faster than the general path, whose float64 transforms and powers saturate
-// the slow float64 pipe.  An explicit CUFFT pipeline and per-kernel profiling stay with the
-// general path.
+// 2.7 to 3.1 times faster than the general path (32^3 with TFvW, 128^3 with WT, 64 x 72 x 80 with
+// 64 nodes), whose float64 transforms and powers saturate the slow float64 pipe.  An explicit
+// CUFFT pipeline stays with the general path.
 bool fix_applies(ofdft_eval* e) {
     const ofdft_config& c = e->cfg;
     const int known = OFDFT_KE_TF | OFDFT_KE_VW | OFDFT_KE_WT | OFDFT_KE_LWT;
-    if (e->g->prec != OFDFT_F64 || (c.kedf_terms & ~known) || c.vw_sigma > 0.0 || c.wte || c.external || e->prof)
+    if (e->g->prec != OFDFT_F64 || (c.kedf_terms & ~known) || c.vw_sigma > 0.0 || c.wte || c.external)
         return false;
     if ((c.kedf_terms & OFDFT_KE_WT) && c.wt_kernel != OFDFT_LWT_KERNEL_WT) return false;
     if ((c.kedf_terms & OFDFT_KE_LWT) &&
@@ -1956,6 +1958,14 @@ const double* table_knots(ofdft_eval* e) {
     return e->tab_x;
 }
 
+// per-class times of these evaluations, in the general path's classes where the work is the same
+int fix_time_begin(void* owner, fix::Part part, double bytes, cudaStream_t st) {
+    static const int cls[] = {P_PREPASS, P_POSTPASS, P_REDUCE, P_FIX_FFT, P_LWT_NODES, P_FZ_AXIS1, P_LWT_INTERP, P_FZ_HAT,
+                              P_LWT_POT2};
+    return prof_begin(static_cast<ofdft_eval*>(owner), cls[part], bytes, st);
+}
+void fix_time_end(void* owner, int at, cudaStream_t st) { prof_end(static_cast<ofdft_eval*>(owner), at, st); }
+
 void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, double* energies, cudaStream_t st) {
     ofdft_grid* g = e->g;
     const ofdft_config& c = e->cfg;
@@ -1965,6 +1975,7 @@ void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, dou
     OFDFT_REQUIRE(!(c.pseudo && !e->have_vloc), "ofdft_eval_compute: pseudo enabled but no v_loc set");
     OFDFT_REQUIRE(!(wantV && !V), "ofdft_eval_compute: V requested but v_out is NULL");
     fix::LocalArgs a{};
+    if (e->prof) a.time = fix::Timing{e, fix_time_begin, fix_time_end};
     a.rho = rho;
     a.vloc = c.pseudo ? (const double*)e->vloc : nullptr;
     a.V = wantV ? V : nullptr;
@@ -1995,6 +2006,7 @@ void fix_compute(ofdft_eval* e, const double* rho, double* V, unsigned calc, dou
         if (active) {
             const size_t rb = g->real_bytes();
             fix::LwtArgs r{};
+            r.time = a.time;
             r.kdd = wantV ? c.lwt_kdd : 1;
             r.kf = f.kf;
             r.rA = f.ra ? f.ra : f.rb;
