@@ -76,13 +76,11 @@ __device__ __forceinline__ void agree(const double2 (&v)[R], I2 (&u)[R], bool on
         atomicAdd(&sm.sum[l], s);
     }
     __syncthreads();
-    Scale c;
-    c.emax = em;
-    c.sh = 32 - __clz((int)(sm.most[l] | 1u));
+    const Scale c = scale_of(em, sm.most[l]);
     const int k = fix_shift(c);
     if (j == 0) {
         sm.k[l] = k;
-        sm.ds[l] = np > 1 ? (32 - __clz((int)(sm.sum[l] | 1u))) - c.sh : 0;
+        sm.ds[l] = later_shift(c, sm.sum[l], np);
     }
 #pragma unroll
     for (int q = 0; q < R; ++q) u[q] = I2{to_fix(v[q].x, k), to_fix(v[q].y, k)};

@@ -443,7 +443,7 @@ const Grid3* grid_plans(ofdft_grid* g) {
         bool ok = true;
         size_t total = 0;
         for (int d = 0; d < 3; ++d) {
-            ok = ok && g->nr[d] <= kMaxAxis && plan_radices(g->nr[d], *p[d]);
+            ok = ok && plan_radices(g->nr[d], *p[d]);
             total += (size_t)g->nr[d];
         }
         if (ok) {

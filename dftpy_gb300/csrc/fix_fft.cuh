@@ -8,12 +8,14 @@
 //
 // Precision.  With R the first pass's radix, the scale maps the largest 1-norm
 // sum |re| + |im| of the subsets that the first pass transforms (every (n/R)-th
-// element; a bound taken from every element's exponent) to at most 2^61,
-// and the later passes' sums, up to the line's whole 1-norm, to at most 2^61 as well.  Every
+// element) to at most 2^61, and the later passes' sums, up to the line's whole 1-norm,
+// to at most 2^61 as well.  The norms are bounds from the elements' exponents; elements 22
+// binades or more below the line's largest count as nothing, which leaves out less than
+// 2^-12 of the norm and is covered by the room up to 2^62 that the products have.  Every
 // intermediate of an FFT is a sum of the inputs with weights of modulus one, so none
 // exceeds these bounds: nothing overflows, and no bits are given up that the line's
-// own values do not need.  For flat lines of up to 1024 elements the unit is 2^-56 of
-// the mean element in the first pass and 2^-51 of the mean element, 2^-56 of the mean
+// own values do not need.  For flat lines of up to 512 elements the unit is 2^-56 of
+// the mean element in the first pass and 2^-52 of the mean element, 2^-56 of the mean
 // output, after it; for a line with one dominant element it is 2^-61 of that.  That
 // is below the rounding of a float64 FFT, whose every addition rounds to 2^-53 of the
 // partial sum.  Twiddles carry 61 bits; elements are rounded to float64 once, on return.
@@ -230,7 +232,7 @@ struct Dft<16> {
 template <int A, int B>
 struct DftPfa {
     static constexpr int R = A * B;
-    static constexpr int out(int p, int q) {
+    FIX_HD static constexpr int out(int p, int q) {
         int k = 0;
         while (k % A != p || k % B != q) ++k;
         return k;
@@ -304,6 +306,17 @@ constexpr int kNonFinite = 0x7ff;
 struct Scale {
     int emax, sh;
 };
+FIX_HD int bit_length(unsigned v) {  // 1 for 0
+#ifdef __CUDA_ARCH__
+    return 32 - __clz((int)(v | 1u));
+#else
+    return 32 - __builtin_clz(v | 1u);
+#endif
+}
+// from the largest first-pass subset's bound, and the shift that the whole line's bound asks
+// for after that pass
+FIX_HD Scale scale_of(int emax, unsigned most) { return Scale{emax, bit_length(most)}; }
+FIX_HD int later_shift(Scale s, unsigned sum, int np) { return np > 1 ? bit_length(sum) - s.sh : 0; }
 // The shift in front of pass q >= 1 when the whole line needs ds: what the pass can grow
 // by (ceil log2 of its radix), or what is left
 FIX_HD int pass_shift(int ds, int q, int np, int r1) {
@@ -347,10 +360,9 @@ FIX_HD double to_dbl(long long v, int k, bool nan) {
 
 // ---- plans: radices of a length, largest first where twiddles are fewest
 constexpr int kMaxPass = 3;
-constexpr int kMaxLen = 1024;
-// Axes the three-dimensional transforms take: a tile of at least two lines of two
-// exchange buffers fits in shared memory.
-constexpr int kMaxAxis = 512;
+// The longest line: its two bounds per element are added up in 32 bits.
+constexpr int kMaxLen = 512;
+static_assert(2ULL * kMaxLen * 0x200000u < 1ULL << 32, "the 1-norm's bound wraps");
 struct Plan {
     int n = 0, np = 0;
     int r[kMaxPass] = {0, 0, 0};
