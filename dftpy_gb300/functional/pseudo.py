@@ -198,26 +198,26 @@ class LocalPseudo(NativeFunctional):
         h = self._native.get(dtype)
         if h is None:
             lib = _lib.load()
-            made = self._settings()
-            _, pme, order, keys, gps, vps = made
+            made = (self.grid,) + self._settings()
+            _, pme, order, keys, tables = made
+            tables = [np.array(t, dtype=np.float64) for t in tables]  # copies: a later change shows
+            gps, vps = tables[:len(keys)], tables[len(keys):]
             npts = (_lib.C.c_int * len(keys))(*[len(g) for g in gps])
             gpp = (_lib._PD * len(keys))(*[_lib.dptr(g) for g in gps])
             vpp = (_lib._PD * len(keys))(*[_lib.dptr(v) for v in vps])
             ptr = _lib.C.c_void_p()
             _lib.check(lib.ofdft_pseudo_create(self.grid.native_for(dtype), len(keys), npts, gpp, vpp, pme, order,
                                                _lib.C.byref(ptr)))
-            h = _PseudoHandle(lib, ptr, made)
+            h = _PseudoHandle(lib, ptr, made[:4] + (tables,))
             self._set_ions(h)
             self._native[dtype] = h
         return h.ptr
 
     def _settings(self):
-        """What a native handle is made from, besides the ions: copies, so that a later
-        change of an attribute or of a table's values shows."""
-        keys = self.species_keys
-        return (self.grid, 1 if self.PME else 0, int(self.BsplineOrder), keys,
-                [np.array(self.readpp.gp[k], dtype=np.float64) for k in keys],
-                [np.array(self.readpp.vp[k], dtype=np.float64) for k in keys])
+        """What a native handle is made from, besides the grid and the ions."""
+        keys, pp = self.species_keys, self.readpp
+        return (1 if self.PME else 0, int(self.BsplineOrder), keys,
+                [pp.gp[k] for k in keys] + [pp.vp[k] for k in keys])
 
     def _set_ions(self, h):
         ions, keys = self.ions, self.species_keys
@@ -314,8 +314,9 @@ class LocalPseudo(NativeFunctional):
         self._ions.positions = np.array(positions, dtype=np.float64).reshape(self._ions.nat, 3)
         self._vreal, self.ewald = {}, None
         handles, self._native = self._native, {}
+        now = self._settings() if handles else None
         for dtype, h in handles.items():
-            if h.made_with(self._settings()):
+            if h.made_with(self.grid, now):
                 self._set_ions(h)
                 self._native[dtype] = h
 
@@ -332,10 +333,11 @@ class _PseudoHandle:
     def __init__(self, lib, ptr, made):
         self.lib, self.ptr, self.made = lib, ptr, made
 
-    def made_with(self, now):
-        (grid, *a), (grid_now, *b) = self.made, now
-        same = lambda x, y: len(x) == len(y) and all(map(np.array_equal, x, y))
-        return grid is grid_now and a[:3] == b[:3] and same(a[3], b[3]) and same(a[4], b[4])
+    def made_with(self, grid, now):
+        old_grid, *old, old_tables = self.made
+        *new, tables = now
+        return grid is old_grid and old == new and all(
+            np.shape(a) == b.shape and not np.any(a != b) for a, b in zip(tables, old_tables))
 
     def __del__(self):
         try:
