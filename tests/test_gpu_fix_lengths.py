@@ -61,3 +61,12 @@ def test_nan_reaches_every_point(kedf, kw):
     rho = D.DirectField(D.DirectGrid(np.diag([H * n for n in nr]), nr), data=rho_np)
     out = _total(kedf, **kw)(rho)
     assert np.isnan(out.energy) and np.isnan(out.potential.numpy()).all()
+
+
+@pytest.mark.parametrize("kedf", ["TFVW", "WT"])
+def test_infinity_reaches_every_point(kedf):
+    nr = (16, 15, 18)
+    rho_np = _case(nr)[0].numpy().copy()
+    rho_np[3, 4, 5] = np.inf
+    out = _total(kedf)(D.DirectField(D.DirectGrid(np.diag([H * n for n in nr]), nr), data=rho_np))
+    assert not np.isfinite(out.energy) and not np.isfinite(out.potential.numpy()).any()

@@ -43,3 +43,27 @@ def test_capture_and_replay(PME, dtype):
     assert torch.equal(out, ref)
     assert torch.equal(pp.vreal_for(dtype).as_subclass(torch.Tensor),
                        make(moved).vreal_for(dtype).as_subclass(torch.Tensor))
+
+
+@pytest.mark.parametrize("PME", [True, False])
+def test_moved_ions_beside_another_stream(PME):
+    """Ions moved while a call on another stream may still run, and a call on a third stream after it."""
+    lat, pos = syn.fcc_cell(7.6)
+    nr = (48, 40, 36)
+    g, v = syn.analytic_vloc(3.0, 1.0)
+    rng = np.random.default_rng(5)
+    moves = [pos + rng.normal(0, 0.2, pos.shape) for _ in range(6)]
+
+    def make(p):
+        return D.LocalPseudo(grid=D.DirectGrid(lat, nr), ions=D.Ions(symbols=["Al"] * 4, positions=p, cell=lat),
+                             PP_list={"Al": D.functional.RECPOT(r=g, v=v, zval=3)}, PME=PME)
+
+    want = [make(p).vreal.as_subclass(torch.Tensor) for p in moves]
+    torch.cuda.synchronize()
+    pp, streams, got = make(pos), [torch.cuda.Stream() for _ in range(3)], []
+    for i, p in enumerate(moves):
+        pp.set_positions(p)
+        with torch.cuda.stream(streams[i % 3]):
+            got.append(pp.vreal.as_subclass(torch.Tensor))
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
