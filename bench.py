@@ -62,17 +62,19 @@ TRAFFIC_RATIO_SPLIT = {
     "lwt_pot2": (1.0845 + 0.0635) / ((16 + 1) * 67633152 / 1e9),
     "fz_hat": (0.1345 + 1.0206) / ((16 * 67633152 + 2 * 4 * 16777216) / 1e9),
 }
-# DRAM traffic per algorithmic byte of each kernel class, from one ncu capture of
-# the same kernels on the 256^3 grid with 16 nodes (dram__bytes_read.sum +
-# dram__bytes_write.sum over the bytes the launch must move); a launch at 64
-# nodes moves 4x the planes of that capture, so its traffic scales with them.
+# DRAM traffic per algorithmic byte of each kernel class, from ncu captures of the same kernels
+# on the 256^3 grid with 16 nodes (dram__bytes_read.sum + dram__bytes_write.sum over the bytes
+# the launch must move; NEED: the rows that the nodes need there, from the hat pass's writes); a
+# launch at 64 nodes moves 4x the planes of those captures, so its traffic scales with them.
 TRAFFIC_SOURCE = "ncu dram__bytes of the same kernel at 256^3 with 16 nodes, scaled by planes per launch"
+NEED = 0.4455
+PLANE, FIELD = 67633152 / 1e9, 4 * 16777216 / 1e9
 TRAFFIC_RATIO = {
-    "fz_axis1": (2.165 + 2.104) / (32 * 2 * 67633152 / 1e9),
-    "lwt_nodes": (0.072 + 1.021) / ((16 + 1) * 67633152 / 1e9),
-    "lwt_interp": (1.150 + 0.066) / ((16 * 67633152 + 2 * 4 * 16777216) / 1e9),
-    "lwt_pot2": (1.083 + 0.014) / ((16 + 1) * 67633152 / 1e9),
-    "fz_hat": (0.134 + 1.021) / ((16 * 67633152 + 2 * 4 * 16777216) / 1e9),
+    "fz_axis1": (2.165 + 1.064) / (32 * (1 + NEED) * PLANE),
+    "lwt_nodes": (0.072 + 1.021) / ((16 + 1) * PLANE),
+    "lwt_interp": (0.067 + 2 * (0.612 + 0.061)) / (FIELD + 2 * (16 * NEED * PLANE + 2 * FIELD)),
+    "lwt_pot2": (1.083 + 0.014) / ((16 + 1) * PLANE),
+    "fz_hat": (0.135 + 0.482) / (16 * NEED * PLANE + 2 * FIELD),
 }
 
 

@@ -9,12 +9,12 @@
 // butterflies, exchanges go through one shared buffer of the tile (read, barrier, write),
 // and the last pass of a column hands its outputs to the caller from registers.
 //
-// What bounds it: neither a pipe (ALU, FMA and FP64 at 27 to 35%) nor memory, but latency:
-// straight-line butterflies of up to 16 elements on a dozen warps per SM.  Hence the small
-// blocks with every thread busy and 128 registers per thread.  128^3, three fields: one axis
-// pass 52 us, the axis-0 pair with its factor 190 us, rows 73 and 78 us (a cuFFT float64
-// transform of one field takes 240 us; tiles padded along k2, two buffers and 168 registers
-// per thread took 79, 291, 85 and 88 us).
+// What bounds it: neither a pipe (k_cols at 128^3: ALU 39, FP64 37, FMA 15% busy, issue slots
+// 37%) nor memory (11%), but latency: straight-line butterflies of up to 16 elements on a dozen
+// warps per SM, and instruction fetches.  Hence the small blocks with every thread busy and 128
+// registers per thread.  128^3, three fields: one axis pass 52 us, the axis-0 pair with its factor
+// 205 us, rows 73 and 78 us (a cuFFT float64 transform of one field takes 240 us; tiles padded
+// along k2, two buffers and 168 registers per thread took 79, 291, 85 and 88 us).
 #pragma once
 #include "common.cuh"
 #include "fix_fft.cuh"

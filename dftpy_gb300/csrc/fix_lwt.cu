@@ -11,8 +11,8 @@
 // node are left out, and a plane's value is converted back to float64 at about 1 in 30 points.
 //
 // 64 x 72 x 80 with 64 nodes (linear, potential): 8.8 ms an evaluation on float64 library
-// transforms, 2.9 ms here, of which nodes 0.66, axis 1 0.38 + 0.22, rows 0.42, pot2 0.35,
-// hats 0.21 ms.
+// transforms, 2.9 ms here, of which nodes 0.66, axis 1 0.38 + 0.22, rows 0.43, pot2 0.36,
+// hats 0.22 ms and the local terms 0.5 (profiles/fix_kernels_float64.md).
 #include "fix_eval.h"
 
 #include "fix_3d.cuh"
@@ -170,7 +170,7 @@ __device__ __forceinline__ void stage_column(const Lwt& a, int lb, double* sq, d
 
 // Axis 0 inverse of K_j FFT(rho^beta)/N (plane jj) and, nm = 2, K'_j/k_j FFT(rho^beta)/N (plane
 // nb + jj) for the block's share of the batch's nodes; |G| and FFT(rho^beta)/N of the tile stay
-// in shared memory.  Bound by the float64 pipe, 83% busy at 64 x 72 x 80: eleven operations per
+// in shared memory.  Bound by the float64 pipe, 82% busy at 64 x 72 x 80: eleven operations per
 // value (table 4, product 2, conversions 5); the interval's float32 argument is taken from the
 // bits instead of converted, and K'_j's factor 1/k_j is left to the points that use it.
 __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_nodes(Lwt a) {
@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_nodes(Lwt a) {
 }
 
 // Axis 1 of the planes (node j0 + plane % nb), in place: the inverse stores and the forward
-// transform reads the rows that the node needs only.  Integer issue slots about half used with
-// 14 warps per SM, which the registers allow.
+// transform reads the rows that the node needs only.  Issue slots 49% used with the 14 warps per
+// SM that the registers allow (ALU 44%, float64 34%).
 template <bool INV>
 __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_axis1(Lwt a) {
     extern __shared__ __align__(16) unsigned char fix_smem[];
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_axis1(Lwt a) {
 // The row passes: a block has two rows (one complex line) and transforms them for its part of
 // the planes that they need, as many at a time as the tile has lines.  One row pair per tile keeps the
 // list short (a warp with eight rows to a node transformed 1.5 times as much), and warps that
-// run the same passes together share the instruction cache (one-warp blocks: 60% of the stalls
-// were fetches).  In shared memory: the codes of the points and the planes' list (2 node + plane).
+// run the same passes together share the instruction cache (fetches are still the most common
+// stall of k_fx_rows).  In shared memory: the codes of the points and the planes' list (2 node + plane).
 struct RowPair {
     long long row0;
     int two;                // rows: 1 or 2
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_hats(Lwt a) {
 
 // Axis 0 forward of the hat planes, times K_j (plane jj) or K'_j/k_j (plane nb + jj) over N,
 // summed over the block's share of the nodes into pot2(G) (share = nb) or into one partial
-// spectrum per share.  Float64 pipe 83% busy, as k_fx_nodes.
+// spectrum per share.  Float64 pipe 82% busy, as k_fx_nodes.
 __global__ void __launch_bounds__(kThreads, kBlocks) k_fx_pot2(Lwt a) {
     extern __shared__ __align__(16) unsigned char fix_smem[];
     __shared__ LineSm sm;
