@@ -71,7 +71,9 @@ class TotalFunctional(AbstractFunctional):
 
     def evaluator(self, grid, dtype):
         """The fused native evaluator of this total functional on (grid, dtype)."""
-        c = self._config()
+        return self._evaluator(self._config(), grid, dtype)
+
+    def _evaluator(self, c, grid, dtype):
         key = (id(grid), dtype, c.key)
         ev = self._evals.get(key)
         if ev is None:
@@ -102,7 +104,10 @@ class TotalFunctional(AbstractFunctional):
         if split or not self._fusable():
             return self._separate(rho, calcType, split)
         calc = calc_bits(calcType)
-        ev = self.evaluator(rho.grid, rho.dtype)
+        if type(self).evaluator is TotalFunctional.evaluator and "evaluator" not in self.__dict__:
+            ev = self._evaluator(self._config_cache, rho.grid, rho.dtype)  # as _fusable has just checked it
+        else:
+            ev = self.evaluator(rho.grid, rho.dtype)
         self.prepare(ev, rho.grid, rho.dtype)
         E, V = ev.compute(rho, calc)
         self.finish(ev)
