@@ -104,7 +104,9 @@ class TotalFunctional(AbstractFunctional):
         if split or not self._fusable():
             return self._separate(rho, calcType, split)
         calc = calc_bits(calcType)
-        if type(self).evaluator is TotalFunctional.evaluator and "evaluator" not in self.__dict__:
+        cls, own = type(self), self.__dict__
+        if cls.evaluator is TotalFunctional.evaluator and cls._fusable is TotalFunctional._fusable and \
+                "evaluator" not in own and "_fusable" not in own:
             ev = self._evaluator(self._config_cache, rho.grid, rho.dtype)  # as _fusable has just checked it
         else:
             ev = self.evaluator(rho.grid, rho.dtype)

@@ -84,3 +84,30 @@ def test_option_values():
     assert _cfg(total).tf_x == 0.5
     ke.options["x"] = 0.6
     assert _cfg(total).tf_x == 0.6
+
+
+def test_overridden_evaluator():
+    """An evaluator() or _fusable() of a derived class is asked on every evaluation."""
+    asked = []
+
+    class Mine(D.TotalFunctional):
+        def evaluator(self, grid, dtype):
+            asked.append("evaluator")
+            raise RuntimeError("mine")
+
+    class Always(D.TotalFunctional):
+        def _fusable(self):
+            return True
+
+        def _evaluator(self, c, grid, dtype):
+            asked.append(c.key is not None)
+            raise RuntimeError("mine")
+
+    lat = np.diag([8.0, 8.0, 8.0])
+    rho = D.DirectField(D.DirectGrid(lat, (6, 6, 6)), data=np.full((6, 6, 6), 0.03), device="cpu")
+    for cls in (Mine, Always):
+        total = cls(KE=D.Functional(type="KEDF", name="TF"))
+        for _ in range(2):
+            with pytest.raises(RuntimeError, match="mine"):
+                total(rho)
+    assert asked == ["evaluator", "evaluator", True, True]
